@@ -217,10 +217,14 @@ int auto_group(int ny, int nx) {
   return (int)g;
 }
 
-// Schedules a plan starts with: the plan autotuner's choice on GB300 (random
-// inputs, bandwidth 1/3, the groups above) -- the paired row transform for
-// rows of 512, 16-column tiles for columns of 768, the first schedule
-// elsewhere.
+// Schedules a plan starts with, by event timings on GB300 of groups of about
+// 1 GiB at bandwidth 1/3 (us per pass):
+//   rows of 512     paired transform 364, first schedule 374
+//   rows of 768     48 x 16 463, 8 x 8 x 12 515 (228 waves)
+//   columns of 768  48 x 16 279, 8 x 8 x 12 342 in 16-column tiles, 391 in 8-column ones
+//   columns of 384  48 x 8 123, 8 x 8 x 6 149 (400 waves; rows of 384 are
+//                   faster with 8 x 8 x 6: 230 against 239)
+// and the first schedule elsewhere.
 int schedule_index(int n, const char* name) {
   const SchedOps* ops = nullptr;
   const int k = schedule_table(n, &ops);
@@ -228,8 +232,12 @@ int schedule_index(int n, const char* name) {
     if (std::strcmp(ops[i].name, name) == 0) return i;
   return 0;
 }
-int default_row_schedule(int nx) { return nx == 512 ? schedule_index(512, "t32_r16x2x16_pair") : 0; }
-int default_col_schedule(int ny) { return ny == 768 ? schedule_index(768, "t32_r8x8x12_c16") : 0; }
+int default_row_schedule(int nx) {
+  return nx == 512 ? schedule_index(512, "t32_r16x2x16_pair") : nx == 768 ? schedule_index(768, "t16_r48x16") : 0;
+}
+int default_col_schedule(int ny) {
+  return ny == 768 ? schedule_index(768, "t16_r48x16") : ny == 384 ? schedule_index(384, "t8_r48x8") : 0;
+}
 
 struct MsArgs {
   const float* trans; int num_slices; const float* psik; const double* norm; const float* pos; int num_probes;

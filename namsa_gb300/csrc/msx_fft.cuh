@@ -305,6 +305,13 @@ template <bool INV> struct Dft<16, INV> {
 template <bool INV> struct Dft<24, INV> {
   static __host__ __device__ __forceinline__ void run(float2 (&v)[24]) { dft_ct<8, 3, INV>(v); }
 };
+// 48 points as 16 x 3: three 16-point transforms, then sixteen 3-point ones.  A
+// thread that holds 48 values (768 = 48 x 16 with 16 threads, 384 = 48 x 8 with
+// 8) needs one exchange through shared memory where radices 8 x 8 x 12 or
+// 8 x 8 x 6 need two.
+template <bool INV> struct Dft<48, INV> {
+  static __host__ __device__ __forceinline__ void run(float2 (&v)[48]) { dft_ct<16, 3, INV>(v); }
+};
 template <bool INV> struct Dft<32, INV> {
   static __host__ __device__ __forceinline__ void run(float2 (&v)[32]) { dft_ct<4, 8, INV>(v); }
 };

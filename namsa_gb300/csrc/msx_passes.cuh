@@ -25,7 +25,7 @@ namespace msx {
 // A schedule fixes the line transform (threads per line T, radices) and the
 // launch shape for one line length N.  Several schedules exist per N; the
 // autotuner in the host library picks one per grid size.  COL_C columns share
-// a column-pass CTA, whose COL_C * T threads (256 or 512) are also the CTA size
+// a column-pass CTA, whose COL_C * T threads (128 to 512) are also the CTA size
 // of the row pass; MINB is the minimum number of resident CTAs requested from
 // the register allocator.
 template <int N_, int T_, int COL_C_, int MINB_, int... Rs>
@@ -46,7 +46,7 @@ struct Sched {
   static constexpr size_t row_smem() { return sizeof(float2) * (TW_PAD + (size_t)ROW_LINES * ROW_LINE_WORDS); }
   // plain column pass: twiddles, the exchange buffer and (probe formation) one complex factor per row
   static constexpr size_t col_smem() { return sizeof(float2) * (TW_PAD + (size_t)C * N + N); }
-  static_assert(THREADS == 256 || THREADS == 512, "CTA of 256 or 512 threads");
+  static_assert(THREADS == 128 || THREADS == 256 || THREADS == 512, "CTA of 128, 256 or 512 threads");
   static_assert(T <= 32 && 32 % T == 0, "a row line must live inside one warp");
   static constexpr bool PAIRED = false;  // persistent row pass uses PairedFFT512
 };
