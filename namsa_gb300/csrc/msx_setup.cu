@@ -3,6 +3,9 @@
 // normalisation, and the propagator table.
 #include "msx_internal.h"
 
+#include <cooperative_groups.h>
+
+#include <atomic>
 #include <cmath>
 
 namespace msx {
@@ -10,18 +13,37 @@ namespace msx {
 // ------------------------------------------------------------------ Bessel K0
 // K0(x) = int_0^inf exp(-x cosh u) du (x > 0).  The integrand is analytic and
 // decays double-exponentially in the strip |Im u| < pi/2, so the trapezoidal
-// rule with step h converges like exp(-pi^2 / h); h = 1/8 leaves an error far
-// below double rounding for the arguments used here (x >= 0.1).  The sum stops
-// once a term falls below 1e-18 of the running sum.
+// rule with step h converges like exp(-pi^2 / h) while the peak at u = 0, of
+// width 1/sqrt(x), is wide against h: h = 1/4 is within 7e-15 of the limit for
+// x < 6 (measured against h = 1/16 on [0.1, 6.5]), h = 1/8 serves the larger x,
+// whose sums are short.  The sum stops once a term falls below 1e-18 of the
+// running sum: cosh(u) < 1 + 42 / x, so u < 7 for every x >= 0.1.
+constexpr int kCoshTable = 64;  // cosh(k / 8)
+struct CoshTable {
+  double v[kCoshTable];
+  constexpr CoshTable() : v() {
+    for (int k = 0; k < kCoshTable; ++k) {
+      const double x = k / 8.0;
+      double term = 1.0, sum = 1.0;  // all terms positive: x < 8 needs 30 of them
+      for (int n = 1; n < 40; ++n) {
+        term *= x * x / double((2 * n - 1) * (2 * n));
+        sum += term;
+      }
+      v[k] = sum;
+    }
+  }
+};
+__constant__ CoshTable kCosh{};
+
 __device__ double bessel_k0(double x) {
-  const double h = 0.125;
+  const int step = x < 6.0 ? 2 : 1;  // in units of 1/8
   double sum = 0.5 * exp(-x);
-  for (int k = 1; k < 400; ++k) {
-    const double term = exp(-x * cosh(k * h));
+  for (int k = step; k < kCoshTable; k += step) {
+    const double term = exp(-x * kCosh.v[k]);
     sum += term;
     if (term < 1e-18 * sum) break;
   }
-  return h * sum;
+  return 0.125 * step * sum;
 }
 
 // ------------------------------------------------------------------ atom windows
@@ -32,50 +54,77 @@ __device__ double bessel_k0(double x) {
 // with a0 = 0.529, e = 14.4, the oversample x oversample mean, minus the window
 // minimum, rounded to float32.  All arithmetic is double.
 //
-// Every Kirkland coefficient is positive, so v decreases with r and the
-// window minimum is the corner bin (each of its samples lies farther out than
-// the matching sample of any other bin); every CTA evaluates the corner bins
-// itself, which needs no grid-wide reduction.  Grid: (species, bin blocks).
-__device__ double window_bin(const double* c, int i, int j, int os, double sx, double sy, double start) {
+// The grid is symmetric about its centre, so bins (i, j), (H-1-i, j), (i, W-1-j)
+// and (H-1-i, W-1-j) are equal and one quadrant is evaluated.  Every Kirkland
+// coefficient is positive, so v decreases with r and the window minimum is the
+// corner bin, which each CTA evaluates beside its own bins.
+//
+// Bound by double-precision instructions (about two fused multiply-adds a
+// clock and SM): an exponential per quadrature term.  The quadrant takes a
+// quarter of the samples, the table the cosh of every term, the coarser step
+// half of the terms of small x, and one thread per oversampled row of a bin
+// fills the chip.  94 x 94 bins of one species at oversample 2: 938 us with
+// every bin evaluated by one thread, 110 us so.
+constexpr int kWinThreads = 128;
+
+// sum over b (in order) of the samples (i os + a, j os + b)
+__device__ double window_row(const double* c, int i, int j, int a, int os, double sx, double sy, double start) {
   const double pi = 3.14159265358979323846;
   const double pre = 4.0 * pi * pi * 0.529 * 14.4;
-  double acc0 = 0;  // numpy's order: mean over the last axis, then over the second-to-last
-  for (int a = 0; a < os; ++a) {
-    double accr = 0;
-    for (int b = 0; b < os; ++b) {
-      const double gx = (double)(i * os + a) * sx + start;
-      const double gy = (double)(j * os + b) * sy + start;
-      const double r = sqrt(gx * gx + gy * gy);
-      double v = 0;
-      for (int k = 0; k < 3; ++k) {
-        const double ak = c[k], bk = c[3 + k], ck = c[6 + k], dk = c[9 + k];
-        const double term = pre * ak * bessel_k0(2 * pi * r * sqrt(bk) + 0.1) + pre / 2. * ck / dk * exp(-pi * pi * r * r / dk);
-        v = (k == 0) ? term : v + term;
-      }
-      accr = (b == 0) ? v : accr + v;
+  double accr = 0;
+  for (int b = 0; b < os; ++b) {
+    const double gx = (double)(i * os + a) * sx + start;
+    const double gy = (double)(j * os + b) * sy + start;
+    const double r = sqrt(gx * gx + gy * gy);
+    double v = 0;
+    for (int k = 0; k < 3; ++k) {
+      const double ak = c[k], bk = c[3 + k], ck = c[6 + k], dk = c[9 + k];
+      const double term = pre * ak * bessel_k0(2 * pi * r * sqrt(bk) + 0.1) + pre / 2. * ck / dk * exp(-pi * pi * r * r / dk);
+      v = (k == 0) ? term : v + term;
     }
-    accr /= os;
-    acc0 = (a == 0) ? accr : acc0 + accr;
+    accr = (b == 0) ? v : accr + v;
   }
-  return acc0 / os;
+  return accr / os;
 }
 
-__global__ void atom_window_kernel(const double* __restrict__ coeff, int n0, int n1, int os, double range,
-                                   float* __restrict__ out) {
-  __shared__ double corner[4];
+// Grid: (species, blocks of bins of the quadrant).  `rows` threads share a bin
+// (the oversampled rows a, a + rows, ...); slot 0 is the corner bin, slots
+// 1 .. bins are the block's own.  numpy's order: mean over the last axis, then
+// over the second-to-last.
+__global__ void __launch_bounds__(kWinThreads)
+atom_window_kernel(const double* __restrict__ coeff, int n0, int n1, int os, int rows, int bins, double range,
+                   float* __restrict__ out) {
+  __shared__ double part[kWinThreads];
+  __shared__ double val[kWinThreads];
   const int h0 = n0 / os, h1 = n1 / os;
+  const int q1 = (h1 + 1) / 2, quad = ((h0 + 1) / 2) * q1;
   const double* c = coeff + 12 * blockIdx.x;
   const double start = -range / 2, sx = range / (double)(n0 - 1), sy = range / (double)(n1 - 1);
-  if (threadIdx.x < 4) {
-    const int ci = (threadIdx.x & 1) ? h0 - 1 : 0, cj = (threadIdx.x & 2) ? h1 - 1 : 0;
-    corner[threadIdx.x] = window_bin(c, ci, cj, os, sx, sy, start);
+  const int slot = threadIdx.x / rows, a0 = threadIdx.x % rows;
+  const int bin = slot == 0 ? 0 : blockIdx.y * bins + slot - 1;  // bin 0 is the corner
+  const bool live = slot <= bins && bin < quad;
+  double acc = 0;
+  for (int base = 0; base < os; base += rows) {
+    const int a = base + a0;
+    part[threadIdx.x] = live && a < os ? window_row(c, bin / q1, bin % q1, a, os, sx, sy, start) : 0.0;
+    __syncthreads();
+    if (live && a0 == 0)
+      for (int k = 0; k < rows && base + k < os; ++k) {
+        const double v = part[threadIdx.x + k];
+        acc = (base + k == 0) ? v : acc + v;
+      }
+    __syncthreads();
   }
+  if (a0 == 0) val[slot] = acc / os;
   __syncthreads();
-  const double vmin = fmin(fmin(corner[0], corner[1]), fmin(corner[2], corner[3]));
-  const int o = blockIdx.y * blockDim.x + threadIdx.x;
-  if (o < h0 * h1) {
-    const double v = window_bin(c, o / h1, o % h1, os, sx, sy, start);
-    out[(size_t)blockIdx.x * h0 * h1 + o] = (float)(v - vmin);
+  if (live && slot > 0 && a0 == 0) {
+    const float v = (float)(val[slot] - val[0]);
+    const int i = bin / q1, j = bin % q1;
+    float* o = out + (size_t)blockIdx.x * h0 * h1;
+    o[(size_t)i * h1 + j] = v;
+    o[(size_t)(h0 - 1 - i) * h1 + j] = v;
+    o[(size_t)i * h1 + h1 - 1 - j] = v;
+    o[(size_t)(h0 - 1 - i) * h1 + h1 - 1 - j] = v;
   }
 }
 
@@ -92,6 +141,7 @@ __global__ void atom_window_kernel(const double* __restrict__ coeff, int n0, int
 // tested against the tile and the overlapping ones are compacted in order.
 constexpr int kPotTile = 32;
 constexpr int kPotThreads = 256;
+constexpr int kPotBatch = 4;
 
 __global__ void __launch_bounds__(kPotThreads)
 potential_kernel(const int4* __restrict__ sites, const int* __restrict__ slice_off, const float* __restrict__ windows,
@@ -129,18 +179,28 @@ potential_kernel(const int4* __restrict__ sites, const int* __restrict__ slice_o
     }
     if (hit) list[offset + __popc(ballot & ((1u << lane) - 1u))] = st;
     __syncthreads();
-    for (int i = 0; i < total; ++i) {
-      const int4 e = list[i];
-      const int ys = e.w;
-      const int ye = (int)rintf((float)e.y + hh);
-      const int xs = (int)rintf((float)e.z - hw), xe = (int)rintf((float)e.z + hw);
-      const float* win = windows + (size_t)e.x * H * W;
-      const bool colok = px >= 0 && px < xe && px < Nx && px >= xs && (px - xs) < W;
+    // the windows of four sites are read before the first is added: sixteen loads
+    // in flight per thread, the additions still in site order (a pixel outside a
+    // window adds +0, which leaves the sum as it is)
+    for (int i0 = 0; i0 < total; i0 += kPotBatch) {
+      float w[kPotBatch][kPotTile / 8];
 #pragma unroll
-      for (int k = 0; k < kPotTile / 8; ++k) {
-        const int py = py0 + 8 * k;
-        if (colok && py < ye && py < Ny && py >= ys && (py - ys) < H) acc[k] += __ldg(win + (py - ys) * W + (px - xs));
+      for (int u = 0; u < kPotBatch; ++u) {
+        const int4 e = list[min(i0 + u, total - 1)];
+        const int ys = e.w, xs = (int)rintf((float)e.z - hw);
+        const int ye = min((int)rintf((float)e.y + hh), Ny), xe = min((int)rintf((float)e.z + hw), Nx);
+        const float* win = windows + (size_t)e.x * H * W + (px - xs);
+        const bool colok = i0 + u < total && px < xe && px >= xs && px - xs < W;
+#pragma unroll
+        for (int k = 0; k < kPotTile / 8; ++k) {
+          const int py = py0 + 8 * k;
+          w[u][k] = colok && py < ye && py >= ys && py - ys < H ? __ldg(win + (py - ys) * W) : 0.f;
+        }
       }
+#pragma unroll
+      for (int u = 0; u < kPotBatch; ++u)
+#pragma unroll
+        for (int k = 0; k < kPotTile / 8; ++k) acc[k] += w[u][k];
     }
     __syncthreads();
   }
@@ -151,7 +211,8 @@ potential_kernel(const int4* __restrict__ sites, const int* __restrict__ slice_o
       if (py < Ny) {
         const size_t o = ((size_t)s * Ny + py) * Nx + px;
         const float arg = acc[k] * sigma;
-        float2 tv = make_float2(cosf(arg), sinf(arg));
+        float2 tv;
+        sincosf(arg, &tv.y, &tv.x);
         if (isnan(tv.x)) tv.x = 1.f;
         if (isnan(tv.y)) tv.y = 1.f;
         trans[o] = tv;
@@ -185,34 +246,69 @@ __global__ void probe_kernel(int Ny, int Nx, float kmax, double lambda, float k_
   const int y = blockIdx.y;
   if (x >= Nx) return;
   const double k = krad_exact(x, y, Nx, Ny, kmax);
+  const size_t o = (size_t)y * Nx + x;
   double a;
-  if (smooth) a = 1.0 / (1.0 + exp(-160.0 * ((double)k_semi - k)));
-  else a = ((float)k < k_semi) ? 1.0 : 0.0;
+  if (smooth) {
+    // 1 / (1 + exp(u)): exactly 1 in double below u = -38, and 0 after rounding to
+    // float32 above u = 104 (the smallest float32 is 1.4e-45), where the phase is
+    // not needed: most of the grid.  The kernel is bound by double-precision
+    // instructions.
+    const double u = -160.0 * ((double)k_semi - k);
+    if (u > 104.0 && isfinite(C1 + C3 + C5)) {
+      psik[o] = make_float2(0.f, 0.f);
+      if (aperture) aperture[o] = 0.f;
+      return;
+    }
+    a = u < -38.0 ? 1.0 : 1.0 / (1.0 + exp(u));
+  } else {
+    a = ((float)k < k_semi) ? 1.0 : 0.0;
+    if (a == 0.0 && isfinite(C1 + C3 + C5)) {
+      psik[o] = make_float2(0.f, 0.f);
+      if (aperture) aperture[o] = 0.f;
+      return;
+    }
+  }
   const double kl = k * lambda, kl2 = kl * kl;
   const double chi = 2.0 * 3.14159265358979323846 / lambda * (-0.5 * C1 * kl2 + 0.25 * C3 * kl2 * kl2 + C5 / 6.0 * kl2 * kl2 * kl2);
   double sn, cs;
   sincos(chi, &sn, &cs);
-  const size_t o = (size_t)y * Nx + x;
   psik[o] = make_float2((float)(a * cs), (float)(-a * sn));
   if (aperture) aperture[o] = (float)a;
 }
 
 // normalisation = sum |fftshift(ifft2_u(psi_k))|^2 = N * sum |psi_k|^2 (Parseval),
-// accumulated in double by one CTA in a fixed order (msa.py:721-727).
-__global__ void probe_norm_kernel(const float2* __restrict__ psik, long long n, double* __restrict__ out) {
-  __shared__ double red[1024];
+// accumulated in double in a fixed order (msa.py:721-727) by one cluster of 16
+// CTAs: strided partial sums per thread, a tree per CTA, and the CTAs' sums in
+// rank order through distributed shared memory, which needs no scratch in
+// global memory.  Bound by double-precision instructions (three a value on
+// about two lanes a clock and SM): 512^2 368 us on one CTA, 28 us so.
+constexpr int kNormCtas = 16, kNormThreads = 512;
+__global__ void __launch_bounds__(kNormThreads) probe_norm_kernel(const float2* __restrict__ psik, long long n,
+                                                                  double* __restrict__ out) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ double red[kNormThreads];
+  __shared__ double ranks[kNormCtas];
+  const int rank = (int)cl.block_rank(), nr = (int)cl.num_blocks();
+  cl.sync();  // every CTA runs before its shared memory is written
   double acc = 0;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
+  for (long long i = (long long)rank * kNormThreads + threadIdx.x; i < n; i += (long long)nr * kNormThreads) {
     const float2 v = psik[i];
     acc += (double)v.x * v.x + (double)v.y * v.y;
   }
   red[threadIdx.x] = acc;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+  for (int s = kNormThreads / 2; s > 0; s >>= 1) {
+    if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[0] = red[0] * (double)n;
+  if (threadIdx.x == 0) *cl.map_shared_rank(&ranks[rank], 0) = red[0];
+  cl.sync();  // rank 0's array is complete
+  if (rank == 0 && threadIdx.x == 0) {
+    double sum = 0;
+    for (int r = 0; r < nr; ++r) sum += ranks[r];
+    out[0] = sum * (double)n;
+  }
 }
 
 // ------------------------------------------------------------------ propagator table
@@ -319,10 +415,11 @@ cudaError_t launch_detect_reduce(const float* partial, int G, int tiles, int nde
 
 cudaError_t launch_atom_windows(const double* coeff, int nspecies, int n0, int n1, int os, double range, float* out,
                                 cudaStream_t st) {
-  const int h0 = n0 / os, h1 = n1 / os;
-  const int threads = 128;
-  const dim3 grid(nspecies, (h0 * h1 + threads - 1) / threads);
-  atom_window_kernel<<<grid, threads, 0, st>>>(coeff, n0, n1, os, range, out);
+  const int rows = os < kWinThreads / 2 ? os : kWinThreads / 2;  // threads per bin
+  const int bins = kWinThreads / rows - 1;                       // a block's own bins; one slot is the corner
+  const int quad = ((n0 / os + 1) / 2) * ((n1 / os + 1) / 2);
+  const dim3 grid(nspecies, (quad + bins - 1) / bins);
+  atom_window_kernel<<<grid, kWinThreads, 0, st>>>(coeff, n0, n1, os, rows, bins, range, out);
   return cudaGetLastError();
 }
 
@@ -339,13 +436,27 @@ cudaError_t launch_probe(int Ny, int Nx, float kmax, double lambda, float k_semi
   probe_kernel<<<grid, 128, 0, st>>>(Ny, Nx, kmax, lambda, k_semi, C1, C3, C5, smooth, psik, aperture);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || norm == nullptr) return e;
-  probe_norm_kernel<<<1, 1024, 0, st>>>(psik, (long long)Ny * Nx, norm);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_probe_norm(const float2* psik, int Ny, int Nx, double* norm, cudaStream_t st) {
-  probe_norm_kernel<<<1, 1024, 0, st>>>(psik, (long long)Ny * Nx, norm);
-  return cudaGetLastError();
+  // clusters of 16 are above the portable size: allowed once per device
+  static std::atomic<unsigned long long> allowed{0};
+  int dev = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (!(allowed.load(std::memory_order_acquire) & bit)) {
+    e = cudaFuncSetAttribute(probe_norm_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    allowed.fetch_or(bit, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kNormCtas);
+  cfg.blockDim = dim3(kNormThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kNormCtas;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, probe_norm_kernel, psik, (long long)Ny * Nx, norm);
 }
 
 cudaError_t launch_ptab(int Ny, int Nx, float kmax, double lambda, double slice_t, float k_band, float2* ptab,
