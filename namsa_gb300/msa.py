@@ -24,6 +24,7 @@ tensors (``trans``, ``cbed``); the reference's host attributes
 """
 from __future__ import annotations
 
+import functools
 import os
 from warnings import warn
 
@@ -40,9 +41,14 @@ DEFAULT_PROBE = {'smooth_apert': True, 'apert_smooth': 50, 'spherical_phase': Tr
                  'aberration_dict': {'C1': 0., 'C3': 0., 'C5': 0.}, 'scherzer': True}
 
 
+@functools.lru_cache(maxsize=1)
+def _kirkland_file():
+    return np.load(os.path.join(_DATA, 'kirkland_params.npy'))
+
+
 def kirkland_table():
     """(103, 4, 3) float64 Kirkland parameters indexed by Z-1 (namsa/database.py:7-8)."""
-    return np.load(os.path.join(_DATA, 'kirkland_params.npy'))
+    return _kirkland_file().copy()
 
 
 # ----------------------------------------------------------------------------- host tables
@@ -83,19 +89,26 @@ def slice_sites(xyz, Z, pix_size, slice_t, num_slices):
     Z = np.asarray(Z)
     uz = np.unique(Z)
     zidx = np.searchsorted(uz, Z)
-    pix = xyz[:, :2] / np.asarray(pix_size)[::-1]
     z = xyz[:, 2]
-    rows, offs = [], [0]
-    for s in range(num_slices):
-        m = np.logical_and(z >= s * slice_t, z < (s + 1) * slice_t)
-        yx = pix[m]
-        st = np.column_stack([zidx[m], yx[:, 1], yx[:, 0]]).astype(np.int32)
-        rows.append(st)
-        offs.append(offs[-1] + len(st))
-    sites = np.zeros((offs[-1], 4), np.int32)
-    if offs[-1]:
-        sites[:, :3] = np.concatenate(rows)
-    return sites, np.asarray(offs, np.int32)
+    # the slice edges in the type that comparing float32 z with s * slice_t uses: float32 for a
+    # Python number or a float32, else the wider type
+    edges = np.asarray([s * slice_t for s in range(num_slices + 1)])
+    edges = edges.astype(np.result_type(z, slice_t))
+    # edges rise with s, so z lies in the last slice that starts at or below it (NaN sorts past the
+    # end); one stable sort groups the atoms by slice, in supercell order within each
+    s_of = np.searchsorted(edges, z, side='right') - 1
+    inside = (s_of >= 0) & (s_of < num_slices)
+    order = np.flatnonzero(inside)
+    key = s_of[order]
+    order = order[np.argsort(key.astype(np.int16) if num_slices < 32768 else key, kind='stable')]  # 16 bits: radix sort
+    offs = np.zeros(max(num_slices, 0) + 1, np.int32)
+    offs[1:] = np.cumsum(np.bincount(s_of[order], minlength=num_slices)[:num_slices]) if num_slices > 0 else 0
+    pix = xyz[order, :2] / np.asarray(pix_size)[::-1]
+    sites = np.zeros((len(order), 4), np.int32)
+    sites[:, 0] = zidx[order]
+    sites[:, 1] = pix[:, 1].astype(np.int32)
+    sites[:, 2] = pix[:, 0].astype(np.int32)
+    return sites, offs
 
 
 def probe_positions_grid(dims, probe_step=np.array([0.1, 0.1]), probe_range=np.array([[0., 1.0], [0., 1.0]]),
@@ -166,9 +179,12 @@ class MSAGPU:
         rng = np.random.default_rng(seed) if seed is not None else np.random
         for Z in np.unique(self.supercell_Z):
             idx = np.where(self.supercell_Z == Z)[0]
-            dw = self.supercell_dw[idx][0]
-            self.supercell_xyz[idx] += float(self.debye_waller) * dw * rng.standard_normal(size=self.supercell_xyz[idx].shape)
-        self.dims = self.supercell_xyz.max(0) - self.supercell_xyz.min(0)
+            scale = float(self.debye_waller) * self.supercell_dw[idx][0]
+            noise = rng.standard_normal(size=(len(idx),) + self.supercell_xyz.shape[1:])  # drawn in any case
+            if scale != 0:
+                self.supercell_xyz[idx] += scale * noise
+        axes = np.ascontiguousarray(self.supercell_xyz.T)
+        self.dims = axes.max(1) - axes.min(1)
         self.max_angle = max_angle
         if max_angle is None:
             self.sampling = np.asarray(sampling)
