@@ -330,9 +330,14 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
   const int gmax = a.num_probes < a.group ? a.num_probes : a.group;
   if (!workspace_holds(p, gmax))
     return fail(MSX_ERR_ALLOC, "the plan's workspace does not hold %d waves (an earlier allocation failed)", gmax);
-  MSX_CUDA(launch_ptab(ny, nx, a.kmax, a.lambda, a.slice_t, a.k_band, p->ptab, st), "propagator table");
-  if (p->use_tma && p->map_ok)
+  // the persistent passes form the propagator from its factors and the mask band;
+  // the table of N values (26 us of double precision at 512^2, 89 us at 1024^2)
+  // serves the plain passes
+  const bool factors = p->use_tma && p->map_ok;
+  if (factors)
     MSX_CUDA(launch_pfac(ny, nx, a.kmax, a.lambda, a.slice_t, a.k_band, p->pyx, p->band, st), "propagator factors");
+  else
+    MSX_CUDA(launch_ptab(ny, nx, a.kmax, a.lambda, a.slice_t, a.k_band, p->ptab, st), "propagator table");
   const size_t wave = (size_t)ny * nx;
   const int y0 = ny / 2 - a.crop_y / 2, x0 = nx / 2 - a.crop_x / 2;
   const float2* trans = reinterpret_cast<const float2*>(a.trans);
@@ -364,6 +369,10 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
     c.kmax = a.kmax;
     c.y0 = y0;
     c.crop_y = a.crop_y;
+    if (factors) {
+      c.band = p->band;
+      c.inv_n = (float)(1.0 / ((double)ny * (double)nx));
+    }
     if (a.num_slices == 0) {
       c.x_begin = x0;
       c.ncols = a.crop_x;

@@ -128,6 +128,10 @@ struct ColArgs {
   int ndet;
   float* partial;          // (G, Nx / C, ndet) per-tile detector sums (detect)
   const double* init_norm; // init: when set, the probe is scaled by 1/sqrt(*init_norm)
+  // final and detect: when set, the factor is inv_n on the rows [x, y] of the
+  // column's mask band and 0 elsewhere instead of ptab (|P| = 1 drops out of |psi|^2)
+  const int2* band;
+  float inv_n;
 };
 
 template <class S, int MODE>
@@ -195,8 +199,17 @@ __global__ void __launch_bounds__(S::THREADS, S::MINB) col_pass_kernel(ColArgs a
     S::FFT::template run<true, true>(v, buf, tw, t);
   } else if constexpr (MODE == COL_FINAL || MODE == COL_DETECT) {
     S::FFT::template run<false, true>(v, buf, tw, t);
+    if (a.band) {
+      const int2 bd = __ldg(a.band + x);
 #pragma unroll
-    for (int m = 0; m < S::E; ++m) v[m] = cmul(v[m], __ldg(pcol + (t + S::T * m) * Nx));
+      for (int m = 0; m < S::E; ++m) {
+        const int ky = t + S::T * m;
+        v[m] = cscale(v[m], ky >= bd.x && ky <= bd.y ? a.inv_n : 0.f);
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < S::E; ++m) v[m] = cmul(v[m], __ldg(pcol + (t + S::T * m) * Nx));
+    }
   }
   // COL_INIT_FINAL (no slices): fft2(ifft2_u(Y)) = N*Y, so v already holds Y.
 

@@ -139,6 +139,14 @@ atom_window_kernel(const double* __restrict__ coeff, int n0, int n1, int os, int
 //
 // Sites are binned per tile in shared memory: each chunk of 256 sites is
 // tested against the tile and the overlapping ones are compacted in order.
+//
+// Bound by instructions (at eight overlapping sites a pixel the 8-byte results
+// need a sixth of the time): the thread that finds a site clips its rectangle
+// once, a warp's rows are tested with warp-uniform branches, and the windows of
+// four sites are read before the first is added (sixteen loads in flight per
+// thread, the additions still in site order; a pixel outside a window adds +0,
+// which leaves the sum as it is).  199 slices of 512^2, 128 sites of 94 x 94
+// each: 391 us with the tests in the inner loop, 290 us so.
 constexpr int kPotTile = 32;
 constexpr int kPotThreads = 256;
 constexpr int kPotBatch = 4;
@@ -146,28 +154,29 @@ constexpr int kPotBatch = 4;
 __global__ void __launch_bounds__(kPotThreads)
 potential_kernel(const int4* __restrict__ sites, const int* __restrict__ slice_off, const float* __restrict__ windows,
                  int H, int W, int Ny, int Nx, float sigma, float2* __restrict__ trans, float* __restrict__ pot) {
-  __shared__ int4 list[kPotThreads];
+  __shared__ int4 rect[kPotThreads];        // rows [x, y), columns [z, w) of a site's window inside the grid
+  __shared__ const float* base[kPotThreads];  // the window's element of pixel (0, 0)
   __shared__ int warp_count[kPotThreads / 32];
   const int s = blockIdx.z;
   const int ty0 = blockIdx.y * kPotTile, tx0 = blockIdx.x * kPotTile;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int px = tx0 + lane;
   const int py0 = ty0 + warp;  // rows py0 + 8*k, k = 0..3
   float acc[kPotTile / 8] = {0.f, 0.f, 0.f, 0.f};
   const int begin = slice_off[s], end = slice_off[s + 1];
   const float hh = H * 0.5f, hw = W * 0.5f;
-  for (int base = begin; base < end; base += kPotThreads) {
-    const int idx = base + threadIdx.x;
-    int4 st = make_int4(0, 0, 0, 0);
+  for (int chunk = begin; chunk < end; chunk += kPotThreads) {
+    const int idx = chunk + threadIdx.x;
+    int4 r = make_int4(0, 0, 0, 0);
+    const float* w0 = windows;
     bool hit = false;
     if (idx < end) {
-      st = sites[idx];
+      const int4 st = sites[idx];
       const int ys = (int)rintf((float)st.y - hh), ye = (int)rintf((float)st.y + hh);
       const int xs = (int)rintf((float)st.z - hw), xe = (int)rintf((float)st.z + hw);
-      const int r0 = max(max(ys, 0), ty0), r1 = min(min(min(ye, Ny), ys + H), ty0 + kPotTile);
-      const int c0 = max(max(xs, 0), tx0), c1 = min(min(min(xe, Nx), xs + W), tx0 + kPotTile);
-      hit = (r1 > r0) && (c1 > c0);
-      st.w = ys;  // keep the start row; the start column is recomputed below
+      r = make_int4(max(ys, 0), min(min(ye, Ny), ys + H), max(xs, 0), min(min(xe, Nx), xs + W));
+      hit = min(r.y, ty0 + kPotTile) > max(r.x, ty0) && min(r.w, tx0 + kPotTile) > max(r.z, tx0);
+      w0 = windows + ((size_t)st.x * H * W - ((long long)ys * W + xs));
     }
     const unsigned ballot = __ballot_sync(0xffffffffu, hit);
     if (lane == 0) warp_count[warp] = __popc(ballot);
@@ -177,30 +186,31 @@ potential_kernel(const int4* __restrict__ sites, const int* __restrict__ slice_o
       if (w < warp) offset += warp_count[w];
       total += warp_count[w];
     }
-    if (hit) list[offset + __popc(ballot & ((1u << lane) - 1u))] = st;
+    if (hit) {
+      const int at = offset + __popc(ballot & ((1u << lane) - 1u));
+      rect[at] = r;
+      base[at] = w0;
+    }
     __syncthreads();
-    // the windows of four sites are read before the first is added: sixteen loads
-    // in flight per thread, the additions still in site order (a pixel outside a
-    // window adds +0, which leaves the sum as it is)
     for (int i0 = 0; i0 < total; i0 += kPotBatch) {
-      float w[kPotBatch][kPotTile / 8];
+      float v[kPotBatch][kPotTile / 8];
 #pragma unroll
       for (int u = 0; u < kPotBatch; ++u) {
-        const int4 e = list[min(i0 + u, total - 1)];
-        const int ys = e.w, xs = (int)rintf((float)e.z - hw);
-        const int ye = min((int)rintf((float)e.y + hh), Ny), xe = min((int)rintf((float)e.z + hw), Nx);
-        const float* win = windows + (size_t)e.x * H * W + (px - xs);
-        const bool colok = i0 + u < total && px < xe && px >= xs && px - xs < W;
+        const int i = min(i0 + u, total - 1);
+        const int4 q = rect[i];
+        const float* w = base[i] + px;
+        const bool colok = i0 + u < total && px >= q.z && px < q.w;
 #pragma unroll
         for (int k = 0; k < kPotTile / 8; ++k) {
           const int py = py0 + 8 * k;
-          w[u][k] = colok && py < ye && py >= ys && py - ys < H ? __ldg(win + (py - ys) * W) : 0.f;
+          v[u][k] = 0.f;
+          if (py >= q.x && py < q.y && colok) v[u][k] = __ldg(w + (long long)py * W);
         }
       }
 #pragma unroll
       for (int u = 0; u < kPotBatch; ++u)
 #pragma unroll
-        for (int k = 0; k < kPotTile / 8; ++k) acc[k] += w[u][k];
+        for (int k = 0; k < kPotTile / 8; ++k) acc[k] += v[u][k];
     }
     __syncthreads();
   }
@@ -226,11 +236,15 @@ potential_kernel(const int4* __restrict__ sites, const int* __restrict__ slice_o
 // |k| on the centred grid, evaluated with the reference's operation order
 // (calc_krad, probe_kernels.cu:11-16) and without FMA contraction, so that the
 // float32 aperture and bandwidth decisions are reproducible on the host.
-__device__ __forceinline__ double krad_exact(int x, int y, int Nx, int Ny, float kmax) {
+__device__ __forceinline__ double kaxis_exact(int j, int n, float kmax) {
   const double km = (double)kmax;
-  const double kx = __dsub_rn(__ddiv_rn(__dmul_rn((double)x, km), (double)(Nx - 1)), __ddiv_rn(km, 2.0));
-  const double ky = __dsub_rn(__ddiv_rn(__dmul_rn((double)y, km), (double)(Ny - 1)), __ddiv_rn(km, 2.0));
+  return __dsub_rn(__ddiv_rn(__dmul_rn((double)j, km), (double)(n - 1)), __ddiv_rn(km, 2.0));
+}
+__device__ __forceinline__ double krad_of(double kx, double ky) {
   return __dsqrt_rn(__dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)));
+}
+__device__ __forceinline__ double krad_exact(int x, int y, int Nx, int Ny, float kmax) {
+  return krad_of(kaxis_exact(x, Nx, kmax), kaxis_exact(y, Ny, kmax));
 }
 
 // k-space probe psi_k = A(k) exp(-i chi(k)) on the centred grid
@@ -240,40 +254,49 @@ __device__ __forceinline__ double krad_exact(int x, int y, int Nx, int Ny, float
 // (probe_kernels.cu:180-194); chi = 2 pi/lambda (-C1/2 (k lambda)^2 +
 // C3/4 (k lambda)^4 + C5/6 (k lambda)^6) (probe_kernels.cu:208-222).  Evaluated
 // in double, stored as complex64 like the reference's psi_k (msa.py:710-717).
-__global__ void probe_kernel(int Ny, int Nx, float kmax, double lambda, float k_semi, double C1, double C3, double C5,
-                             int smooth, float2* __restrict__ psik, float* __restrict__ aperture) {
+//
+// A thread takes kProbeRows rows of one column, so that the divisions of kx and
+// ky are done once per thread.  Bound by double-precision instructions: 34 us at
+// 512^2 with one pixel per thread, 30 us so.
+constexpr int kProbeRows = 8;
+__global__ void __launch_bounds__(128) probe_kernel(int Ny, int Nx, float kmax, double lambda, float k_semi, double C1,
+                                                    double C3, double C5, int smooth, float2* __restrict__ psik,
+                                                    float* __restrict__ aperture) {
+  __shared__ double ky_s[kProbeRows];
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y;
+  const int y0 = blockIdx.y * kProbeRows;
+  if (threadIdx.x < kProbeRows) ky_s[threadIdx.x] = kaxis_exact(y0 + threadIdx.x, Ny, kmax);
+  __syncthreads();
   if (x >= Nx) return;
-  const double k = krad_exact(x, y, Nx, Ny, kmax);
-  const size_t o = (size_t)y * Nx + x;
-  double a;
-  if (smooth) {
-    // 1 / (1 + exp(u)): exactly 1 in double below u = -38, and 0 after rounding to
-    // float32 above u = 104 (the smallest float32 is 1.4e-45), where the phase is
-    // not needed: most of the grid.  The kernel is bound by double-precision
-    // instructions.
-    const double u = -160.0 * ((double)k_semi - k);
-    if (u > 104.0 && isfinite(C1 + C3 + C5)) {
-      psik[o] = make_float2(0.f, 0.f);
-      if (aperture) aperture[o] = 0.f;
-      return;
+  const double kx = kaxis_exact(x, Nx, kmax);
+  const bool finite = isfinite(C1 + C3 + C5);  // else every value is NaN
+  for (int r = 0; r < kProbeRows && y0 + r < Ny; ++r) {
+    const double k = krad_of(kx, ky_s[r]);
+    const size_t o = (size_t)(y0 + r) * Nx + x;
+    double a;
+    bool zero;
+    if (smooth) {
+      // 1 / (1 + exp(u)): exactly 1 in double below u = -38, and 0 after rounding to
+      // float32 above u = 104 (the smallest float32 is 1.4e-45), where the phase is
+      // not needed: most of the grid.
+      const double u = -160.0 * ((double)k_semi - k);
+      zero = u > 104.0;
+      a = zero ? 0.0 : u < -38.0 ? 1.0 : 1.0 / (1.0 + exp(u));
+    } else {
+      a = ((float)k < k_semi) ? 1.0 : 0.0;
+      zero = a == 0.0;
     }
-    a = u < -38.0 ? 1.0 : 1.0 / (1.0 + exp(u));
-  } else {
-    a = ((float)k < k_semi) ? 1.0 : 0.0;
-    if (a == 0.0 && isfinite(C1 + C3 + C5)) {
+    if (zero && finite) {
       psik[o] = make_float2(0.f, 0.f);
-      if (aperture) aperture[o] = 0.f;
-      return;
+    } else {
+      const double kl = k * lambda, kl2 = kl * kl;
+      const double chi = 2.0 * 3.14159265358979323846 / lambda * (-0.5 * C1 * kl2 + 0.25 * C3 * kl2 * kl2 + C5 / 6.0 * kl2 * kl2 * kl2);
+      double sn, cs;
+      sincos(chi, &sn, &cs);
+      psik[o] = make_float2((float)(a * cs), (float)(-a * sn));
     }
+    if (aperture) aperture[o] = (float)a;
   }
-  const double kl = k * lambda, kl2 = kl * kl;
-  const double chi = 2.0 * 3.14159265358979323846 / lambda * (-0.5 * C1 * kl2 + 0.25 * C3 * kl2 * kl2 + C5 / 6.0 * kl2 * kl2 * kl2);
-  double sn, cs;
-  sincos(chi, &sn, &cs);
-  psik[o] = make_float2((float)(a * cs), (float)(-a * sn));
-  if (aperture) aperture[o] = (float)a;
 }
 
 // normalisation = sum |fftshift(ifft2_u(psi_k))|^2 = N * sum |psi_k|^2 (Parseval),
@@ -360,23 +383,34 @@ __global__ void pfac_kernel(int Ny, int Nx, float kmax, double lambda, double sl
     const float inv_n = (float)(1.0 / ((double)Ny * (double)Nx));
     pyx[Ny + i] = make_float2(cs * inv_n, -sn * inv_n);
   }
-  // band of column x: one warp per column, the lanes stride over the rows; the
-  // first and last passing rows are the minimum and maximum over the lanes
+  // Band of column x, one warp per column.  ky rises with y and every step of the
+  // float32 test is monotone in |ky|, so on each side of the centre the passing
+  // rows are those nearest to it: the lanes search 32 ways for the outermost one
+  // (two rounds up to 1024 rows; a test costs a double division and a root):
+  // 19 us with a test of every row at 512^2, 7 us so.
   const int warp = i >> 5, lane = i & 31;
   if (warp < Nx) {
-    int lo = Ny, hi = -1;
-    for (int y = lane; y < Ny; y += 32) {
-      if ((float)krad_exact(warp, y, Nx, Ny, kmax) < k_band) {
-        lo = min(lo, y);
-        hi = max(hi, y);
-      }
-    }
+    const double kx = kaxis_exact(warp, Nx, kmax);
+    auto pass = [&](int y) { return (float)krad_of(kx, kaxis_exact(y, Ny, kmax)) < k_band; };
+    int edge[2];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    for (int side = 0; side < 2; ++side) {
+      const int from = side ? Ny / 2 : (Ny - 1) / 2;  // the centre row of this side
+      const int reach = side ? Ny - 1 - from : from;  // rows from + s, s = 0 .. reach, outwards
+      int good = -1, bad = reach + 1;                 // s = good passes (or -1), s = bad does not (or is past the end)
+      while (bad - good > 1) {
+        const int step = (bad - good + 31) / 32, s = good + 1 + lane * step;
+        const bool ok = s < bad && pass(side ? from + s : from - s);
+        const int n = __popc(__ballot_sync(0xffffffffu, ok));  // the passing lanes come first
+        bad = min(bad, good + 1 + n * step);
+        if (n > 0) good = good + 1 + (n - 1) * step;
+      }
+      edge[side] = good;
     }
-    if (lane == 0) band[warp] = hi < 0 ? make_int2(1, 0) : make_int2(lo, hi);
+    if (lane == 0) {
+      const int lo = edge[0] >= 0 ? (Ny - 1) / 2 - edge[0] : Ny / 2, hi = edge[1] >= 0 ? Ny / 2 + edge[1] : (Ny - 1) / 2;
+      band[warp] = edge[0] < 0 && edge[1] < 0 ? make_int2(1, 0) : make_int2(lo, hi);
+    }
   }
 }
 
@@ -432,7 +466,7 @@ cudaError_t launch_potential(const int4* sites, const int* slice_off, int num_sl
 
 cudaError_t launch_probe(int Ny, int Nx, float kmax, double lambda, float k_semi, double C1, double C3, double C5,
                          int smooth, float2* psik, float* aperture, double* norm, cudaStream_t st) {
-  dim3 grid((Nx + 127) / 128, Ny);
+  dim3 grid((Nx + 127) / 128, (Ny + kProbeRows - 1) / kProbeRows);
   probe_kernel<<<grid, 128, 0, st>>>(Ny, Nx, kmax, lambda, k_semi, C1, C3, C5, smooth, psik, aperture);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || norm == nullptr) return e;
