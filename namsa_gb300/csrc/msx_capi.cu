@@ -219,11 +219,13 @@ int auto_group(int ny, int nx) {
 
 // Schedules a plan starts with, by event timings on GB300 of groups of about
 // 1 GiB at bandwidth 1/3 (us per pass):
-//   rows of 512     paired transform 364, first schedule 374
-//   rows of 768     48 x 16 463, 8 x 8 x 12 515 (228 waves)
-//   columns of 768  48 x 16 279, 8 x 8 x 12 342 in 16-column tiles, 391 in 8-column ones
-//   columns of 384  48 x 8 123, 8 x 8 x 6 149 (400 waves; rows of 384 are
-//                   faster with 8 x 8 x 6: 230 against 239)
+//   rows of 256     in CTAs of four warps 149, of eight 159 (912 waves)
+//   rows of 384     48 x 8 199, 8 x 8 x 6 231 (400 waves)
+//   rows of 512     32 x 16 in CTAs of four warps 355, of eight 365, paired
+//                   transform 364 (512 waves)
+//   rows of 768     48 x 16 422, 8 x 8 x 12 496 (228 waves)
+//   columns of 384  48 x 8 117, 8 x 8 x 6 149
+//   columns of 768  48 x 16 265, 8 x 8 x 12 342 in 16-column tiles, 391 in 8-column ones
 // and the first schedule elsewhere.
 int schedule_index(int n, const char* name) {
   const SchedOps* ops = nullptr;
@@ -233,7 +235,13 @@ int schedule_index(int n, const char* name) {
   return 0;
 }
 int default_row_schedule(int nx) {
-  return nx == 512 ? schedule_index(512, "t32_r16x2x16_pair") : nx == 768 ? schedule_index(768, "t16_r48x16") : 0;
+  switch (nx) {
+    case 256: return schedule_index(256, "t16_r16x16_c8");
+    case 384: return schedule_index(384, "t8_r48x8");
+    case 512: return schedule_index(512, "t16_r32x16_c8");
+    case 768: return schedule_index(768, "t16_r48x16");
+    default: return 0;
+  }
 }
 int default_col_schedule(int ny) {
   return ny == 768 ? schedule_index(768, "t16_r48x16") : ny == 384 ? schedule_index(384, "t8_r48x8") : 0;

@@ -103,34 +103,6 @@ __host__ __device__ constexpr double ce_trig2pi(long m, long R, bool want_sin) {
   return want_sin ? sq : cq;
 }
 
-// v * exp(sign * 2*pi*i * M / R), sign = -1 forward, +1 inverse, M a compile-time constant.
-template <int R, int M, bool INV>
-__host__ __device__ __forceinline__ float2 twc(float2 v) {
-  constexpr int m = ((M % R) + R) % R;
-  if constexpr (m == 0) {
-    return v;
-  } else if constexpr (2 * m == R) {
-    return make_float2(-v.x, -v.y);
-  } else if constexpr (4 * m == R) {           // fwd: -i   inv: +i
-    return INV ? make_float2(-v.y, v.x) : make_float2(v.y, -v.x);
-  } else if constexpr (4 * m == 3 * R) {       // fwd: +i   inv: -i
-    return INV ? make_float2(v.y, -v.x) : make_float2(-v.y, v.x);
-  } else if constexpr ((8 * m) % R == 0) {     // odd multiples of pi/4
-    constexpr float h = 0.70710678118654752440f;
-    constexpr int o = (8 * m) / R;             // 1, 3, 5, 7
-    // e^{-i pi o/4} (fwd) = (cx + i sx)/sqrt2 with the signs below
-    constexpr float cx = (o == 1 || o == 7) ? 1.f : -1.f;
-    constexpr float sxf = (o == 1 || o == 3) ? -1.f : 1.f;  // sign of sin for forward
-    constexpr float sx = INV ? -sxf : sxf;
-    // (a + ib)(cx + i sx) = (a cx - b sx) + i (a sx + b cx)
-    return make_float2(h * (cx * v.x - sx * v.y), h * (sx * v.x + cx * v.y));
-  } else {
-    constexpr float c = (float)ce_trig2pi(m, R, false);
-    constexpr float s = (INV ? 1.f : -1.f) * (float)ce_trig2pi(m, R, true);
-    return make_float2(fmaf(v.x, c, -v.y * s), fmaf(v.x, s, v.y * c));
-  }
-}
-
 // ----------------------------------------------------------------- register DFT codelets
 template <int R, bool INV> struct Dft;
 
@@ -148,16 +120,13 @@ template <bool INV> struct Dft<2, INV> {
 
 template <bool INV> struct Dft<3, INV> {
   static __host__ __device__ __forceinline__ void run(float2 (&v)[3]) {
-    constexpr float s3 = 0.86602540378443864676f;  // sin(2 pi / 3)
-    float2 t1 = cadd(v[1], v[2]);
-    float2 t2 = make_float2(fmaf(-0.5f, t1.x, v[0].x), fmaf(-0.5f, t1.y, v[0].y));
-    float2 h = cscale(csub(v[1], v[2]), s3);
+    constexpr float s3 = (INV ? 1.f : -1.f) * 0.86602540378443864676f;  // s sin(2 pi / 3), s = -1 forward, +1 inverse
+    const float2 t1 = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+    const float2 t2 = caxpy(-0.5f, t1, v[0]);
     v[0] = cadd(v[0], t1);
-    // forward: X1 = t2 - i h, X2 = t2 + i h
-    float2 m1 = make_float2(t2.x + h.y, t2.y - h.x);
-    float2 m2 = make_float2(t2.x - h.y, t2.y + h.x);
-    v[1] = INV ? m2 : m1;
-    v[2] = INV ? m1 : m2;
+    // t2 +- s3 i d
+    v[1] = make_float2(fmaf(-s3, d.y, t2.x), fmaf(s3, d.x, t2.y));
+    v[2] = make_float2(fmaf(s3, d.y, t2.x), fmaf(-s3, d.x, t2.y));
   }
 };
 
@@ -174,44 +143,42 @@ template <bool INV> struct Dft<4, INV> {
   }
 };
 
-// Composite DFT of size A*B by one Cooley-Tukey step in registers:
-// X[ka + A*kb] = sum_b W_B^{b kb} W_{AB}^{b ka} sum_a x[b + B a] W_A^{a ka}.
-template <int A, int B, bool INV, int b, int... ka>
-__host__ __device__ __forceinline__ void ct_twiddle(float2 (&u)[A], float2 (&tmp)[A * B], std::integer_sequence<int, ka...>) {
-  ((tmp[b + B * ka] = twc<A * B, b * ka, INV>(u[ka])), ...);
-}
-template <int A, int B, bool INV, int b>
-__host__ __device__ __forceinline__ void ct_first(float2 (&v)[A * B], float2 (&tmp)[A * B]) {
-  float2 u[A];
-#pragma unroll
-  for (int a = 0; a < A; ++a) u[a] = v[b + B * a];
-  Dft<A, INV>::run(u);
-  ct_twiddle<A, B, INV, b>(u, tmp, std::make_integer_sequence<int, A>{});
-}
-template <int A, int B, bool INV, int... bs>
-__host__ __device__ __forceinline__ void ct_first_all(float2 (&v)[A * B], float2 (&tmp)[A * B], std::integer_sequence<int, bs...>) {
-  (ct_first<A, B, INV, bs>(v, tmp), ...);
+// Composite DFT of size A * B, A and B coprime, by the prime-factor index maps
+// (Good 1958, Thomas 1963): with n = (B na + A nb) mod AB and
+// k = (B (B^-1 mod A) ka + A (A^-1 mod B) kb) mod AB the exponent nk / AB splits
+// into na ka / A + nb kb / B, so no twiddle is left between the two factors.  The
+// maps are compile-time register names.
+constexpr int inverse_mod(int x, int m) {
+  for (int y = 1; y < m; ++y)
+    if ((x * y) % m == 1) return y;
+  return 1;
 }
 template <int A, int B, bool INV>
-__host__ __device__ __forceinline__ void dft_ct(float2 (&v)[A * B]) {
-  float2 tmp[A * B];
-  ct_first_all<A, B, INV>(v, tmp, std::make_integer_sequence<int, B>{});
+__host__ __device__ __forceinline__ void dft_pfa(float2 (&v)[A * B]) {
+  constexpr int N = A * B, ea = B * inverse_mod(B % A, A), eb = A * inverse_mod(A % B, B);
+  float2 tmp[B][A];
+#pragma unroll
+  for (int nb = 0; nb < B; ++nb) {
+#pragma unroll
+    for (int na = 0; na < A; ++na) tmp[nb][na] = v[(B * na + A * nb) % N];
+    Dft<A, INV>::run(tmp[nb]);
+  }
 #pragma unroll
   for (int ka = 0; ka < A; ++ka) {
     float2 w[B];
 #pragma unroll
-    for (int b = 0; b < B; ++b) w[b] = tmp[b + B * ka];
+    for (int nb = 0; nb < B; ++nb) w[nb] = tmp[nb][ka];
     Dft<B, INV>::run(w);
 #pragma unroll
-    for (int kb = 0; kb < B; ++kb) v[ka + A * kb] = w[kb];
+    for (int kb = 0; kb < B; ++kb) v[(ea * ka + eb * kb) % N] = w[kb];
   }
 }
 
 template <bool INV> struct Dft<6, INV> {
-  static __host__ __device__ __forceinline__ void run(float2 (&v)[6]) { dft_ct<2, 3, INV>(v); }
+  static __host__ __device__ __forceinline__ void run(float2 (&v)[6]) { dft_pfa<2, 3, INV>(v); }
 };
 template <bool INV> struct Dft<12, INV> {
-  static __host__ __device__ __forceinline__ void run(float2 (&v)[12]) { dft_ct<4, 3, INV>(v); }
+  static __host__ __device__ __forceinline__ void run(float2 (&v)[12]) { dft_pfa<4, 3, INV>(v); }
 };
 // 16-point DFT as 4 x 4 (X[ka + 4 kb] over inner DFTs of x[b + 4 a]) with the
 // twiddle scales folded into fused multiply-adds.  With s = -1 forward, +1
@@ -303,17 +270,61 @@ template <bool INV> struct Dft<16, INV> {
   static __host__ __device__ __forceinline__ void run(float2 (&v)[16]) { dft16<INV>(v, 1.f); }
 };
 template <bool INV> struct Dft<24, INV> {
-  static __host__ __device__ __forceinline__ void run(float2 (&v)[24]) { dft_ct<8, 3, INV>(v); }
+  static __host__ __device__ __forceinline__ void run(float2 (&v)[24]) { dft_pfa<8, 3, INV>(v); }
 };
-// 48 points as 16 x 3: three 16-point transforms, then sixteen 3-point ones.  A
-// thread that holds 48 values (768 = 48 x 16 with 16 threads, 384 = 48 x 8 with
-// 8) needs one exchange through shared memory where radices 8 x 8 x 12 or
-// 8 x 8 x 6 need two.
+// 48 points as 16 x 3: three 16-point transforms and sixteen 3-point ones, 624
+// operations without twiddles (784 as 16 x 3 with them).  A thread that holds 48
+// values (768 = 48 x 16 with 16 threads, 384 = 48 x 8 with 8) needs one exchange
+// through shared memory where radices 8 x 8 x 12 or 8 x 8 x 6 need two.
 template <bool INV> struct Dft<48, INV> {
-  static __host__ __device__ __forceinline__ void run(float2 (&v)[48]) { dft_ct<16, 3, INV>(v); }
+  static __host__ __device__ __forceinline__ void run(float2 (&v)[48]) { dft_pfa<16, 3, INV>(v); }
 };
+// 32 points as 2 x 16: X_k = E_k + W^k O_k, X_{k+16} = E_k - W^k O_k, the twiddle
+// applied as a scale times (1 + i s t) or (t + i s) with t <= 1 and the scale in
+// the butterfly's FMAs: 380 operations (416 as 4 x 8).  Rounded constants change a
+// transform's norm by the same factor every time, which adds up over the slices:
+// cos(pi/16) lies midway between two floats, and its upper one in three of four
+// places keeps the mean of |X|^2 / (32 |x|^2) - 1 at -3.6e-8, that of a 4 x 8 form
+// with rounded cosines and sines (-4.7e-8 with the lower one everywhere).
+template <bool INV, int K>
+__host__ __device__ __forceinline__ void dft32_pair(float2 e, float2 o, float2& lo, float2& hi) {
+  constexpr float s = INV ? 1.f : -1.f;
+  constexpr double cw = ce_trig2pi(K, 32, false), sw = ce_trig2pi(K, 32, true);  // W_32^K = cw + i s sw, 0 <= K < 16
+  if constexpr (K == 0) {
+    lo = cadd(e, o);
+    hi = csub(e, o);
+  } else if constexpr (K == 8) {
+    const float2 q = make_float2(-s * o.y, s * o.x);
+    lo = cadd(e, q);
+    hi = csub(e, q);
+  } else {
+    constexpr double ac = cw < 0 ? -cw : cw;
+    constexpr bool by_cos = ac >= sw;
+    constexpr float scale = K == 1 || K == 7 || K == 9 ? 0.98078531f : (float)(by_cos ? cw : sw);
+    constexpr float t = (float)(by_cos ? sw / cw : cw / sw);
+    const float2 q = by_cos ? make_float2(fmaf(-s * t, o.y, o.x), fmaf(s * t, o.x, o.y))    // o (1 + i s t)
+                            : make_float2(fmaf(t, o.x, -s * o.y), fmaf(t, o.y, s * o.x));  // o (t + i s)
+    lo = caxpy(scale, q, e);
+    hi = caxpy(-scale, q, e);
+  }
+}
+template <bool INV, int... Ks>
+__host__ __device__ __forceinline__ void dft32_pairs(const float2 (&e)[16], const float2 (&o)[16], float2 (&v)[32],
+                                                     std::integer_sequence<int, Ks...>) {
+  (dft32_pair<INV, Ks>(e[Ks], o[Ks], v[Ks], v[Ks + 16]), ...);
+}
 template <bool INV> struct Dft<32, INV> {
-  static __host__ __device__ __forceinline__ void run(float2 (&v)[32]) { dft_ct<4, 8, INV>(v); }
+  static __host__ __device__ __forceinline__ void run(float2 (&v)[32]) {
+    float2 e[16], o[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      e[j] = v[2 * j];
+      o[j] = v[2 * j + 1];
+    }
+    dft16<INV>(e, 1.f);
+    dft16<INV>(o, 1.f);
+    dft32_pairs<INV>(e, o, v, std::make_integer_sequence<int, 16>{});
+  }
 };
 
 // ----------------------------------------------------------------- shared-memory indexers

@@ -8,6 +8,7 @@ int schedules_256(const SchedOps** out) {
     SchedImpl<Sched<256, 32, 8, 2, 8, 8, 4>>::ops("t32_r8x8x4"),
     SchedImpl<Sched<256, 16, 32, 1, 16, 16>>::ops("t16_r16x16_c32"),
     SchedImpl<Sched<256, 32, 16, 1, 8, 8, 4>>::ops("t32_r8x8x4_c16"),
+    SchedImpl<Sched<256, 16, 8, 4, 16, 16>>::ops("t16_r16x16_c8"),
   };
   *out = table;
   return (int)(sizeof(table) / sizeof(table[0]));

@@ -87,15 +87,18 @@ __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bu
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // Row line inside a staged, densely packed row: element i lives at
-// i ^ ((i >> SH) & 15).  SH = log2(elements per thread) makes the first
-// Stockham scatter (stride E) and the gathers (stride T) conflict-free.
+// i ^ ((i >> SH) & 15) ^ flip.  SH = log2(elements per thread) makes the first
+// Stockham scatter (stride E) and the gathers (stride T) conflict-free; with 48
+// elements SH = 4 does, whose scatter steps (3 t mod 16) are distinct.  With eight
+// threads per line a half warp covers two lines, and flip = 8 in every second
+// one keeps their accesses in different banks.
 template <int SH>
 struct SwizzledLine {
   float2* base;
-  __host__ __device__ __forceinline__ float2& operator[](int i) const { return base[i ^ ((i >> SH) & 15)]; }
+  int flip;
+  __host__ __device__ __forceinline__ float2& operator[](int i) const { return base[(i ^ ((i >> SH) & 15)) ^ flip]; }
 };
-
-__host__ __device__ constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v / 2); }
+__host__ __device__ constexpr int swizzle_shift(int e) { return e == 48 ? 4 : e <= 1 ? 0 : 1 + swizzle_shift(e / 2); }
 
 struct TmaPassArgs {
   float2* psi;            // (Galloc, Ny, Nx) workspace
@@ -220,7 +223,7 @@ __global__ void __launch_bounds__(S::THREADS, S::MINB) row_pass_tma_kernel(TmaPa
       for (int m = 0; m < E; ++m) v[m] = cmul(v[m], trow[t + T * m]);
       PairedFFT512::run<false>(v, la, tw, t);
     } else {
-      SwizzledLine<ilog2(E)> buf{line};
+      const SwizzledLine<swizzle_shift(E)> buf{line, T == 8 ? (lw & 1) * 8 : 0};
       S::FFT::template run<true, false>(v, buf, tw, t);
 #pragma unroll
       for (int m = 0; m < E; ++m) v[m] = cmul(v[m], trow[t + T * m]);
