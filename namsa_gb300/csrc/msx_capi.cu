@@ -10,6 +10,8 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -49,6 +51,17 @@ int schedule_table(int n, const SchedOps** ops) {
     case 768: return schedules_768(ops);
     case 1024: return schedules_1024(ops);
     default: *ops = nullptr; return 0;
+  }
+}
+
+// The all-slices kernel of a grid, or null.
+const StreamOps* stream_ops(int ny, int nx) {
+  switch (nx) {
+    case 256: return stream_ops_256(ny);
+    case 384: return stream_ops_384(ny);
+    case 512: return stream_ops_512(ny);
+    case 768: return stream_ops_768(ny);
+    default: return nullptr;
   }
 }
 
@@ -100,12 +113,20 @@ struct msx_plan {
   std::vector<unsigned char> gkey_host;
   // persistent TMA-pipelined passes
   bool use_tma = true;
+  void* tables = nullptr;        // one allocation behind the small tables:
   int* err = nullptr;            // device error word of the bounded waits
   float2* pyx = nullptr;         // py[ny] then px[nx]
   int2* band = nullptr;          // mask band per column
   CUtensorMap map{};             // workspace as (psi_waves*ny) x nx 8-byte elements, box col_c x col_boxr
   bool map_ok = false;
-  int row_ctas = 0, col_ctas = 0;
+  int row_ctas = 0, col_ctas = 0, sms = 0;
+  // all slices of a group in one kernel (msx_stream.cuh); off while schedules are set by hand
+  const StreamOps* stream = nullptr;
+  bool use_stream = false;
+  CUtensorMap smap{};            // the workspace with the kernel's column tile as box
+  float2* stw_row = nullptr;     // in `tables`, like the counters (2 * kMaxChunks)
+  float2* stw_col = nullptr;
+  int* counters = nullptr;
   float* partial = nullptr;      // detector partial sums
   size_t partial_words = 0;
   float2* inv_n = nullptr;       // constant (1/N, 0) table for CBEDs of real-space waves
@@ -126,14 +147,75 @@ struct msx_plan {
 
 namespace {
 
+constexpr int kMaxChunks = 1024;  // chunks of a group of the all-slices kernel
+
+// A schedule's twiddle table, computed once per process (they are constants; there
+// are as many as compiled schedules).
+const std::vector<float2>& host_twiddles(int words, void (*fill)(float2*)) {
+  static std::mutex m;
+  static std::map<void (*)(float2*), std::vector<float2>> tables;
+  std::lock_guard<std::mutex> lock(m);
+  std::vector<float2>& h = tables[fill];
+  if (h.empty()) {
+    h.resize(words > 0 ? words : 1);
+    fill(h.data());
+  }
+  return h;  // a map's elements stay where they are
+}
+
 int upload_twiddles(const SchedOps& op, float2** dst) {
-  std::vector<float2> h(op.tw_words > 0 ? op.tw_words : 1);
-  op.host_twiddles(h.data());
+  const std::vector<float2>& h = host_twiddles(op.tw_words, op.host_twiddles);
   if (*dst) cudaFree(*dst);
   *dst = nullptr;
   cudaError_t e = cudaMalloc(dst, sizeof(float2) * h.size());
   if (e != cudaSuccess) return fail(MSX_ERR_ALLOC, "twiddle table allocation failed: %s", cudaGetErrorString(e));
   MSX_CUDA(cudaMemcpy(*dst, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice), "twiddle upload");
+  return MSX_OK;
+}
+
+// The propagator table of the plain passes, allocated for the first call that runs
+// them (which may be under a stream capture).
+int ensure_ptab(msx_plan* p) {
+  if (p->ptab) return MSX_OK;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  MSX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+  const cudaError_t e = cudaMalloc(&p->ptab, sizeof(float2) * (size_t)p->ny * p->nx);
+  MSX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    p->ptab = nullptr;
+    return fail(MSX_ERR_ALLOC, "propagator table allocation failed");
+  }
+  return MSX_OK;
+}
+
+// The plan's small tables in one allocation: propagator factors, mask bands, the
+// error word, and the all-slices kernel's counters and twiddles.
+int create_tables(msx_plan* p) {
+  auto round = [](size_t b) { return (b + 255) / 256 * 256; };
+  const size_t pyx = 0, band = pyx + round(sizeof(float2) * (size_t)(p->ny + p->nx));
+  const size_t err = band + round(sizeof(int2) * (size_t)p->nx), counters = err + 256;
+  const size_t rows = counters + (p->stream ? round(sizeof(int) * 2 * kMaxChunks) : 0);
+  const size_t cols = rows + (p->stream ? round(sizeof(float2) * p->stream->twr_words) : 0);
+  const size_t total = cols + (p->stream ? round(sizeof(float2) * p->stream->twc_words) : 0);
+  if (cudaMalloc(&p->tables, total) != cudaSuccess) return fail(MSX_ERR_ALLOC, "plan table allocation failed");
+  char* base = static_cast<char*>(p->tables);
+  p->pyx = reinterpret_cast<float2*>(base + pyx);
+  p->band = reinterpret_cast<int2*>(base + band);
+  p->err = reinterpret_cast<int*>(base + err);
+  MSX_CUDA(cudaMemset(p->err, 0, sizeof(int)), "clearing the plan error word");
+  if (!p->stream) return MSX_OK;
+  p->counters = reinterpret_cast<int*>(base + counters);
+  p->stw_row = reinterpret_cast<float2*>(base + rows);
+  p->stw_col = reinterpret_cast<float2*>(base + cols);
+  const std::vector<float2>& r = host_twiddles(p->stream->twr_words, p->stream->tw_row);
+  const std::vector<float2>& c = host_twiddles(p->stream->twc_words, p->stream->tw_col);
+  std::vector<char> h(total - rows, 0);
+  std::memcpy(h.data(), r.data(), sizeof(float2) * p->stream->twr_words);
+  std::memcpy(h.data() + (cols - rows), c.data(), sizeof(float2) * p->stream->twc_words);
+  MSX_CUDA(cudaMemcpy(base + rows, h.data(), h.size(), cudaMemcpyHostToDevice), "twiddle upload");
+  MSX_CUDA(p->stream->configure(), "configuring the all-slices kernel");
+  p->use_stream = true;
   return MSX_OK;
 }
 
@@ -179,17 +261,22 @@ int prepare_tma(msx_plan* p) {
   if (!enc) return fail(MSX_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
   const cuuint64_t dims[2] = {(cuuint64_t)p->nx, (cuuint64_t)p->psi_waves * p->ny};
   const cuuint64_t strides[1] = {(cuuint64_t)p->nx * sizeof(float2)};
-  const cuuint32_t box[2] = {(cuuint32_t)p->col_ops->col_c, (cuuint32_t)p->col_ops->col_boxr};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(&p->map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, p->psi, dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&](CUtensorMap* map, int c, int boxr) {
+    const cuuint32_t box[2] = {(cuuint32_t)c, (cuuint32_t)boxr};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, p->psi, dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode(&p->map, p->col_ops->col_c, p->col_ops->col_boxr);
+  if (r == CUDA_SUCCESS && p->stream) r = encode(&p->smap, p->stream->col_c, p->stream->col_boxr);
   if (r != CUDA_SUCCESS) return fail(MSX_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
   int sms = 0, rr = 0, cr = 0, dummy = 0;
   MSX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device), "SM count");
   MSX_CUDA(p->row_ops->occupancy(&rr, &dummy), "occupancy");
   MSX_CUDA(p->col_ops->occupancy(&dummy, &cr), "occupancy");
   if (rr < 1 || cr < 1) return fail(MSX_ERR_CUDA, "persistent passes do not fit on an SM");
+  p->sms = sms;
   p->row_ctas = sms * rr;
   p->col_ctas = sms * cr;
   p->map_ok = true;
@@ -284,8 +371,8 @@ void band_columns(int nx, float kmax, float k_band, int C, int* x_lo, int* x_hi)
 // x_lo, x_hi: the column range of the TMA passes (0, 0 = all columns); the
 // plain passes always cover every column.
 int slice_passes(msx_plan* p, const float2* trans_s, int gn, const ColArgs& c, bool with_col, cudaStream_t st,
-                 int x_lo = 0, int x_hi = 0) {
-  if (p->use_tma && p->map_ok) {
+                 int x_lo, int x_hi, bool tma) {
+  if (tma) {
     TmaPassArgs ta{};
     ta.psi = p->psi; ta.trans = trans_s; ta.tw = p->tw_row; ta.pyx = p->pyx; ta.band = p->band; ta.err = p->err;
     ta.G = gn; ta.Ny = p->ny; ta.Nx = p->nx; ta.x_lo = x_lo; ta.x_hi = x_hi;
@@ -333,15 +420,75 @@ int grow(T** buf, size_t* have, size_t words, const char* what) {
   return MSX_OK;
 }
 
+// Whether a call runs through the all-slices kernel, and the waves of its groups.
+// A group is as many waves as stay in L2 (kStreamBytes of their band columns: the
+// row and column tiles read and write nothing else), in equal parts.
+//
+// The line between it and the separate passes, by event timings on GB300 (us per
+// wave and slice, passes / all slices):
+//   512^2  P 1 15.5 / 13.9   8 2.52 / 2.06   16 1.78 / 1.42   64 1.43 / 1.34   128 1.38 / 1.34   1024 1.28 / 1.29
+//   768^2  P 1 39.6 / 30.4   8 6.2 / 5.0     16 4.0 / 3.4     64 3.41 / 3.25
+//   384^2  P 8 2.48 / 2.54   16 1.39 / 1.37  32 1.07 / 0.88   64 0.92 / 0.79
+//   256^2  P 8 1.16 / 1.36   16 0.74 / 0.63  64 0.41 / 0.33   512 0.327 / 0.319
+// The passes gain with long launches (no part-filled last waves of tiles), the
+// kernel's waits between the passes of one wave cost most on short lines.
+constexpr size_t kStreamBytes = (size_t)80 << 20;
+constexpr size_t kStreamMost = (size_t)320 << 20;  // band columns of all waves of a call
+constexpr int kStreamFewShort = 12;                // least positions where a line is shorter than 512
+int stream_group(const msx_plan* p, const MsArgs& a) {
+  if (!p->use_stream || !p->stream || !p->use_tma || !p->map_ok || a.num_slices < 2 || a.num_probes < 1 ||
+      !aligned(a.trans, 16))
+    return 0;
+  if ((p->ny < 512 || p->nx < 512) && a.num_probes < kStreamFewShort) return 0;
+  int lo = 0, hi = 0;
+  band_columns(p->nx, a.kmax, a.k_band, p->stream->col_c, &lo, &hi);
+  const size_t bytes = sizeof(float2) * (size_t)p->ny * (hi - lo);
+  if (bytes * a.num_probes > kStreamMost) return 0;
+  constexpr int unit = 8;  // whole chunks of every instance
+  size_t most = kStreamBytes / bytes / unit * unit;
+  if (most < unit) most = unit;
+  if (most > (size_t)p->stream->wpt * kMaxChunks) most = (size_t)p->stream->wpt * kMaxChunks;
+  const int groups = (int)((a.num_probes + most - 1) / most);
+  int g = ((a.num_probes + groups - 1) / groups + unit - 1) / unit * unit;
+  if (g > a.num_probes) g = a.num_probes;
+  return g <= a.group ? g : 0;
+}
+
+// Slices [s0, s1) of a group of gn waves; `more`: slices follow, so the last one has its column pass.
+int stream_slices(msx_plan* p, const MsArgs& a, int s0, int s1, bool more, int gn, cudaStream_t st) {
+  StreamArgs sa{};
+  sa.psi = p->psi;
+  sa.trans = reinterpret_cast<const float2*>(a.trans) + (size_t)s0 * p->ny * p->nx;
+  sa.tw_row = p->stw_row;
+  sa.tw_col = p->stw_col;
+  sa.pyx = p->pyx;
+  sa.band = p->band;
+  sa.counters = p->counters;
+  sa.err = p->err;
+  sa.first = s0 == 0 ? 1 : 0;
+  band_columns(p->nx, a.kmax, a.k_band, p->stream->col_c, &sa.x_lo, &sa.x_hi);
+  sa.sh = StreamShape{gn, p->stream->wpt, p->stream->ypt, p->ny, (sa.x_hi - sa.x_lo) / p->stream->col_c, s1 - s0, more ? 1 : 0};
+  MSX_CUDA(cudaMemsetAsync(p->counters, 0, sizeof(int) * 2 * sa.sh.chunks(), st), "clearing the tile counters");
+  MSX_CUDA(p->stream->launch(p->smap, sa, p->sms, st), "all-slices kernel");
+  return MSX_OK;
+}
+
 int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const HostPipe* hp = nullptr) {
   const int ny = p->ny, nx = p->nx;
-  const int gmax = a.num_probes < a.group ? a.num_probes : a.group;
+  const int streamed = stream_group(p, a);
+  const int group = streamed ? streamed : a.group;
+  const int gmax = a.num_probes < group ? a.num_probes : group;
   if (!workspace_holds(p, gmax))
     return fail(MSX_ERR_ALLOC, "the plan's workspace does not hold %d waves (an earlier allocation failed)", gmax);
   // the persistent passes form the propagator from its factors and the mask band;
   // the table of N values (26 us of double precision at 512^2, 89 us at 1024^2)
   // serves the plain passes
-  const bool factors = p->use_tma && p->map_ok;
+  const bool tma = p->use_tma && p->map_ok && aligned(a.trans, 16);  // bulk copies start on 16-byte boundaries
+  const bool factors = tma;
+  if (!factors) {
+    const int rc = ensure_ptab(p);
+    if (rc != MSX_OK) return rc;
+  }
   if (factors)
     MSX_CUDA(launch_pfac(ny, nx, a.kmax, a.lambda, a.slice_t, a.k_band, p->pyx, p->band, st), "propagator factors");
   else
@@ -362,11 +509,11 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
              "CBED download");
     return MSX_OK;
   };
-  for (int g0 = 0, gi = 0; g0 < a.num_probes; g0 += a.group, ++gi) {
-    const int gn = (a.num_probes - g0 < a.group) ? a.num_probes - g0 : a.group;
+  for (int g0 = 0, gi = 0; g0 < a.num_probes; g0 += group, ++gi) {
+    const int gn = (a.num_probes - g0 < group) ? a.num_probes - g0 : group;
     ColArgs c{};
     c.psi = p->psi;
-    c.ptab = p->ptab;
+    c.ptab = p->ptab;  // null where the persistent passes run
     c.psik = reinterpret_cast<const float2*>(a.psik);
     c.pos_yx = a.pos + 2 * (size_t)g0;
     c.tw = p->tw_col;
@@ -395,9 +542,16 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
     for (int s = 0; s < a.num_slices; ++s) {
       if (hp && gi == 0 && s % hp->chunk == 0)
         MSX_CUDA(cudaStreamWaitEvent(st, (*hp->chunk_ev)[s / hp->chunk], 0), "cudaStreamWaitEvent");
-      // the first slice covers every column (the probe may reach beyond the band)
-      const int rc = slice_passes(p, trans + (size_t)s * wave, gn, c, s + 1 < a.num_slices, st, s > 0 ? bx_lo : 0,
-                                  s > 0 ? bx_hi : 0);
+      int rc;
+      if (streamed) {  // all slices, or those of one upload
+        const int s0 = s, step = hp && gi == 0 ? hp->chunk : a.num_slices;
+        s = (s0 + step < a.num_slices ? s0 + step : a.num_slices) - 1;
+        rc = stream_slices(p, a, s0, s + 1, s + 1 < a.num_slices, gn, st);
+      } else {
+        // the first slice covers every column (the probe may reach beyond the band)
+        rc = slice_passes(p, trans + (size_t)s * wave, gn, c, s + 1 < a.num_slices, st, s > 0 ? bx_lo : 0,
+                          s > 0 ? bx_hi : 0, tma);
+      }
       if (rc != MSX_OK) return rc;
       if (s + 1 == a.num_slices) {
         ColArgs f = c;
@@ -525,16 +679,10 @@ int msx_plan_create(int ny, int nx, int group, msx_plan** out) {
   p->ny = ny;
   p->nx = nx;
   p->device = device;
+  p->stream = stream_ops(ny, nx);
   int rc = msx_plan_set_schedule(p, default_row_schedule(nx), default_col_schedule(ny),
                                  group > 0 ? group : auto_group(ny, nx));
-  if (rc == MSX_OK) {
-    cudaError_t e = cudaMalloc(&p->ptab, sizeof(float2) * (size_t)ny * nx);
-    if (e == cudaSuccess) e = cudaMalloc(&p->pyx, sizeof(float2) * (size_t)(ny + nx));
-    if (e == cudaSuccess) e = cudaMalloc(&p->band, sizeof(int2) * (size_t)nx);
-    if (e == cudaSuccess) e = cudaMalloc(&p->err, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(p->err, 0, sizeof(int));
-    if (e != cudaSuccess) rc = fail(MSX_ERR_ALLOC, "plan table allocation failed");
-  }
+  if (rc == MSX_OK) rc = create_tables(p);
   if (rc == MSX_OK) {
     cudaError_t e = cudaStreamCreateWithFlags(&p->work, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->ev_in, cudaEventDisableTiming);
@@ -554,9 +702,7 @@ int msx_plan_destroy(msx_plan* p) {
   drop_graph(p);
   if (p->psi) cudaFree(p->psi);
   if (p->ptab) cudaFree(p->ptab);
-  if (p->pyx) cudaFree(p->pyx);
-  if (p->band) cudaFree(p->band);
-  if (p->err) cudaFree(p->err);
+  if (p->tables) cudaFree(p->tables);
   if (p->partial) cudaFree(p->partial);
   if (p->inv_n) cudaFree(p->inv_n);
   if (p->tw_row) cudaFree(p->tw_row);
@@ -590,6 +736,7 @@ int msx_plan_set_schedule(msx_plan* p, int row_schedule, int col_schedule, int g
     rc = upload_twiddles(cops[col_schedule], &p->tw_col);
     if (rc != MSX_OK) return rc;
   }
+  p->use_stream = false;  // schedules set by hand are the passes that run
   p->row_sched = row_schedule;
   p->col_sched = col_schedule;
   p->row_ops = &rops[row_schedule];
@@ -874,7 +1021,7 @@ int msx_multislice_host(msx_plan* p, const float* trans_host, int num_slices, co
   hk.d_cbed = p->io_cbed; hk.normalization = normalization; hk.lambda = lambda; hk.slice_t = slice_t;
   hk.kmax = kmax; hk.k_band = k_band; hk.num_slices = num_slices; hk.num_probes = num_probes; hk.crop_y = crop_y;
   hk.crop_x = crop_x; hk.group = p->group; hk.row_sched = p->row_sched; hk.col_sched = p->col_sched;
-  hk.tma = p->use_tma ? 1 : 0;
+  hk.tma = (p->use_tma ? 1 : 0) + (p->use_stream ? 2 : 0);
   std::vector<unsigned char> key(sizeof(hk));
   std::memcpy(key.data(), &hk, sizeof(hk));
   // everything here follows the caller's earlier work and this plan's earlier calls
@@ -892,10 +1039,18 @@ int msx_multislice_host(msx_plan* p, const float* trans_host, int num_slices, co
     p->gkey_host.clear();
     MSX_CUDA(cudaStreamBeginCapture(w, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
   }
+  MsArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.trans = reinterpret_cast<const float*>(p->io_trans); a.num_slices = num_slices;
+  a.psik = reinterpret_cast<const float*>(p->io_psik); a.norm = p->io_norm; a.pos = p->io_pos;
+  a.num_probes = num_probes; a.kmax = kmax; a.lambda = lambda; a.slice_t = slice_t; a.k_band = k_band;
+  a.cbed = p->io_cbed; a.crop_y = crop_y; a.crop_x = crop_x;
+  a.group = p->group; a.row_sched = p->row_sched; a.col_sched = p->col_sched;
+  const int streamed = stream_group(p, a), step = streamed ? streamed : p->group;
+  const int ngroups = (num_probes + step - 1) / step;
   const int chunk = 8;
   const int nchunks = (num_slices + chunk - 1) / chunk;
-  const int ngroups = (num_probes + p->group - 1) / p->group;
-  std::vector<cudaEvent_t> chunk_ev(nchunks + 1, nullptr), group_ev(ngroups, nullptr);
+  std::vector<cudaEvent_t> chunk_ev(nchunks + 1, nullptr), group_ev;
   auto release = [&]() {  // events still pending are released when they complete
     for (cudaEvent_t e : chunk_ev) if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : group_ev) if (e) cudaEventDestroy(e);
@@ -903,6 +1058,7 @@ int msx_multislice_host(msx_plan* p, const float* trans_host, int num_slices, co
   // everything between the start and the end of a capture: any failure returns
   // through here, so that the capture is always ended
   auto run = [&]() -> int {
+    group_ev.resize(ngroups, nullptr);
     for (auto& e : chunk_ev)
       if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(MSX_ERR_CUDA, "cudaEventCreate");
     for (auto& e : group_ev)
@@ -924,13 +1080,6 @@ int msx_multislice_host(msx_plan* p, const float* trans_host, int num_slices, co
       MSX_CUDA(cudaEventRecord(chunk_ev[i], cp), "cudaEventRecord");
     }
     MSX_CUDA(cudaStreamWaitEvent(w, chunk_ev[nchunks], 0), "cudaStreamWaitEvent");
-    MsArgs a;
-    std::memset(&a, 0, sizeof(a));
-    a.trans = reinterpret_cast<const float*>(p->io_trans); a.num_slices = num_slices;
-    a.psik = reinterpret_cast<const float*>(p->io_psik); a.norm = p->io_norm; a.pos = p->io_pos;
-    a.num_probes = num_probes; a.kmax = kmax; a.lambda = lambda; a.slice_t = slice_t; a.k_band = k_band;
-    a.cbed = p->io_cbed; a.crop_y = crop_y; a.crop_x = crop_x;
-    a.group = p->group; a.row_sched = p->row_sched; a.col_sched = p->col_sched;
     HostPipe hp{cp, chunk, &chunk_ev, &group_ev, cbed_host, pattern};
     int r = enqueue_multislice(p, a, w, &hp);
     if (r != MSX_OK) return r;
@@ -978,6 +1127,8 @@ int msx_plan_profile(msx_plan* p, const float* trans_dev, int num_slices, const 
     return fail(MSX_ERR_ALLOC, "the plan's workspace does not hold %d waves (an earlier allocation failed)", gn);
   const size_t wave = (size_t)ny * nx;
   cudaStream_t st = (cudaStream_t)stream;
+  const int rcp = ensure_ptab(p);
+  if (rcp != MSX_OK) return rcp;
   cudaEvent_t ev[4];
   for (auto& e : ev) MSX_CUDA(cudaEventCreate(&e), "cudaEventCreate");
   MSX_CUDA(launch_ptab(ny, nx, kmax, lambda, slice_t, k_band, p->ptab, st), "propagator table");
@@ -995,7 +1146,7 @@ int msx_plan_profile(msx_plan* p, const float* trans_dev, int num_slices, const 
   for (int i = 0; i < iters; ++i) {
     const int s = i % num_slices;
     MSX_CUDA(cudaEventRecord(ev[0], st), "cudaEventRecord");
-    int rc = slice_passes(p, trans + (size_t)s * wave, gn, c, false, st, bx_lo, bx_hi);
+    int rc = slice_passes(p, trans + (size_t)s * wave, gn, c, false, st, bx_lo, bx_hi, p->use_tma && p->map_ok);
     if (rc != MSX_OK) return rc;
     MSX_CUDA(cudaEventRecord(ev[1], st), "cudaEventRecord");
     if (p->use_tma && p->map_ok) {
@@ -1028,6 +1179,8 @@ int msx_plan_autotune(msx_plan* p, const float* trans_dev, int num_slices, const
   if (!p) return fail(MSX_ERR_INVALID, "null plan");
   if (iters <= 0 || num_slices <= 0 || num_probes <= 0 || !trans_dev || !psi_k_dev || !normalization_dev || !positions_dev)
     return fail(MSX_ERR_INVALID, "autotune needs slices, probes, inputs and iters > 0");
+  const int rcp = ensure_ptab(p);
+  if (rcp != MSX_OK) return rcp;
   const SchedOps *rops, *cops;
   const int nr = schedule_table(p->nx, &rops), nc = schedule_table(p->ny, &cops);
   const size_t wave_bytes = sizeof(float2) * (size_t)p->ny * p->nx;
@@ -1064,7 +1217,8 @@ int msx_plan_autotune(msx_plan* p, const float* trans_dev, int num_slices, const
       MSX_CUDA(cudaEventRecord(e0, st), "cudaEventRecord");
       for (int i = 0; i < iters; ++i) {
         if (row_pass) {
-          const int r2 = slice_passes(p, trans + (size_t)(i % num_slices) * wave, g, c, false, st, bx_lo, bx_hi);
+          const int r2 = slice_passes(p, trans + (size_t)(i % num_slices) * wave, g, c, false, st, bx_lo, bx_hi,
+                                       p->use_tma && p->map_ok);
           if (r2 != MSX_OK) return r2;
         } else if (p->use_tma && p->map_ok) {
           TmaPassArgs ta{};
@@ -1106,10 +1260,42 @@ int msx_plan_autotune(msx_plan* p, const float* trans_dev, int num_slices, const
     const float ns = (best_row + best_col) * 1e6f / ((float)iters * (float)g);
     if (ns < best) { best = ns; br = gr; bc = gc; bg = g; }
   }
+  if (rc == MSX_OK) rc = msx_plan_set_schedule(p, br, bc, bg);
+  if (rc == MSX_OK) {  // the all-slices kernel on the same inputs, where the call would take it
+    MsArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.trans = trans_dev; a.num_slices = num_slices; a.num_probes = num_probes; a.kmax = kmax; a.lambda = lambda;
+    a.slice_t = slice_t; a.k_band = k_band; a.group = p->group;
+    p->use_stream = p->stream != nullptr;
+    const int g = stream_group(p, a), s = num_slices < iters ? num_slices : iters;
+    p->use_stream = false;
+    if (g > 0 && workspace_holds(p, g)) {
+      ColArgs c{};
+      c.psi = p->psi; c.psik = reinterpret_cast<const float2*>(psi_k_dev); c.pos_yx = positions_dev; c.tw = p->tw_col;
+      c.G = g; c.Nx = p->nx; c.kmax = kmax; c.ncols = p->nx;
+      rc = [&]() -> int {
+        MSX_CUDA(p->col_ops->col(COL_INIT, c, st), "probe formation pass");
+        for (int pass = 0; pass < 2; ++pass) {
+          MSX_CUDA(cudaEventRecord(e0, st), "cudaEventRecord");
+          const int r2 = stream_slices(p, a, 0, s, true, g, st);
+          if (r2 != MSX_OK) return r2;
+          MSX_CUDA(cudaEventRecord(e1, st), "cudaEventRecord");
+        }
+        MSX_CUDA(cudaEventSynchronize(e1), "cudaEventSynchronize");
+        float ms = 0;
+        MSX_CUDA(cudaEventElapsedTime(&ms, e0, e1), "cudaEventElapsedTime");
+        const float ns = ms * 1e6f / ((float)s * (float)g);
+        if (ns < best) {
+          best = ns;
+          p->use_stream = true;
+        }
+        return MSX_OK;
+      }();
+    }
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc != MSX_OK) return rc;
-  rc = msx_plan_set_schedule(p, br, bc, bg);
   if (best_ns_per_wave_slice) *best_ns_per_wave_slice = best;
   return rc;
 }
@@ -1133,7 +1319,7 @@ struct msx_batch {
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
   cudaGraphExec_t gexec = nullptr;
   std::vector<unsigned char> gkey;
-  std::vector<std::pair<long long, std::array<int, 3>>> sched;  // (ny<<32|nx) -> row, col, group
+  std::vector<std::pair<long long, std::array<int, 4>>> sched;  // (ny<<32|nx) -> row, col, group, all-slices kernel
 };
 
 namespace {
@@ -1147,10 +1333,10 @@ msx_plan* batch_plan(msx_batch* b, int branch, int ny, int nx, int* rc) {
   int group = (int)(((size_t)1 << 30) / (sizeof(float2) * (size_t)ny * nx));
   if (group < 2) group = 2;
   int r = 0, c = 0;
-  bool tuned = false;  // schedules set for this grid (else the plan's defaults)
+  bool tuned = false, stream = false;  // schedules set for this grid (else the plan's defaults)
   for (auto& kv : b->sched)
     if (kv.first == key) {
-      r = kv.second[0]; c = kv.second[1]; tuned = true;
+      r = kv.second[0]; c = kv.second[1]; tuned = true; stream = kv.second[3] != 0;
       if (kv.second[2] > 0) group = kv.second[2];
     }
   msx_plan* p = nullptr;
@@ -1159,9 +1345,34 @@ msx_plan* batch_plan(msx_batch* b, int branch, int ny, int nx, int* rc) {
   if (tuned) {
     *rc = msx_plan_set_schedule(p, r, c, group);
     if (*rc != MSX_OK) { msx_plan_destroy(p); return nullptr; }
+    p->use_stream = stream && p->stream;
   }
   b->plans[branch].push_back({key, p});
   return p;
+}
+
+int batch_set_schedule(msx_batch* b, int ny, int nx, int row_schedule, int col_schedule, int group, bool stream) {
+  if (!b) return fail(MSX_ERR_INVALID, "null batch");
+  if (!msx_supported_size(ny) || !msx_supported_size(nx)) return fail(MSX_ERR_UNSUPPORTED, "grid %d x %d", ny, nx);
+  if (row_schedule < 0 || row_schedule >= msx_num_schedules(nx) || col_schedule < 0 ||
+      col_schedule >= msx_num_schedules(ny) || group < 0)
+    return fail(MSX_ERR_INVALID, "schedule (%d, %d, group %d) out of range", row_schedule, col_schedule, group);
+  const long long key = ((long long)ny << 32) | (unsigned)nx;
+  bool found = false;
+  for (auto& kv : b->sched)
+    if (kv.first == key) { kv.second = {row_schedule, col_schedule, group, stream}; found = true; }
+  if (!found) b->sched.push_back({key, {row_schedule, col_schedule, group, stream}});
+  for (auto& br : b->plans)
+    for (auto& kv : br)
+      if (kv.first == key) {
+        const int rc = msx_plan_set_schedule(kv.second, row_schedule, col_schedule, group);
+        if (rc != MSX_OK) return rc;
+        kv.second->use_stream = stream && kv.second->stream;
+      }
+  if (b->gexec) cudaGraphExecDestroy(b->gexec);
+  b->gexec = nullptr;
+  b->gkey.clear();
+  return MSX_OK;
 }
 
 }  // namespace
@@ -1209,26 +1420,7 @@ int msx_batch_destroy(msx_batch* b) {
 }
 
 int msx_batch_set_schedule(msx_batch* b, int ny, int nx, int row_schedule, int col_schedule, int group) {
-  if (!b) return fail(MSX_ERR_INVALID, "null batch");
-  if (!msx_supported_size(ny) || !msx_supported_size(nx)) return fail(MSX_ERR_UNSUPPORTED, "grid %d x %d", ny, nx);
-  if (row_schedule < 0 || row_schedule >= msx_num_schedules(nx) || col_schedule < 0 ||
-      col_schedule >= msx_num_schedules(ny) || group < 0)
-    return fail(MSX_ERR_INVALID, "schedule (%d, %d, group %d) out of range", row_schedule, col_schedule, group);
-  const long long key = ((long long)ny << 32) | (unsigned)nx;
-  bool found = false;
-  for (auto& kv : b->sched)
-    if (kv.first == key) { kv.second = {row_schedule, col_schedule, group}; found = true; }
-  if (!found) b->sched.push_back({key, {row_schedule, col_schedule, group}});
-  for (auto& br : b->plans)
-    for (auto& kv : br)
-      if (kv.first == key) {
-        const int rc = msx_plan_set_schedule(kv.second, row_schedule, col_schedule, group);
-        if (rc != MSX_OK) return rc;
-      }
-  if (b->gexec) cudaGraphExecDestroy(b->gexec);
-  b->gexec = nullptr;
-  b->gkey.clear();
-  return MSX_OK;
+  return batch_set_schedule(b, ny, nx, row_schedule, col_schedule, group, false);
 }
 
 int msx_batch_autotune(msx_batch* b, const msx_job* jobs, int njobs, int iters, void* stream) {
@@ -1257,8 +1449,9 @@ int msx_batch_autotune(msx_batch* b, const msx_job* jobs, int njobs, int iters, 
                            stream);
     int row = 0, col = 0, group = 0;
     if (rc == MSX_OK) rc = msx_plan_get_schedule(p, &row, &col, &group);
+    const bool stream = rc == MSX_OK && p->use_stream;
     msx_plan_destroy(p);
-    if (rc == MSX_OK) rc = msx_batch_set_schedule(b, j.ny, j.nx, row, col, group);
+    if (rc == MSX_OK) rc = batch_set_schedule(b, j.ny, j.nx, row, col, group, stream);
     if (rc != MSX_OK) return rc;
   }
   return MSX_OK;
