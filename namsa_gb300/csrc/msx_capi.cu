@@ -122,7 +122,12 @@ struct msx_plan {
   int row_ctas = 0, col_ctas = 0, sms = 0;
   // all slices of a group in one kernel (msx_stream.cuh); off while schedules are set by hand
   const StreamOps* stream = nullptr;
-  bool use_stream = false;
+  bool use_stream = false;       // may take `stream` and `resident`
+  // a wave in the shared memory of a cluster (msx_resident.cuh), small grids
+  const ResidentOps* resident = nullptr;
+  float2* rtw_row = nullptr;     // in `tables`
+  float2* rtw_col = nullptr;
+  int rclusters[3] = {-1, -1, -1}, rclusters_w = -1;  // clusters of kResidentSizes at the same time, for that many band columns
   CUtensorMap smap{};            // the workspace with the kernel's column tile as box
   float2* stw_row = nullptr;     // in `tables`, like the counters (2 * kMaxChunks)
   float2* stw_col = nullptr;
@@ -195,26 +200,45 @@ int create_tables(msx_plan* p) {
   auto round = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t pyx = 0, band = pyx + round(sizeof(float2) * (size_t)(p->ny + p->nx));
   const size_t err = band + round(sizeof(int2) * (size_t)p->nx), counters = err + 256;
-  const size_t rows = counters + (p->stream ? round(sizeof(int) * 2 * kMaxChunks) : 0);
-  const size_t cols = rows + (p->stream ? round(sizeof(float2) * p->stream->twr_words) : 0);
-  const size_t total = cols + (p->stream ? round(sizeof(float2) * p->stream->twc_words) : 0);
+  size_t at = counters + (p->stream ? round(sizeof(int) * 2 * kMaxChunks) : 0);
+  const size_t twiddles = at;
+  std::vector<char> h;
+  auto table = [&](int words, void (*fill)(float2*)) {  // its offset
+    const std::vector<float2>& t = host_twiddles(words, fill);
+    const size_t off = at;
+    at += round(sizeof(float2) * words);
+    h.resize(at - twiddles, 0);
+    std::memcpy(h.data() + (off - twiddles), t.data(), sizeof(float2) * words);
+    return off;
+  };
+  size_t srow = 0, scol = 0, rrow = 0, rcol = 0;
+  if (p->stream) {
+    srow = table(p->stream->twr_words, p->stream->tw_row);
+    scol = table(p->stream->twc_words, p->stream->tw_col);
+  }
+  if (p->resident) {
+    rrow = table(p->resident->twr_words, p->resident->tw_row);
+    rcol = table(p->resident->twc_words, p->resident->tw_col);
+  }
+  const size_t total = at;
   if (cudaMalloc(&p->tables, total) != cudaSuccess) return fail(MSX_ERR_ALLOC, "plan table allocation failed");
   char* base = static_cast<char*>(p->tables);
   p->pyx = reinterpret_cast<float2*>(base + pyx);
   p->band = reinterpret_cast<int2*>(base + band);
   p->err = reinterpret_cast<int*>(base + err);
   MSX_CUDA(cudaMemset(p->err, 0, sizeof(int)), "clearing the plan error word");
-  if (!p->stream) return MSX_OK;
-  p->counters = reinterpret_cast<int*>(base + counters);
-  p->stw_row = reinterpret_cast<float2*>(base + rows);
-  p->stw_col = reinterpret_cast<float2*>(base + cols);
-  const std::vector<float2>& r = host_twiddles(p->stream->twr_words, p->stream->tw_row);
-  const std::vector<float2>& c = host_twiddles(p->stream->twc_words, p->stream->tw_col);
-  std::vector<char> h(total - rows, 0);
-  std::memcpy(h.data(), r.data(), sizeof(float2) * p->stream->twr_words);
-  std::memcpy(h.data() + (cols - rows), c.data(), sizeof(float2) * p->stream->twc_words);
-  MSX_CUDA(cudaMemcpy(base + rows, h.data(), h.size(), cudaMemcpyHostToDevice), "twiddle upload");
-  MSX_CUDA(p->stream->configure(), "configuring the all-slices kernel");
+  if (!h.empty()) MSX_CUDA(cudaMemcpy(base + twiddles, h.data(), h.size(), cudaMemcpyHostToDevice), "twiddle upload");
+  if (p->stream) {
+    p->counters = reinterpret_cast<int*>(base + counters);
+    p->stw_row = reinterpret_cast<float2*>(base + srow);
+    p->stw_col = reinterpret_cast<float2*>(base + scol);
+    MSX_CUDA(p->stream->configure(), "configuring the all-slices kernel");
+  }
+  if (p->resident) {
+    p->rtw_row = reinterpret_cast<float2*>(base + rrow);
+    p->rtw_col = reinterpret_cast<float2*>(base + rcol);
+    MSX_CUDA(p->resident->configure(), "configuring the cluster-resident kernel");
+  }
   p->use_stream = true;
   return MSX_OK;
 }
@@ -424,26 +448,37 @@ int grow(T** buf, size_t* have, size_t words, const char* what) {
 // A group is as many waves as stay in L2 (kStreamBytes of their band columns: the
 // row and column tiles read and write nothing else), in equal parts.
 //
-// The line between it and the separate passes, by event timings on GB300 (us per
-// wave and slice, passes / all slices):
-//   512^2  P 1 15.5 / 13.9   8 2.52 / 2.06   16 1.78 / 1.42   64 1.43 / 1.34   128 1.38 / 1.34   1024 1.28 / 1.29
-//   768^2  P 1 39.6 / 30.4   8 6.2 / 5.0     16 4.0 / 3.4     64 3.41 / 3.25
-//   384^2  P 8 2.48 / 2.54   16 1.39 / 1.37  32 1.07 / 0.88   64 0.92 / 0.79
-//   256^2  P 8 1.16 / 1.36   16 0.74 / 0.63  64 0.41 / 0.33   512 0.327 / 0.319
-// The passes gain with long launches (no part-filled last waves of tiles), the
-// kernel's waits between the passes of one wave cost most on short lines.
+// The line between it and the separate passes is that of event timings on GB300
+// of every pair of its line lengths from 1 to 512 positions (24 slices, bandwidth
+// 1/3): from `few` positions on, and up to `most` MB of band columns of all
+// waves, it was the faster one.  The passes gain with long launches (no
+// part-filled last waves of tiles); the kernel's waits between the passes of one
+// wave cost most on short lines.  Passes / all slices, us, at 1, 16, 64, 256 positions:
+//   256 x 256   226/235   303/274   650/530    2133/2005
+//   384 x 384   473/461   567/545   1442/1243  5203/4855
+//   512 x 512   388/358   706/569   2256/2103  8359/8271
+//   768 x 768   972/729   1574/1259 5123/4917  (128: 9626/10078)
+//   768 x 256   399/371   646/555   1809/1835  6098/7289
+//   256 x 768   414/336   597/530   1796/1712  6515/6762
 constexpr size_t kStreamBytes = (size_t)80 << 20;
-constexpr size_t kStreamMost = (size_t)320 << 20;  // band columns of all waves of a call
-constexpr int kStreamFewShort = 12;                // least positions where a line is shorter than 512
+struct StreamRange {
+  int few, most;
+};
+constexpr StreamRange kStreamRange[4][4] = {  // [ny][nx], lines of 256, 384, 512, 768
+    {{12, 180}, {24, 130}, {12, 60}, {1, 130}},
+    {{24, 36}, {16, 400}, {12, 130}, {1, 300}},
+    {{8, 60}, {1, 500}, {1, 360}, {1, 500}},
+    {{1, 36}, {1, 300}, {1, 380}, {1, 310}}};
 int stream_group(const msx_plan* p, const MsArgs& a) {
   if (!p->use_stream || !p->stream || !p->use_tma || !p->map_ok || a.num_slices < 2 || a.num_probes < 1 ||
       !aligned(a.trans, 16))
     return 0;
-  if ((p->ny < 512 || p->nx < 512) && a.num_probes < kStreamFewShort) return 0;
+  auto line = [](int n) { return n == 256 ? 0 : n == 384 ? 1 : n == 512 ? 2 : 3; };
+  const StreamRange range = kStreamRange[line(p->ny)][line(p->nx)];
   int lo = 0, hi = 0;
   band_columns(p->nx, a.kmax, a.k_band, p->stream->col_c, &lo, &hi);
   const size_t bytes = sizeof(float2) * (size_t)p->ny * (hi - lo);
-  if (bytes * a.num_probes > kStreamMost) return 0;
+  if (a.num_probes < range.few || bytes * a.num_probes > ((size_t)range.most << 20)) return 0;
   constexpr int unit = 8;  // whole chunks of every instance
   size_t most = kStreamBytes / bytes / unit * unit;
   if (most < unit) most = unit;
@@ -452,6 +487,38 @@ int stream_group(const msx_plan* p, const MsArgs& a) {
   int g = ((a.num_probes + groups - 1) / groups + unit - 1) / unit * unit;
   if (g > a.num_probes) g = a.num_probes;
   return g <= a.group ? g : 0;
+}
+
+// Whether a call keeps each wave in a cluster, and the CTAs of a cluster: as many as
+// let all positions run at the same time (more CTAs shorten a slice).  Event
+// timings on GB300, us per slice in the passes / clusters of 16 / 8 / 4:
+//   256^2      P 1 8.7 / 6.0 / 10.0 / -     8 9.3 / 11.4 / 10.0 / -
+//   128 x 256  P 1 7.8 / 5.1 / 5.7 / 10.0   8 8.4 / 9.4 / 5.7 / 9.9   32 11.5 / 22 / 16 / 10.0
+//   128^2      P 4 8.9 / 5.1 / 5.0 / 6.1   16 9.3 / 14 / 8.9 / 6.1   64 13.2 / 43 / 21 / 11.5
+//   64^2       P 1 6.4 / 3.6 / 3.1 / 3.2   64 7.6 / 31 / 14 / 5.7   128 9.1 / 58 / 24 / 10.9
+// so 16 only above 128^2, fewer only below 256^2, and the smallest grids take up
+// to two rounds of clusters of four.
+constexpr int kResidentSizes[3] = {16, 8, 4};
+int resident_cluster(msx_plan* p, const MsArgs& a) {
+  if (!p->use_stream || !p->resident || !p->use_tma || !p->map_ok || a.det || a.num_slices < 2 || a.num_probes < 1 ||
+      a.num_probes > a.group || !aligned(a.trans, 16))
+    return 0;
+  int lo = 0, hi = 0;
+  band_columns(p->nx, a.kmax, a.k_band, 1, &lo, &hi);
+  if (p->rclusters_w != hi - lo) {
+    for (int i = 0; i < 3; ++i)
+      if (p->resident->clusters(hi - lo, kResidentSizes[i], &p->rclusters[i]) != cudaSuccess) {
+        cudaGetLastError();
+        p->rclusters[i] = 0;
+      }
+    p->rclusters_w = hi - lo;
+  }
+  const int area = p->ny * p->nx;
+  if (area > 128 * 128 && a.num_probes <= p->rclusters[0]) return kResidentSizes[0];
+  if (area >= 256 * 256) return 0;
+  if (a.num_probes <= p->rclusters[1]) return kResidentSizes[1];
+  if (a.num_probes <= (area <= 128 * 128 ? 2 : 1) * p->rclusters[2]) return kResidentSizes[2];
+  return 0;
 }
 
 // Slices [s0, s1) of a group of gn waves; `more`: slices follow, so the last one has its column pass.
@@ -473,9 +540,18 @@ int stream_slices(msx_plan* p, const MsArgs& a, int s0, int s1, bool more, int g
   return MSX_OK;
 }
 
+// A call of so few launches that issuing them costs less than recording a graph
+// for every new set of buffers (an output allocated by the caller is one).
+bool few_launches(msx_plan* p, const MsArgs& a) {
+  if (resident_cluster(p, a)) return true;
+  const int g = stream_group(p, a);
+  return g > 0 && a.num_probes <= 2 * g;
+}
+
 int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const HostPipe* hp = nullptr) {
   const int ny = p->ny, nx = p->nx;
-  const int streamed = stream_group(p, a);
+  const int cluster = resident_cluster(p, a);
+  const int streamed = cluster ? 0 : stream_group(p, a);
   const int group = streamed ? streamed : a.group;
   const int gmax = a.num_probes < group ? a.num_probes : group;
   if (!workspace_holds(p, gmax))
@@ -539,6 +615,20 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
     c.x_begin = 0;
     c.ncols = nx;
     MSX_CUDA(p->col_ops->col(COL_INIT, c, st), "probe formation pass");
+    if (cluster) {  // one group: every position
+      if (hp)
+        for (int i = 0; i * hp->chunk < a.num_slices; ++i)
+          MSX_CUDA(cudaStreamWaitEvent(st, (*hp->chunk_ev)[i], 0), "cudaStreamWaitEvent");
+      ResidentArgs ra{};
+      ra.psi = p->psi; ra.trans = trans; ra.tw_row = p->rtw_row; ra.tw_col = p->rtw_col; ra.pyx = p->pyx;
+      ra.band = p->band; ra.norm = a.norm; ra.cbed = c.cbed; ra.err = p->err; ra.slices = a.num_slices;
+      band_columns(nx, a.kmax, a.k_band, 1, &ra.x_lo, &ra.x_hi);
+      ra.x0 = x0; ra.y0 = y0; ra.crop_y = a.crop_y; ra.crop_x = a.crop_x;
+      MSX_CUDA(p->resident->launch(ra, gn, cluster, st), "cluster-resident kernel");
+      const int rc = hand_off(gi, g0, gn);
+      if (rc != MSX_OK) return rc;
+      continue;
+    }
     for (int s = 0; s < a.num_slices; ++s) {
       if (hp && gi == 0 && s % hp->chunk == 0)
         MSX_CUDA(cudaStreamWaitEvent(st, (*hp->chunk_ev)[s / hp->chunk], 0), "cudaStreamWaitEvent");
@@ -680,6 +770,7 @@ int msx_plan_create(int ny, int nx, int group, msx_plan** out) {
   p->nx = nx;
   p->device = device;
   p->stream = stream_ops(ny, nx);
+  p->resident = resident_ops(ny, nx);
   int rc = msx_plan_set_schedule(p, default_row_schedule(nx), default_col_schedule(ny),
                                  group > 0 ? group : auto_group(ny, nx));
   if (rc == MSX_OK) rc = create_tables(p);
@@ -825,6 +916,13 @@ int msx_multislice(msx_plan* p, const float* trans_dev, int num_slices, const fl
   // Run on the plan's stream, ordered after and before the caller's stream.
   MSX_CUDA(cudaEventRecord(p->ev_in, caller), "cudaEventRecord");
   MSX_CUDA(cudaStreamWaitEvent(p->work, p->ev_in, 0), "cudaStreamWaitEvent");
+  if (few_launches(p, a)) {
+    const int rc = enqueue_multislice(p, a, p->work);
+    if (rc != MSX_OK) return rc;
+    MSX_CUDA(cudaEventRecord(p->ev_out, p->work), "cudaEventRecord");
+    MSX_CUDA(cudaStreamWaitEvent(caller, p->ev_out, 0), "cudaStreamWaitEvent");
+    return MSX_OK;
+  }
   std::vector<unsigned char> key(sizeof(MsArgs));
   std::memcpy(key.data(), &a, sizeof(MsArgs));
   if (!p->gexec || key != p->gkey) {
@@ -1046,7 +1144,7 @@ int msx_multislice_host(msx_plan* p, const float* trans_host, int num_slices, co
   a.num_probes = num_probes; a.kmax = kmax; a.lambda = lambda; a.slice_t = slice_t; a.k_band = k_band;
   a.cbed = p->io_cbed; a.crop_y = crop_y; a.crop_x = crop_x;
   a.group = p->group; a.row_sched = p->row_sched; a.col_sched = p->col_sched;
-  const int streamed = stream_group(p, a), step = streamed ? streamed : p->group;
+  const int streamed = resident_cluster(p, a) ? 0 : stream_group(p, a), step = streamed ? streamed : p->group;
   const int ngroups = (num_probes + step - 1) / step;
   const int chunk = 8;
   const int nchunks = (num_slices + chunk - 1) / chunk;

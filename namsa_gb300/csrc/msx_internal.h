@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "msx_sched.cuh"
+#include "msx_resident.cuh"
 #include "msx_stream.cuh"
 
 namespace msx {

@@ -46,8 +46,8 @@ def rel(a, b):
 
 # every pair of line lengths; waves that fill a chunk, spill into the next or stay below one;
 # two slices (the smallest) and more
-SHAPES = [(256, 256, 3, 12), (256, 256, 2, 50), (384, 384, 3, 13), (512, 512, 3, 1), (512, 512, 2, 3), (512, 512, 4, 17),
-          (768, 768, 2, 1), (768, 768, 3, 9), (256, 384, 3, 15), (384, 256, 3, 12), (256, 512, 3, 13), (512, 256, 2, 17),
+SHAPES = [(256, 256, 3, 12), (256, 256, 2, 50), (384, 384, 3, 17), (512, 512, 3, 1), (512, 512, 2, 3), (512, 512, 4, 17),
+          (768, 768, 2, 1), (768, 768, 3, 9), (256, 384, 3, 25), (384, 256, 3, 27), (256, 512, 3, 13), (512, 256, 2, 17),
           (256, 768, 2, 12), (768, 256, 2, 13), (384, 512, 3, 12), (512, 384, 2, 14), (384, 768, 2, 21),
           (768, 384, 2, 12), (512, 768, 2, 3), (768, 512, 3, 2)]
 
