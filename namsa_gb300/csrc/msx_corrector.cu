@@ -40,10 +40,19 @@ __device__ __forceinline__ float gelu_d(float z) {
   return 0.5f * (1.f + th) + 0.5f * z * (1.f - th * th) * k * (1.f + 3.f * 0.044715f * z * z);
 }
 
-__global__ void gelu_bwd_kernel(const float* __restrict__ da, const float* __restrict__ z, long long n,
-                                float* __restrict__ dz) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dz[i] = da[i] * gelu_d(z[i]);
+// V = 4: four values per thread in 16-byte accesses (n / 4 threads; aligned arrays).
+// Memory-bound: 805 MB at 32 x 256^2 x 32 in 115 us (7.0 TB/s), 224 us one value a thread.
+template <int V>
+__global__ void gelu_bwd_kernel(const float* da, const float* z, long long n, float* dz) {  // dz may be da
+  const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * V;
+  if (i >= n) return;
+  if constexpr (V == 4) {
+    const float4 d = *reinterpret_cast<const float4*>(da + i), v = *reinterpret_cast<const float4*>(z + i);
+    *reinterpret_cast<float4*>(dz + i) =
+        make_float4(d.x * gelu_d(v.x), d.y * gelu_d(v.y), d.z * gelu_d(v.z), d.w * gelu_d(v.w));
+  } else {
+    dz[i] = da[i] * gelu_d(z[i]);
+  }
 }
 
 // Column sums of a (rows x n) row-major matrix, first stage: part[chunk][c] over
@@ -384,6 +393,13 @@ int forward(msx_corrector* k, int S, cudaStream_t st) {
   return MSX_OK;
 }
 
+// dz = da * gelu'(z) over n values.  Layers lie n values apart, so an n that is no
+// multiple of 4 (odd grids with few channels) leaves them unaligned.
+void gelu_bwd(const float* da, const float* z, size_t n, float* dz, cudaStream_t st) {
+  if (n % 4 == 0) gelu_bwd_kernel<4><<<blocks_for((long long)(n / 4), 256), 256, 0, st>>>(da, z, (long long)n, dz);
+  else gelu_bwd_kernel<1><<<blocks_for((long long)n, 256), 256, 0, st>>>(da, z, (long long)n, dz);
+}
+
 int backward(msx_corrector* k, const float* dmaps, cudaStream_t st) {
   const int S = k->S_last;
   const long long SP = (long long)S * k->P;
@@ -396,7 +412,7 @@ int backward(msx_corrector* k, const float* dmaps, cudaStream_t st) {
   if ((rc = wgrad(k, dmaps, 4, k->h, C, S, G + k->oP2, st))) return rc;
   if ((rc = colsum(k, dmaps, SP, 4, G + k->oc2, st))) return rc;
   NN_GEMM(k->gemm.run(dmaps, rowmajor(4), Pm + k->oP2, colmajor(C), SP, C, 4, epi(k->dz, rowmajor(C)), st));
-  gelu_bwd_kernel<<<blocks_for((long long)A, 256), 256, 0, st>>>(k->dz, k->zh, (long long)A, k->dz);
+  gelu_bwd(k->dz, k->zh, A, k->dz, st);
   if ((rc = wgrad(k, k->dz, C, k->a + (size_t)k->L * A, C, S, G + k->oP1, st))) return rc;
   if ((rc = colsum(k, k->dz, SP, C, G + k->oc1, st))) return rc;
   NN_GEMM(k->gemm.run(k->dz, rowmajor(C), Pm + k->oP1, colmajor(C), SP, C, C, epi(k->da, rowmajor(C)), st));
@@ -404,7 +420,7 @@ int backward(msx_corrector* k, const float* dmaps, cudaStream_t st) {
     const float* ain = k->a + (size_t)l * A;
     const float* zl = k->z + (size_t)l * A;
     const float* Xl = k->Xh + (size_t)l * x_words(k, S);
-    gelu_bwd_kernel<<<blocks_for((long long)A, 256), 256, 0, st>>>(k->da, zl, (long long)A, k->dz);
+    gelu_bwd(k->da, zl, A, k->dz, st);
     NN_CUDA(cudaGetLastError());
     if ((rc = wgrad(k, k->dz, C, ain, C, S, G + k->oW[l], st))) return rc;
     if ((rc = colsum(k, k->dz, SP, C, G + k->ob[l], st))) return rc;

@@ -367,8 +367,10 @@ namespace ws {
 constexpr int LOADERS = 128;  // warps 0-3
 constexpr int EPI_WARPS = 8;  // warps 4-11
 constexpr int MMA_WARP = 12;
-constexpr int THREADS = 13 * 32;
+constexpr int THREADS = 16 * 32;  // warps 13-15 idle: registers move between groups of four warps
 constexpr int SLOT_FLOATS = BM * BK;  // one FP32 staging slot (32 KB)
+constexpr int EPI_LD = 36;                // row stride of a warp's 32 x 32 block: 16-byte aligned, conflict-free
+constexpr int EPI_BLOCK = 32 * EPI_LD;
 template <int BN>
 struct Cfg {
   static constexpr int STAGES = BN == 256 ? 2 : 3;  // bfloat16 operand stages
@@ -377,7 +379,7 @@ struct Cfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int BROWS = BN;                          // rows of a B tile
   static constexpr int BSLOT_FLOATS = BN == 32 ? 32 * BK : 0;  // FP32 B staging slot (B from FP32: BN = 32)
-  static constexpr int EPI_FLOATS = EPI_WARPS * 32 * 33;
+  static constexpr int EPI_FLOATS = EPI_WARPS * EPI_BLOCK;
   static constexpr int SMEM =
       STAGES * STAGE_BYTES + DEPTH * (SLOT_FLOATS + BSLOT_FLOATS) * 4 + EPI_FLOATS * 4 + 1024;
   static constexpr uint32_t TMEM_COLS = 2 * BN;
@@ -385,6 +387,9 @@ struct Cfg {
 
 __device__ __forceinline__ void cp4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 // the barrier's phase completes (for this thread's arrival) once this thread's copies have landed
 __device__ __forceinline__ void cp_arrive(uint64_t* bar) {
@@ -402,12 +407,54 @@ __device__ __forceinline__ bool loaders_all(bool ok) {
 }
 __device__ __forceinline__ void loaders_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-__device__ __forceinline__ void store_chunk(uint8_t* sa, int row, int ch, const float (&x)[8]) {
+// eight values as bfloat16 to a 16-byte chunk of an operand stage
+__device__ __forceinline__ void put_chunk(uint8_t* dst, const float (&x)[8]) {
   __align__(16) __nv_bfloat162 h[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
-  *reinterpret_cast<uint4*>(sa + sw128(row, ch * 8)) = *reinterpret_cast<const uint4*>(h);
+  *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(h);
 }
+
+// mbar_wait_bounded with the clock read only when the phase has not completed yet
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity) {
+  return mbar_try_wait(bar, parity) || mbar_wait_bounded(bar, parity);
+}
+
+// A cursor over a CTA's items (batch, split, mt, nt), nt fastest: one step is `step`
+// items, split once into its four digits, so that moving on takes carries and no division.
+struct Walk {
+  long long it;
+  int bt, split, mt, nt;
+  int d_bt, d_split, d_mt, d_nt;
+  __device__ __forceinline__ void digits(long long v, int ntiles, int mtiles, int splits, int& bt_, int& split_, int& mt_,
+                                         int& nt_) {
+    long long q = v / ntiles;
+    nt_ = (int)(v - q * ntiles);
+    v = q / mtiles;
+    mt_ = (int)(q - v * mtiles);
+    q = v / splits;
+    split_ = (int)(v - q * splits);
+    bt_ = (int)q;
+  }
+  __device__ __forceinline__ void start(long long first, long long step, int ntiles, int mtiles, int splits) {
+    it = first;
+    digits(first, ntiles, mtiles, splits, bt, split, mt, nt);
+    digits(step, ntiles, mtiles, splits, d_bt, d_split, d_mt, d_nt);
+  }
+  __device__ __forceinline__ void next(long long step, int ntiles, int mtiles, int splits) {
+    it += step;
+    nt += d_nt;
+    const int c0 = nt >= ntiles;
+    nt -= c0 ? ntiles : 0;
+    mt += d_mt + c0;
+    const int c1 = mt >= mtiles;
+    mt -= c1 ? mtiles : 0;
+    split += d_split + c1;
+    const int c2 = split >= splits;
+    split -= c2 ? splits : 0;
+    bt += d_bt + c2;
+  }
+};
 
 // How the rows r0 .. r0 + R - 1 of an operand (R = 128 for A, BN for B), K block kb
 // (nk = min(64, K - 64 kb) values), reach a staging slot:
@@ -416,15 +463,24 @@ __device__ __forceinline__ void store_chunk(uint8_t* sa, int row, int ch, const 
 //   GROUPRUN rows contiguous in groups of rc with k stride rc (a group's K block is one
 //            run of nk * rc values; rc may be all the operand's rows): thread i < R / rc
 //            copies group i to slot[i * 64 rc ..], element (k, r mod rc) at k rc + r mod rc;
-//   GENERIC  thread i copies row r0 + i value by value (4-byte asynchronous copies),
-//            element (r, k) at ((k / 8) R + i) 8 + k mod 8;
+//   PIECES   rows contiguous in groups of rc at any k stride, each with its kc = 1 or 2
+//            neighbouring k values: 16-byte asynchronous copies dealt over all threads,
+//            group i to slot[i * 64 rc ..], element (k, r mod rc) at
+//            ((k / kc) rc + r mod rc) kc + k mod kc (GROUPRUN's layout for kc = 1);
+//   GENERIC  value by value (4-byte asynchronous copies), a row's values dealt over the
+//            threads that have no row of their own, element (r, k) at ((k / 8) R + i) 8 + k mod 8;
 //   TILERUN  rows of K <= 64 values stored back to back: thread 0 copies the tile's rows
 //            as one run (or the loaders load it, when the run is not 16-byte aligned),
 //            element (r, k) at r K + k.
 // Bulk bytes are announced on the slot's barrier without arriving; each loader thread
 // arrives once per slot after its copies of A and B are issued (through the async-copy
-// unit when it issued 4-byte copies, so the arrival waits for them).
-enum { ROWRUN = 0, GROUPRUN = 1, GENERIC = 2, TILERUN = 3 };
+// unit when it issued asynchronous copies, so the arrival waits for them).
+//
+// The loaders are one warp per scheduler, so a block costs them the length of their
+// instruction chain and hardly anything else: offsets are hoisted, steps are additions
+// and shifts, and four chunks are read before the first is stored.
+enum { ANY = -1, ROWRUN = 0, GROUPRUN = 1, GENERIC = 2, TILERUN = 3, PIECES = 4 };
+template <int V> using Tag = std::integral_constant<int, V>;
 
 __device__ __forceinline__ void expect_tx_only(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
@@ -435,7 +491,7 @@ struct Op {
   Addr a;
   long long bs;    // batch stride (floats)
   long long rows;  // M or N
-  int mode, rc;
+  int mode, rc;    // rc: rows of a group (GROUPRUN, PIECES)
 };
 
 __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total) {
@@ -447,26 +503,44 @@ __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total)
     if (a.rc == 1 && k_total <= BK && a.s1 == k_total) o.mode = TILERUN;
     return;
   }
+  const bool aligned = o.bs % 4 == 0 && (reinterpret_cast<uintptr_t>(o.p) & 15u) == 0;
   long long g = -1;
   if (a.s2 == 1 && a.rc > 1) g = a.rc;
   else if (a.rc == 1 && a.s1 == 1) g = o.rows;  // all rows contiguous
-  if (g > 0 && g <= tile_rows && a.kc == 1 && a.t1 == g && g % 4 == 0 && tile_rows % g == 0 && o.rows % g == 0 &&
-      (g == o.rows || a.s1 % 4 == 0) && o.bs % 4 == 0 && (reinterpret_cast<uintptr_t>(o.p) & 15u) == 0) {
+  // one group may be of any size as long as its K blocks are whole 16-byte pieces
+  const bool one = g == o.rows && (k_total % BK) * g % 4 == 0;
+  if (g > 0 && g <= tile_rows && a.kc == 1 && a.t1 == g && (one || (g % 4 == 0 && tile_rows % g == 0)) &&
+      o.rows % g == 0 && (g == o.rows || a.s1 % 4 == 0) && aligned) {
     o.mode = GROUPRUN;
     o.rc = (int)g;
+    return;
+  }
+  // groups that divide the tile or are divided by it
+  const bool pair = a.kc == 2 && a.t2 == 1 && a.s2 == 2 && a.rc > 1;
+  if (pair) g = a.rc;
+  if (g > 0 && (pair || a.kc == 1) && aligned && a.t1 % 4 == 0 && k_total % a.kc == 0 && o.rows % g == 0 &&
+      (g == o.rows || a.s1 % 4 == 0)) {
+    const long long in = g < tile_rows ? g : tile_rows;
+    if (in * a.kc % 4 == 0 && tile_rows % in == 0 && g % in == 0) {
+      o.mode = PIECES;
+      o.rc = (int)in;
+    }
   }
 }
 
-// Thread i's copies of rows r0 .. r0 + R - 1 of operand o (batch bt) into slot stg;
-// returns true when it issued 4-byte asynchronous copies.
-template <int R>
-__device__ __forceinline__ bool issue_op(float* stg, uint64_t* bar, const Op& o, long long bt, long long K,
-                                         long long r0, int kb, int i) {
+// The loader threads' copies of rows r0 .. r0 + R - 1 of operand o (batch bt) into slot
+// stg; true when this thread issued asynchronous (non-bulk) copies.
+template <int R, int MODE>
+__device__ __forceinline__ bool issue_op(float* stg, uint64_t* bar, const Op& o, int bt, long long K, long long r0,
+                                         int kb, int i) {
   const long long kb0 = (long long)kb * BK;
   const int nk = (int)(K - kb0 < BK ? K - kb0 : BK);
   const float* const P = o.p + bt * o.bs;
   const Addr& a = o.a;
-  if (o.mode == TILERUN) {
+  const int mode = MODE == ANY ? o.mode : MODE;
+  // offset of row r; operands with one row stride need no division
+  auto row_off = [&](long long r) { return a.rc == 1 ? r * a.s1 : (r / a.rc) * a.s1 + (r % a.rc) * a.s2; };
+  if (mode == TILERUN) {
     const long long nrow = o.rows - r0 < R ? o.rows - r0 : R;
     const float* src = P + r0 * a.s1;
     const int n = (int)(nrow * nk);
@@ -480,11 +554,10 @@ __device__ __forceinline__ bool issue_op(float* stg, uint64_t* bar, const Op& o,
     }
     return false;
   }
-  if (i >= R && o.mode != GROUPRUN) return false;
-  if (o.mode == ROWRUN) {
+  if (mode == ROWRUN) {
     const long long r = r0 + i;
-    if (r < o.rows) {
-      const float* src = P + (r / a.rc) * a.s1 + (r % a.rc) * a.s2 + kb0;
+    if (i < R && r < o.rows) {
+      const float* src = P + row_off(r) + kb0;
       if ((nk & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
         expect_tx_only(bar, (uint32_t)nk * 4u);
         bulk_g2s(stg + i * BK, src, (uint32_t)nk * 4u, bar);
@@ -494,30 +567,70 @@ __device__ __forceinline__ bool issue_op(float* stg, uint64_t* bar, const Op& o,
     }
     return false;
   }
-  if (o.mode == GROUPRUN) {
+  if (mode == GROUPRUN) {
     const int rc = o.rc;
     const long long r = r0 + (long long)i * rc;
-    if (i < R / rc && r < o.rows) {
+    if (i * rc < R && r < o.rows) {
       const uint32_t bytes = (uint32_t)nk * (uint32_t)rc * 4u;
       expect_tx_only(bar, bytes);
-      bulk_g2s(stg + i * BK * rc, P + (r / a.rc) * a.s1 + kb0 * a.t1, bytes, bar);
+      bulk_g2s(stg + i * BK * rc, P + row_off(r) + kb0 * a.t1, bytes, bar);
     }
     return false;
   }
-  const long long r = r0 + i;
-  if (r >= o.rows) return false;
-  const float* row = P + (r / a.rc) * a.s1 + (r % a.rc) * a.s2;
-  long long q = kb0 / a.kc, rem = kb0 - q * a.kc;
-  for (int k = 0; k < nk; ++k) {
-    cp4(stg + ((k >> 3) * R + i) * 8 + (k & 7), row + q * a.t1 + rem * a.t2);
-    if (++rem == a.kc) { rem = 0; ++q; }
+  if (mode == PIECES) {
+    const int rc = o.rc, run = (rc * (int)a.kc) >> 2;  // 16-byte pieces of a run
+    const int ks = a.kc == 2 ? 1 : 0;
+    const int pieces = (nk >> ks) * run;               // of a group
+    if ((run & (run - 1)) == 0 && run <= LOADERS) {
+      const int sr = 31 - __clz(run);
+      const long long step = (long long)(LOADERS >> sr) * a.t1;
+      for (int g = 0; g * rc < R && r0 + g * rc < o.rows; ++g) {
+        const float* src = P + row_off(r0 + g * rc) + ((kb0 >> ks) + (i >> sr)) * a.t1 + (i & (run - 1)) * 4;
+        float* dst = stg + g * rc * BK + i * 4;
+        for (int j = i; j < pieces; j += LOADERS, src += step, dst += LOADERS * 4) cp16(dst, src);
+      }
+    } else {
+      for (int g = 0; g * rc < R && r0 + g * rc < o.rows; ++g)
+        for (int j = i; j < pieces; j += LOADERS)
+          cp16(stg + g * rc * BK + j * 4, P + row_off(r0 + g * rc) + ((kb0 >> ks) + j / run) * a.t1 + (j % run) * 4);
+    }
+    return true;
   }
-  return nk > 0;
+  // GENERIC: `parts` threads per row, part h the values [h * len, (h + 1) * len)
+  const long long left = o.rows - r0;
+  const int own = left <= 32 ? 32 : left <= 64 ? 64 : LOADERS;  // rows with threads of their own
+  const int row_i = i & (own - 1), parts = LOADERS / own, len = (nk + parts - 1) / parts;
+  const int k0 = (i / own) * len, k1 = k0 + len < nk ? k0 + len : nk;
+  if (row_i >= R || row_i >= left || k0 >= k1) return false;
+  const float* base = P + row_off(r0 + row_i);
+  int rem = 0;
+  if (a.kc == 1) {
+    base += (kb0 + k0) * a.t1;
+  } else {
+    const long long q = (kb0 + k0) / a.kc;
+    rem = (int)(kb0 + k0 - q * a.kc);
+    base += q * a.t1;
+  }
+  const float* src = base + rem * a.t2;
+  const int kc = (int)(a.kc < BK + 1 ? a.kc : kb0 + BK + 1 < a.kc ? kb0 + BK + 1 : a.kc);
+  float* dst = stg + row_i * 8;
+#pragma unroll 4
+  for (int k = k0; k < k1; ++k) {
+    cp4(dst + (k >> 3) * (R * 8) + (k & 7), src);
+    src += a.t2;
+    if (++rem == kc) {
+      rem = 0;
+      base += a.t1;
+      src = base;
+    }
+  }
+  return true;
 }
 
-// Converts the rows r0 .. r0 + R - 1 of a filled slot into the bfloat16 operand image at
-// sa (R rows of 128 bytes, swizzled); any loader thread may convert any value.
-template <int R>
+// Round a landed slot to bfloat16 in the operand stage: 8-value chunk ch of row i
+// goes to the 128-byte swizzled tile (sa).  Only the operand's own rows are rounded
+// (a row past M or N feeds only output that is not stored).
+template <int R, int MODE>
 __device__ __forceinline__ void convert_op(uint8_t* sa, const float* stg, const Op& o, long long K, long long r0,
                                            int kb, int i) {
   const long long kb0 = (long long)kb * BK;
@@ -525,40 +638,102 @@ __device__ __forceinline__ void convert_op(uint8_t* sa, const float* stg, const 
   const int nch = nk >= BK ? 8 : 2 * ((nk + 15) / 16);  // chunks the MMAs read
   const int nrow = (int)(o.rows - r0 < R ? o.rows - r0 : R);  // rows to convert
   if (nrow <= 0) return;
-  if (o.mode == ROWRUN || o.mode == TILERUN) {
-    const int ld = o.mode == ROWRUN ? BK : nk;
-    for (int t = i; t < nrow * nch; t += LOADERS) {  // (row, chunk), chunk fastest
-      const int row = t / nch, ch = t - (t / nch) * nch;
+  const bool whole = nk == nch * 8;
+  const int mode = MODE == ANY ? o.mode : MODE;
+  if (mode == ROWRUN || mode == TILERUN) {  // chunk fastest over the threads
+    const int ld = mode == ROWRUN ? BK : nk;
+    if (nch != 6) {  // a power of two: every round moves on by LOADERS / nch rows, a multiple of 8
+      const int sh = nch == 8 ? 3 : nch == 4 ? 2 : 1, rs = LOADERS >> sh;
+      int row = i >> sh;
+      const int ch = i & (nch - 1);
       const float* src = stg + row * ld + ch * 8;
-      float x[8];
-      if (ch * 8 + 8 <= nk && (ld & 3) == 0) {
-        const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
-        x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w; x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
+      uint8_t* dst = sa + sw128(row, ch * 8);
+      if (whole) {
+        for (; row + 3 * rs < nrow; row += 4 * rs, src += 4 * rs * ld, dst += 4 * rs * 128) {
+          float4 lo[4], hi[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            lo[u] = *reinterpret_cast<const float4*>(src + u * rs * ld);
+            hi[u] = *reinterpret_cast<const float4*>(src + u * rs * ld + 4);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float x[8] = {lo[u].x, lo[u].y, lo[u].z, lo[u].w, hi[u].x, hi[u].y, hi[u].z, hi[u].w};
+            put_chunk(dst + u * rs * 128, x);
+          }
+        }
+        for (; row < nrow; row += rs, src += rs * ld, dst += rs * 128) {
+          const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
+          const float x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+          put_chunk(dst, x);
+        }
       } else {
+        for (; row < nrow; row += rs, src += rs * ld, dst += rs * 128) {
+          float x[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = ch * 8 + e < nk ? src[e] : 0.f;
+          for (int e = 0; e < 8; ++e) x[e] = ch * 8 + e < nk ? src[e] : 0.f;
+          put_chunk(dst, x);
+        }
       }
-      store_chunk(sa, row, ch, x);
+      return;
     }
-  } else if (o.mode == GROUPRUN) {
-    const int rc = o.rc;
-    for (int t = i; t < nrow * nch; t += LOADERS) {  // (row, chunk), row fastest
-      const int ch = t / nrow, row = t - ch * nrow;
-      const float* src = stg + (row / rc) * (BK * rc) + (ch * 8) * rc + (row % rc);
-      float x[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) x[e] = ch * 8 + e < nk ? src[e * rc] : 0.f;
-      store_chunk(sa, row, ch, x);
-    }
-  } else {
-    for (int t = i; t < nrow * nch; t += LOADERS) {  // (row, chunk), row fastest
-      const int ch = t / nrow, row = t - ch * nrow;
-      const float* src = stg + (ch * R + row) * 8;
+    for (int t = i; t < nrow * nch; t += LOADERS) {
+      const int row = t / nch, ch = t - row * nch;
+      const float* src = stg + row * ld + ch * 8;
       float x[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[e] = ch * 8 + e < nk ? src[e] : 0.f;
-      store_chunk(sa, row, ch, x);
+      put_chunk(sa + sw128(row, ch * 8), x);
     }
+    return;
+  }
+  // row fastest over the threads
+  const int rc = o.rc;
+  const bool pair = mode == PIECES && o.a.kc == 2;
+  if (mode != GENERIC && whole && (nrow & (nrow - 1)) == 0 && (rc & (rc - 1)) == 0) {
+    // a thread keeps its row; every round moves on by LOADERS / nrow chunks
+    const int sr = 31 - __clz(nrow), sg = 31 - __clz(rc), cs = LOADERS >> sr;
+    const int row = i & (nrow - 1), in = row & (rc - 1);
+    const float* src = stg + ((row >> sg) * (BK << sg)) + (pair ? 2 * in : in);
+    uint8_t* const dst = sa + row * 128;
+    for (int ch = i >> sr; ch < nch; ch += 2 * cs) {  // two chunks at a time
+      float x[2][8];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int c = min(ch + u * cs, nch - 1);
+        const float* p = src + ((c * 8) << sg);
+        if (pair) {
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) {
+            const float2 v = *reinterpret_cast<const float2*>(p + (e << sg));
+            x[u][e] = v.x;
+            x[u][e + 1] = v.y;
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[u][e] = p[e << sg];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (ch + u * cs < nch) put_chunk(dst + (((ch + u * cs) ^ (row & 7)) << 4), x[u]);
+    }
+    return;
+  }
+  for (int t = i; t < nrow * nch; t += LOADERS) {
+    const int ch = t / nrow, row = t - ch * nrow;
+    float x[8];
+    if (mode == GENERIC) {
+      const float* src = stg + (ch * R + row) * 8;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = ch * 8 + e < nk ? src[e] : 0.f;
+    } else {
+      const float* src = stg + (row / rc) * (BK * rc) + (ch * 8) * rc + (pair ? 2 : 1) * (row % rc);
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        x[e] = ch * 8 + e < nk ? (pair ? src[(e >> 1) * 2 * rc + (e & 1)] : src[e * rc]) : 0.f;
+    }
+    put_chunk(sa + sw128(row, ch * 8), x);
   }
 }
 }  // namespace ws
@@ -580,6 +755,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 // (b_img, one image per batch) or, for BN = 32, as an FP32 operand (b.p) staged and
 // rounded like A.  With part set the epilogue writes raw partial tiles
 // part[((batch * splits + split) * tiles + tile) * 128 * BN + row * BN + col] instead.
+// Forms of the epilogue's output: raw partial tiles; columns contiguous in whole 16-byte
+// pieces; columns contiguous; any other layout, rows along the lanes.
+enum { OUT_PART, OUT_VEC, OUT_COLS, OUT_ROWS };
+
 struct WsArgs {
   ws::Op a, b;
   const uint8_t* b_img;
@@ -587,9 +766,10 @@ struct WsArgs {
   int kblocks, kper, splits, ntiles;
   long long mtiles, items;
   float* part;
+  int vec;  // rows of the output (and of add, act) in whole 16-byte pieces
 };
 
-template <int BN>
+template <int BN, bool FUSE>
 __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e, int* __restrict__ err) {
   using C = ws::Cfg<BN>;
   constexpr int ST = C::STAGES, D = C::DEPTH;
@@ -603,11 +783,6 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
   __shared__ long long off_s[ws::EPI_WARPS][32];  // epilogue: per warp, 32 row (or column) offsets
   __shared__ float bias_s[ws::EPI_WARPS][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool fuse_b = w.b_img == nullptr;
-  if (fuse_b && C::BSLOT_FLOATS == 0) {  // host error: FP32 B needs BN = 32
-    if (threadIdx.x == 0) atomicOr(err, 64);
-    return;
-  }
   if (warp == ws::MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
                  "r"(C::TMEM_COLS)
@@ -633,97 +808,127 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base;
   const long long tiles = w.mtiles * w.ntiles;
-  // item -> (batch, split, mt, nt) and its K blocks
-  auto decode = [&](long long it, long long& bt, int& split, long long& mt, int& nt, int& kb0, int& kb1) {
-    nt = (int)(it % w.ntiles);
-    const long long t2 = it / w.ntiles;
-    mt = t2 % w.mtiles;
-    const long long t3 = t2 / w.mtiles;
-    split = (int)(t3 % w.splits);
-    bt = t3 / w.splits;
-    kb0 = split * w.kper;
-    kb1 = kb0 + w.kper < w.kblocks ? kb0 + w.kper : w.kblocks;
-  };
+  const int mtiles = (int)w.mtiles;
+  auto k_end = [&](int split) { return min((split + 1) * w.kper, w.kblocks); };
 
   if (warp < 4) {  // operand loaders
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
     const int i = threadIdx.x;
     // stages of this CTA in order: a cursor over (item, K block)
     struct Cur {
-      long long it, bt, mt;
-      int nt, split, kb, kb1;
+      ws::Walk w;
+      int kb, kb1;
     };
-    auto start = [&](Cur& c, long long it) {
-      c.it = it;
-      if (it < w.items) decode(it, c.bt, c.split, c.mt, c.nt, c.kb, c.kb1);
+    auto open = [&](Cur& c) {
+      c.kb = c.w.split * w.kper;
+      c.kb1 = k_end(c.w.split);
     };
     auto advance = [&](Cur& c) {
-      if (++c.kb >= c.kb1) start(c, c.it + gridDim.x);
-    };
-    auto issue = [&](const Cur& c, long long g) {
-      const int d = (int)(g % D);
-      bool cp = ws::issue_op<BM>(stg0 + d * ws::SLOT_FLOATS, &afull[d], w.a, c.bt, w.K, c.mt * BM, c.kb, i);
-      if (fuse_b)
-        cp |= ws::issue_op<C::BROWS>(stgb + d * C::BSLOT_FLOATS, &afull[d], w.b, c.bt, w.K, (long long)c.nt * BN,
-                                     c.kb, i);
-      if (cp) ws::cp_arrive(&afull[d]);
-      else mbar_arrive(&afull[d]);
-    };
-    Cur cur, ahead;
-    start(cur, blockIdx.x);
-    start(ahead, blockIdx.x);
-    long long issued = 0;
-    for (; issued < D && ahead.it < w.items; ++issued, advance(ahead)) issue(ahead, issued);
-    long long g = 0;
-    for (; cur.it < w.items; ++g, advance(cur)) {
-      const int s = (int)(g % ST), d = (int)(g % D);
-      bool ok = mbar_wait_bounded(&afull[d], (uint32_t)((g / D) & 1));
-      if (ok && g >= ST) ok = mbar_wait_bounded(&empty[s], (uint32_t)(((g / ST) - 1) & 1));
-      if (!ws::loaders_all(ok)) {
-        if (i == 0) atomicOr(err, 2);
-        break;
+      if (++c.kb >= c.kb1) {
+        c.w.next(gridDim.x, w.ntiles, mtiles, w.splits);
+        open(c);
       }
-      uint8_t* st = smem + s * C::STAGE_BYTES;
-      if (fuse_b) {
-        ws::convert_op<C::BROWS>(st + A_BYTES, stgb + d * C::BSLOT_FLOATS, w.b, w.K, (long long)cur.nt * BN, cur.kb,
-                                 i);
-      } else if (i == 0) {
-        mbar_expect_tx(&bfull[s], C::B_BYTES);
-        bulk_g2s(st + A_BYTES, w.b_img + (((size_t)cur.bt * w.ntiles + cur.nt) * w.kblocks + cur.kb) * C::B_BYTES,
-                 C::B_BYTES, &bfull[s]);
+    };
+    // One loop per operand form: what runs is one form's instructions, without the others between
+    auto load = [&](auto form_a, auto form_b) {
+      constexpr int MA = decltype(form_a)::value;
+      [[maybe_unused]] constexpr int MB = decltype(form_b)::value;
+      Cur cur, ahead;
+      cur.w.start(blockIdx.x, gridDim.x, w.ntiles, mtiles, w.splits);
+      open(cur);
+      ahead = cur;
+      int flight = 0, di = 0;  // slots issued and not yet converted: d, d + 1, ... up to di (mod D)
+      // stage s and slot d of the current block, with the phases their barriers complete next
+      int s = 0, d = 0, used = 0;  // used: stages handed to the MMAs, at most ST
+      uint32_t sp = 0, dp = 0;
+      while (true) {
+        for (; flight < D && ahead.w.it < w.items; ++flight, advance(ahead)) {
+          bool cp = ws::issue_op<BM, MA>(stg0 + di * ws::SLOT_FLOATS, &afull[di], w.a, ahead.w.bt, w.K,
+                                         (long long)ahead.w.mt * BM, ahead.kb, i);
+          if constexpr (FUSE)
+            cp |= ws::issue_op<C::BROWS, MB>(stgb + di * C::BSLOT_FLOATS, &afull[di], w.b, ahead.w.bt, w.K,
+                                             (long long)ahead.w.nt * BN, ahead.kb, i);
+          if (cp) ws::cp_arrive(&afull[di]);
+          else mbar_arrive(&afull[di]);
+          if (++di == D) di = 0;
+        }
+        if (cur.w.it >= w.items) break;
+        bool ok = ws::wait_bar(&afull[d], dp);
+        if (ok && used == ST) ok = ws::wait_bar(&empty[s], sp ^ 1u);
+        if (ok) {
+          uint8_t* st = smem + s * C::STAGE_BYTES;
+          if constexpr (FUSE) {
+            ws::convert_op<C::BROWS, MB>(st + A_BYTES, stgb + d * C::BSLOT_FLOATS, w.b, w.K, (long long)cur.w.nt * BN,
+                                         cur.kb, i);
+          } else if (i == 0) {
+            mbar_expect_tx(&bfull[s], C::B_BYTES);
+            bulk_g2s(st + A_BYTES, w.b_img + (((size_t)cur.w.bt * w.ntiles + cur.w.nt) * w.kblocks + cur.kb) * C::B_BYTES,
+                     C::B_BYTES, &bfull[s]);
+          }
+          ws::convert_op<BM, MA>(st, stg0 + d * ws::SLOT_FLOATS, w.a, w.K, (long long)cur.w.mt * BM, cur.kb, i);
+          fence_proxy_async();  // the tensor cores read the stage through the async proxy
+          mbar_arrive(&full[s]);
+          if (FUSE && i == 0) mbar_arrive(&bfull[s]);
+          if (used < ST) ++used;
+          if (++s == ST) { s = 0; sp ^= 1u; }
+        }
+        // every loader is done with slot d; a wait that ran out on one ends them all
+        if (!ws::loaders_all(ok)) {
+          if (i == 0) atomicOr(err, 2);
+          break;
+        }
+        --flight;
+        if (++d == D) { d = 0; dp ^= 1u; }
+        advance(cur);
       }
-      ws::convert_op<BM>(st, stg0 + d * ws::SLOT_FLOATS, w.a, w.K, cur.mt * BM, cur.kb, i);
-      fence_proxy_async();  // the tensor cores read the stage through the async proxy
-      mbar_arrive(&full[s]);
-      if (fuse_b && i == 0) mbar_arrive(&bfull[s]);
-      ws::loaders_sync();  // every loader is done with slot d
-      if (ahead.it < w.items) {
-        issue(ahead, issued++);
-        advance(ahead);
+      // copies in flight land before the CTA's shared memory is released
+      for (; flight > 0; --flight) {
+        mbar_wait_bounded(&afull[d], dp);
+        if (++d == D) { d = 0; dp ^= 1u; }
+      }
+      if (i == 0 && !FUSE) {
+        if (used == ST) sp ^= 1u;  // the last ST stages: s is the oldest of them
+        else s = 0;
+        for (int j = 0; j < used; ++j) {
+          mbar_wait_bounded(&bfull[s], sp);
+          if (++s == ST) { s = 0; sp ^= 1u; }
+        }
+      }
+    };
+    if constexpr (FUSE) {
+      if (w.a.mode == ws::GROUPRUN && w.b.mode == ws::GROUPRUN)
+        load(ws::Tag<ws::GROUPRUN>{}, ws::Tag<ws::GROUPRUN>{});
+      else
+        load(ws::Tag<ws::ANY>{}, ws::Tag<ws::ANY>{});
+    } else {
+      switch (w.a.mode) {
+        case ws::ROWRUN: load(ws::Tag<ws::ROWRUN>{}, ws::Tag<0>{}); break;
+        case ws::GROUPRUN: load(ws::Tag<ws::GROUPRUN>{}, ws::Tag<0>{}); break;
+        case ws::TILERUN: load(ws::Tag<ws::TILERUN>{}, ws::Tag<0>{}); break;
+        case ws::PIECES: load(ws::Tag<ws::PIECES>{}, ws::Tag<0>{}); break;
+        default: load(ws::Tag<ws::GENERIC>{}, ws::Tag<0>{}); break;
       }
     }
-    // copies in flight land before the CTA's shared memory is released
-    for (long long j = g; j < issued; ++j) mbar_wait_bounded(&afull[j % D], (uint32_t)((j / D) & 1));
-    if (i == 0 && !fuse_b)
-      for (long long j = g > ST ? g - ST : 0; j < g; ++j) mbar_wait_bounded(&bfull[j % ST], (uint32_t)((j / ST) & 1));
-  } else if (warp == ws::MMA_WARP) {  // MMA issuer
-    if (lane == 0) {
-      long long g = 0, n = 0;
+  } else if (warp >= ws::MMA_WARP) {  // MMA issuer
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == ws::MMA_WARP && lane == 0) {
+      long long n = 0;
+      int s = 0;
+      uint32_t par = 0;
       bool ok = true;
-      for (long long it = blockIdx.x; it < w.items && ok; it += gridDim.x, ++n) {
-        long long bt, mt;
-        int split, nt, kb0, kb1;
-        decode(it, bt, split, mt, nt, kb0, kb1);
+      ws::Walk t;
+      t.start(blockIdx.x, gridDim.x, w.ntiles, mtiles, w.splits);
+      for (; t.it < w.items && ok; t.next(gridDim.x, w.ntiles, mtiles, w.splits), ++n) {
+        const int kb0 = t.split * w.kper, kb1 = k_end(t.split);
         const int buf = (int)(n & 1);
-        if (n >= 2 && !mbar_wait_bounded(&acce[buf], (uint32_t)(((n >> 1) - 1) & 1))) {
+        if (n >= 2 && !ws::wait_bar(&acce[buf], (uint32_t)(((n >> 1) - 1) & 1))) {
           atomicOr(err, 16);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t dacc = tmem + (uint32_t)(buf * BN);
-        for (int kb = kb0; kb < kb1; ++kb, ++g) {
-          const int s = (int)(g % ST);
-          const uint32_t par = (uint32_t)((g / ST) & 1);
-          if (!mbar_wait_bounded(&full[s], par) || !mbar_wait_bounded(&bfull[s], par)) {
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!ws::wait_bar(&full[s], par) || !ws::wait_bar(&bfull[s], par)) {
             atomicOr(err, 4);
             ok = false;
             break;
@@ -744,6 +949,7 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                            smem_u32(&empty[s]))
                        : "memory");
+          if (++s == ST) { s = 0; par ^= 1u; }
         }
         if (!ok) break;
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -758,143 +964,208 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
     }
     __syncwarp();
   } else {  // epilogue, warps 4-11: group eg takes this CTA's tiles n = eg, eg + 2, ... (accumulator eg)
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
     const int wi = warp - 4, eg = wi >> 2, q = warp & 3;
-    float* const blk = epi_buf + wi * (32 * 33);
-    const bool split_cols = e.out.kc != 1;
-    const bool stage_cols = !split_cols && e.out.t1 == 1;
-    const uint32_t lanes = (uint32_t)(q * 32) << 16;
-    for (long long it = blockIdx.x + (long long)eg * gridDim.x, n = eg; it < w.items;
-         it += 2LL * gridDim.x, n += 2) {
-      const int buf = (int)(n & 1);
-      if (!mbar_wait_bounded(&accf[buf], (uint32_t)((n >> 1) & 1))) {
-        if (lane == 0) atomicOr(err, 8);
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      long long bt, mt;
-      int split, nt, kb0, kb1;
-      decode(it, bt, split, mt, nt, kb0, kb1);
-      const long long r = mt * BM + q * 32 + lane;
-      const bool row_ok = r < e.M;
-      if (w.part) {  // raw partial tile: each lane stores its row's BN values
-        float* pp = w.part + ((bt * w.splits + split) * tiles + mt * w.ntiles + nt) * (long long)(BM * BN) +
-                    (long long)(q * 32 + lane) * BN;
-        for (int c0 = 0; c0 < BN; c0 += 16) {
-          uint32_t v[16];
-          tmem_ld16(tmem + lanes + (uint32_t)(buf * BN + c0), v);
-          if (row_ok) {
+    float* const blk = epi_buf + wi * ws::EPI_BLOCK;
+    const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(eg * BN);
+    // the warp's 32 x 32 accumulator block at column c0, to shared memory by rows
+    auto block_to_smem = [&](int c0) {
 #pragma unroll
-            for (int j = 0; j < 16; j += 4)
-              *reinterpret_cast<float4*>(pp + c0 + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
-                                                                    __uint_as_float(v[j + 2]),
-                                                                    __uint_as_float(v[j + 3]));
-          }
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acce[buf]);
-        continue;
-      }
-      float* const ey = e.y + bt * e.ybs;
-      const float* const eadd = e.add ? e.add + bt * e.ybs : nullptr;
-      float* const eact = e.act ? e.act + bt * e.ybs : nullptr;
-      const float* const p1 = eadd ? eadd : ey;  // first addend (add, else the accumulated output)
-      const bool have_prev = eadd || e.accumulate, both = eadd && e.accumulate;
-      const long long rbase = row_ok ? (r / e.out.rc) * e.out.s1 + (r % e.out.rc) * e.out.s2 : -1;
-      // Offsets and biases of the warp's 32 rows or columns go through shared memory, and
-      // the loads of add / accumulate are unconditional (an invalid element reads word 0
-      // of its array), so 16 of them are in flight before the first is used.
-      for (int c0 = 0; c0 < BN && nt * BN + c0 < e.N; c0 += 32) {
-        const int c = nt * BN + c0 + lane;  // this lane's column
-        const bool col_ok = c < e.N;
-        const uint32_t taddr = tmem + lanes + (uint32_t)(buf * BN + c0);
-        if (stage_cols) {
-          // columns contiguous in the output: the warp's 32 x 32 block goes through shared
-          // memory and each row is stored with the lanes along its columns
+      for (int h = 0; h < 2; ++h) {
+        uint32_t v[16];
+        tmem_ld16(acc + (uint32_t)(c0 + h * 16), v);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
+        for (int j = 0; j < 16; j += 4)
+          *reinterpret_cast<float4*>(blk + lane * ws::EPI_LD + h * 16 + j) =
+              make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]),
+                          __uint_as_float(v[j + 3]));
+      }
+    };
+    // One loop per output form.  In each the loads of add / accumulate are unconditional
+    // (an invalid element reads word 0 of its array) and a whole block of them is in
+    // flight before the accumulator is waited for, for they do not depend on it.
+    auto finish = [&](auto form) {
+      constexpr int F = decltype(form)::value;
+      ws::Walk t;
+      t.start(blockIdx.x + (long long)eg * gridDim.x, 2LL * gridDim.x, w.ntiles, mtiles, w.splits);
+      for (uint32_t phase = 0; t.it < w.items; t.next(2LL * gridDim.x, w.ntiles, mtiles, w.splits), phase ^= 1u) {
+        const int nt = t.nt;
+        const long long bt = t.bt, r = (long long)t.mt * BM + q * 32 + lane;
+        const bool row_ok = r < e.M;
+        auto landed = [&] {
+          const bool ok = ws::wait_bar(&accf[eg], phase);
+          if (!ok && lane == 0) atomicOr(err, 8);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          return __all_sync(0xffffffffu, ok) != 0;
+        };
+        bool ok = true;
+        if constexpr (F == OUT_PART) {  // raw partial tile: each lane stores its row's BN values
+          ok = landed();
+          float* pp = w.part + ((bt * w.splits + t.split) * tiles + (long long)t.mt * w.ntiles + nt) * (long long)(BM * BN) +
+                      (long long)(q * 32 + lane) * BN;
+          for (int c0 = 0; ok && c0 < BN; c0 += 16) {
             uint32_t v[16];
-            tmem_ld16(taddr + (uint32_t)(h * 16), v);
+            tmem_ld16(acc + (uint32_t)c0, v);
+            if (row_ok) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) blk[lane * 33 + h * 16 + j] = __uint_as_float(v[j]);
+              for (int j = 0; j < 16; j += 4)
+                *reinterpret_cast<float4*>(pp + c0 + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
+                                                                      __uint_as_float(v[j + 2]),
+                                                                      __uint_as_float(v[j + 3]));
+            }
           }
-          off_s[wi][lane] = rbase;
+        } else {
+          float* const ey = e.y + bt * e.ybs;
+          const float* const eadd = e.add ? e.add + bt * e.ybs : nullptr;
+          float* const eact = e.act ? e.act + bt * e.ybs : nullptr;
+          const float* const p1 = eadd ? eadd : ey;  // first addend (add, else the accumulated output)
+          const bool have_prev = eadd || e.accumulate, both = eadd && e.accumulate;
+          const long long rbase = !row_ok ? -1
+                                  : e.out.rc == 1 ? r * e.out.s1
+                                                  : (r / e.out.rc) * e.out.s1 + (r % e.out.rc) * e.out.s2;
+          if constexpr (F != OUT_ROWS) off_s[wi][lane] = rbase;
           __syncwarp();
-          const float bias_c = (e.bias && col_ok) ? __ldg(e.bias + c) : 0.f;
+          for (int c0 = 0; ok && c0 < BN && nt * BN + c0 < e.N; c0 += 32) {
+            const int c = nt * BN + c0 + lane;  // this lane's column
+            const bool col_ok = c < e.N;
+            if constexpr (F == OUT_VEC) {
+              // columns contiguous in the output and in whole 16-byte pieces: the warp's
+              // 32 x 32 block goes through shared memory, then a lane takes four columns
+              // of a row and neighbouring lanes the rest of the row, so an access covers
+              // four whole lines.
+              const int cols = e.N - nt * BN - c0;  // 1 << lp lanes cover a row's columns in this block
+              const int lp = cols > 16 ? 3 : cols > 8 ? 2 : cols > 4 ? 1 : 0;
+              const int q4 = (lane & ((1 << lp) - 1)) * 4, c4 = nt * BN + c0 + q4, row0 = lane >> lp, step = 32 >> lp;
+              const bool c_ok = c4 < e.N;
+              long long o4[8];  // 1 << lp rounds of `step` rows
+              float4 prev[8];
 #pragma unroll
-          for (int h = 0; h < 32; h += 16) {
-            float prev[16];
-            if (have_prev) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const long long ro = off_s[wi][h + j];
-                prev[j] = p1[(ro >= 0 && col_ok) ? ro + c : 0];
+              for (int u = 0; u < 8; ++u) {
+                const int row = u * step + row0;
+                const long long rb = off_s[wi][row & 31];
+                o4[u] = row < 32 && rb >= 0 && c_ok ? rb + c4 : -1;
               }
-              if (both) {
+              if (have_prev) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) prev[u] = *reinterpret_cast<const float4*>(p1 + (o4[u] >= 0 ? o4[u] : 0));
+                if (both) {
+#pragma unroll
+                  for (int u = 0; u < 8; ++u) {
+                    const float4 y4 = *reinterpret_cast<const float4*>(ey + (o4[u] >= 0 ? o4[u] : 0));
+                    prev[u] = make_float4(prev[u].x + y4.x, prev[u].y + y4.y, prev[u].z + y4.z, prev[u].w + y4.w);
+                  }
+                }
+              }
+              float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (e.bias && c_ok)
+                b4 = make_float4(__ldg(e.bias + c4), __ldg(e.bias + c4 + 1), __ldg(e.bias + c4 + 2), __ldg(e.bias + c4 + 3));
+              if (c0 == 0) ok = landed();
+              if (!ok) break;
+              block_to_smem(c0);
+              __syncwarp();
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {
+                if (o4[u] < 0) continue;
+                const float4 a4 = *reinterpret_cast<const float4*>(blk + (u * step + row0) * ws::EPI_LD + q4);
+                float4 z = make_float4(fmaf(a4.x, e.scale, b4.x), fmaf(a4.y, e.scale, b4.y), fmaf(a4.z, e.scale, b4.z),
+                                       fmaf(a4.w, e.scale, b4.w));
+                if (have_prev) z = make_float4(z.x + prev[u].x, z.y + prev[u].y, z.z + prev[u].z, z.w + prev[u].w);
+                *reinterpret_cast<float4*>(ey + o4[u]) = z;
+                if (eact)
+                  *reinterpret_cast<float4*>(eact + o4[u]) =
+                      make_float4(gelu_t(z.x), gelu_t(z.y), gelu_t(z.z), gelu_t(z.w));
+              }
+              __syncwarp();
+            } else if constexpr (F == OUT_COLS) {
+              // columns contiguous in the output: the block goes through shared memory and
+              // each row is stored with the lanes along its columns
+              if (c0 == 0) ok = landed();
+              if (!ok) break;
+              block_to_smem(c0);
+              __syncwarp();
+              const float bias_c = (e.bias && col_ok) ? __ldg(e.bias + c) : 0.f;
+#pragma unroll 1
+              for (int h = 0; h < 32; h += 16) {
+                float prev[16];
+                if (have_prev) {
+#pragma unroll
+                  for (int j = 0; j < 16; ++j) {
+                    const long long ro = off_s[wi][h + j];
+                    prev[j] = p1[(ro >= 0 && col_ok) ? ro + c : 0];
+                  }
+                  if (both) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                      const long long ro = off_s[wi][h + j];
+                      prev[j] += ey[(ro >= 0 && col_ok) ? ro + c : 0];
+                    }
+                  }
+                }
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                   const long long ro = off_s[wi][h + j];
-                  prev[j] += ey[(ro >= 0 && col_ok) ? ro + c : 0];
+                  if (ro >= 0 && col_ok) {
+                    float z = fmaf(blk[(h + j) * ws::EPI_LD + lane], e.scale, bias_c);
+                    if (have_prev) z += prev[j];
+                    ey[ro + c] = z;
+                    if (eact) eact[ro + c] = gelu_t(z);
+                  }
                 }
               }
-            }
+              __syncwarp();
+            } else {
+              // lanes along rows; the column offsets (this lane's for column c0 + lane) in shared memory
+              off_s[wi][lane] = !col_ok ? -1
+                                : e.out.kc == 1 ? (long long)c * e.out.t1
+                                                : (long long)(c / e.out.kc) * e.out.t1 + (long long)(c % e.out.kc) * e.out.t2;
+              bias_s[wi][lane] = (e.bias && col_ok) ? __ldg(e.bias + c) : 0.f;
+              __syncwarp();
+              float prev[32];
+              if (have_prev) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const long long ro = off_s[wi][h + j];
-              if (ro >= 0 && col_ok) {
-                float z = fmaf(blk[(h + j) * 33 + lane], e.scale, bias_c);
-                if (have_prev) z += prev[j];
-                ey[ro + c] = z;
-                if (eact) eact[ro + c] = gelu_t(z);
+                for (int j = 0; j < 32; ++j) {
+                  const long long cj = off_s[wi][j];
+                  prev[j] = p1[(row_ok && cj >= 0) ? rbase + cj : 0];
+                }
+                if (both) {
+#pragma unroll
+                  for (int j = 0; j < 32; ++j) {
+                    const long long cj = off_s[wi][j];
+                    prev[j] += ey[(row_ok && cj >= 0) ? rbase + cj : 0];
+                  }
+                }
               }
-            }
-          }
-          __syncwarp();
-        } else {
-          // lanes along rows; the column offsets (this lane's for column c0 + lane) in shared memory
-          off_s[wi][lane] = col_ok ? (split_cols ? (long long)(c / e.out.kc) * e.out.t1 +
-                                                       (long long)(c % e.out.kc) * e.out.t2
-                                                 : (long long)c * e.out.t1)
-                                   : -1;
-          bias_s[wi][lane] = (e.bias && col_ok) ? __ldg(e.bias + c) : 0.f;
-          __syncwarp();
+              if (c0 == 0) ok = landed();
+              if (!ok) break;
 #pragma unroll
-          for (int h = 0; h < 32; h += 16) {
-            uint32_t v[16];
-            tmem_ld16(taddr + (uint32_t)h, v);
-            float prev[16];
-            if (have_prev) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const long long cj = off_s[wi][h + j];
-                prev[j] = p1[(row_ok && cj >= 0) ? rbase + cj : 0];
-              }
-              if (both) {
+              for (int h = 0; h < 32; h += 16) {
+                uint32_t v[16];
+                tmem_ld16(acc + (uint32_t)(c0 + h), v);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                   const long long cj = off_s[wi][h + j];
-                  prev[j] += ey[(row_ok && cj >= 0) ? rbase + cj : 0];
+                  if (row_ok && cj >= 0) {
+                    float z = fmaf(__uint_as_float(v[j]), e.scale, bias_s[wi][h + j]);
+                    if (have_prev) z += prev[h + j];
+                    ey[rbase + cj] = z;
+                    if (eact) eact[rbase + cj] = gelu_t(z);
+                  }
                 }
               }
-            }
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const long long cj = off_s[wi][h + j];
-              if (row_ok && cj >= 0) {
-                float z = fmaf(__uint_as_float(v[j]), e.scale, bias_s[wi][h + j]);
-                if (have_prev) z += prev[j];
-                ey[rbase + cj] = z;
-                if (eact) eact[rbase + cj] = gelu_t(z);
-              }
+              __syncwarp();
             }
           }
-          __syncwarp();
         }
+        if (!ok) break;
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acce[eg]);
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acce[buf]);
-    }
+    };
+    if (w.part) finish(ws::Tag<OUT_PART>{});
+    else if (w.vec) finish(ws::Tag<OUT_VEC>{});
+    else if (e.out.kc == 1 && e.out.t1 == 1) finish(ws::Tag<OUT_COLS>{});
+    else finish(ws::Tag<OUT_ROWS>{});
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -903,9 +1174,9 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::TMEM_COLS) : "memory");
 }
 
-// Resident CTAs per SM of gemm_ws_kernel<BN> (shared memory, registers and the two
+// Resident CTAs per SM of gemm_ws_kernel<BN, FUSE> (shared memory, registers and the two
 // accumulators' tensor-memory columns), per device.
-template <int BN>
+template <int BN, bool FUSE>
 cudaError_t ws_slots(int& slots) {
   static std::atomic<int> cache[64];
   int dev = 0;
@@ -914,14 +1185,14 @@ cudaError_t ws_slots(int& slots) {
   const int d = dev & 63;
   int v = cache[d].load(std::memory_order_acquire);
   if (v <= 0) {
-    c = cudaFuncSetAttribute(gemm_ws_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws::Cfg<BN>::SMEM);
+    c = cudaFuncSetAttribute(gemm_ws_kernel<BN, FUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws::Cfg<BN>::SMEM);
     if (c != cudaSuccess) return c;
     // all of the unified L1 as shared memory
-    c = cudaFuncSetAttribute(gemm_ws_kernel<BN>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    c = cudaFuncSetAttribute(gemm_ws_kernel<BN, FUSE>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);
     if (c != cudaSuccess) return c;
     int occ = 0, sms = 0;
-    c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gemm_ws_kernel<BN>, ws::THREADS, ws::Cfg<BN>::SMEM);
+    c = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gemm_ws_kernel<BN, FUSE>, ws::THREADS, ws::Cfg<BN>::SMEM);
     if (c != cudaSuccess) return c;
     c = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (c != cudaSuccess) return c;
@@ -934,22 +1205,26 @@ cudaError_t ws_slots(int& slots) {
   return cudaSuccess;
 }
 
-template <int BN>
+template <int BN, bool FUSE = false>
 cudaError_t launch_ws_bn(WsArgs w, const Epi& e, int* err, cudaStream_t st, long long batch) {
   int slots = 0;
-  cudaError_t c = ws_slots<BN>(slots);
+  cudaError_t c = ws_slots<BN, FUSE>(slots);
   if (c != cudaSuccess) return c;
   ws::op_mode(w.a, BM, w.K);
-  if (!w.b_img) ws::op_mode(w.b, BN, w.K);
+  if (FUSE) ws::op_mode(w.b, BN, w.K);
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };  // null included
+  w.vec = e.out.kc == 1 && e.out.t1 == 1 && e.N % 4 == 0 && e.out.s1 % 4 == 0 && (e.out.rc == 1 || e.out.s2 % 4 == 0) &&
+          e.ybs % 4 == 0 && al(e.y) && al(e.add) && al(e.act);
   w.items = batch * w.splits * w.mtiles * w.ntiles;
   const unsigned grid = (unsigned)std::min<long long>(w.items, slots);
-  gemm_ws_kernel<BN><<<grid, ws::THREADS, ws::Cfg<BN>::SMEM, st>>>(w, e, err);
+  gemm_ws_kernel<BN, FUSE><<<grid, ws::THREADS, ws::Cfg<BN>::SMEM, st>>>(w, e, err);
   return cudaGetLastError();
 }
 
 cudaError_t launch_ws(int bn, const WsArgs& w, const Epi& e, int* err, cudaStream_t st, long long batch) {
   switch (bn) {
-    case 32: return launch_ws_bn<32>(w, e, err, st, batch);
+    case 32:
+      return w.b_img ? launch_ws_bn<32>(w, e, err, st, batch) : launch_ws_bn<32, true>(w, e, err, st, batch);
     case 64: return launch_ws_bn<64>(w, e, err, st, batch);
     case 128: return launch_ws_bn<128>(w, e, err, st, batch);
     default: return launch_ws_bn<256>(w, e, err, st, batch);
@@ -959,7 +1234,7 @@ cudaError_t launch_ws(int bn, const WsArgs& w, const Epi& e, int* err, cudaStrea
 // Split-K with B from FP32 (BN = 32): one split per resident CTA.
 int ws_split_count(int kblocks, int ksplit) {
   int slots = 0;
-  if (ws_slots<32>(slots) != cudaSuccess) slots = 1;
+  if (ws_slots<32, true>(slots) != cudaSuccess) slots = 1;
   return std::max(1, std::min(kblocks, std::max(ksplit, slots)));
 }
 
