@@ -492,18 +492,21 @@ struct Op {
   long long bs;    // batch stride (floats)
   long long rows;  // M or N
   int mode, rc;    // rc: rows of a group (GROUPRUN, PIECES)
+  int whole;       // TILERUN: every full tile is one 16-byte aligned run
 };
 
 __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total) {
   const Addr& a = o.a;
   o.rc = (int)a.rc;
   o.mode = GENERIC;
+  o.whole = 0;
+  const bool aligned = o.bs % 4 == 0 && (reinterpret_cast<uintptr_t>(o.p) & 15u) == 0;
   if (a.kc == 1 && a.t1 == 1) {
     o.mode = ROWRUN;
     if (a.rc == 1 && k_total <= BK && a.s1 == k_total) o.mode = TILERUN;
+    o.whole = aligned;
     return;
   }
-  const bool aligned = o.bs % 4 == 0 && (reinterpret_cast<uintptr_t>(o.p) & 15u) == 0;
   long long g = -1;
   if (a.s2 == 1 && a.rc > 1) g = a.rc;
   else if (a.rc == 1 && a.s1 == 1) g = o.rows;  // all rows contiguous
@@ -535,9 +538,10 @@ __device__ __forceinline__ bool issue_op(float* stg, uint64_t* bar, const Op& o,
                                          int kb, int i) {
   const long long kb0 = (long long)kb * BK;
   const int nk = (int)(K - kb0 < BK ? K - kb0 : BK);
-  const float* const P = o.p + bt * o.bs;
   const Addr& a = o.a;
   const int mode = MODE == ANY ? o.mode : MODE;
+  if (mode == TILERUN && i != 0 && o.whole && r0 + R <= o.rows) return false;  // thread 0's one copy
+  const float* const P = o.p + bt * o.bs;
   // offset of row r; operands with one row stride need no division
   auto row_off = [&](long long r) { return a.rc == 1 ? r * a.s1 : (r / a.rc) * a.s1 + (r % a.rc) * a.s2; };
   if (mode == TILERUN) {
@@ -630,112 +634,128 @@ __device__ __forceinline__ bool issue_op(float* stg, uint64_t* bar, const Op& o,
 // Round a landed slot to bfloat16 in the operand stage: 8-value chunk ch of row i
 // goes to the 128-byte swizzled tile (sa).  Only the operand's own rows are rounded
 // (a row past M or N feeds only output that is not stored).
+//
+// Convert holds what does not change from one full block to the next: the thread's
+// place, the rounds and the steps between them.  Blocks at the ragged end of the rows
+// or of K, and forms whose chunks do not deal out evenly, take convert_any.
 template <int R, int MODE>
-__device__ __forceinline__ void convert_op(uint8_t* sa, const float* stg, const Op& o, long long K, long long r0,
-                                           int kb, int i) {
+__device__ __forceinline__ void convert_any(uint8_t* sa, const float* stg, const Op& o, long long K, long long r0, int kb,
+                                         int i) {
   const long long kb0 = (long long)kb * BK;
   const int nk = (int)(K - kb0 < BK ? K - kb0 : BK);
   const int nch = nk >= BK ? 8 : 2 * ((nk + 15) / 16);  // chunks the MMAs read
   const int nrow = (int)(o.rows - r0 < R ? o.rows - r0 : R);  // rows to convert
-  if (nrow <= 0) return;
-  const bool whole = nk == nch * 8;
-  const int mode = MODE == ANY ? o.mode : MODE;
-  if (mode == ROWRUN || mode == TILERUN) {  // chunk fastest over the threads
-    const int ld = mode == ROWRUN ? BK : nk;
-    if (nch != 6) {  // a power of two: every round moves on by LOADERS / nch rows, a multiple of 8
-      const int sh = nch == 8 ? 3 : nch == 4 ? 2 : 1, rs = LOADERS >> sh;
-      int row = i >> sh;
-      const int ch = i & (nch - 1);
-      const float* src = stg + row * ld + ch * 8;
-      uint8_t* dst = sa + sw128(row, ch * 8);
-      if (whole) {
-        for (; row + 3 * rs < nrow; row += 4 * rs, src += 4 * rs * ld, dst += 4 * rs * 128) {
-          float4 lo[4], hi[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            lo[u] = *reinterpret_cast<const float4*>(src + u * rs * ld);
-            hi[u] = *reinterpret_cast<const float4*>(src + u * rs * ld + 4);
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float x[8] = {lo[u].x, lo[u].y, lo[u].z, lo[u].w, hi[u].x, hi[u].y, hi[u].z, hi[u].w};
-            put_chunk(dst + u * rs * 128, x);
-          }
-        }
-        for (; row < nrow; row += rs, src += rs * ld, dst += rs * 128) {
-          const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
-          const float x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-          put_chunk(dst, x);
-        }
-      } else {
-        for (; row < nrow; row += rs, src += rs * ld, dst += rs * 128) {
-          float x[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) x[e] = ch * 8 + e < nk ? src[e] : 0.f;
-          put_chunk(dst, x);
-        }
-      }
-      return;
-    }
-    for (int t = i; t < nrow * nch; t += LOADERS) {
-      const int row = t / nch, ch = t - row * nch;
-      const float* src = stg + row * ld + ch * 8;
-      float x[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) x[e] = ch * 8 + e < nk ? src[e] : 0.f;
-      put_chunk(sa + sw128(row, ch * 8), x);
-    }
-    return;
-  }
-  // row fastest over the threads
-  const int rc = o.rc;
-  const bool pair = mode == PIECES && o.a.kc == 2;
-  if (mode != GENERIC && whole && (nrow & (nrow - 1)) == 0 && (rc & (rc - 1)) == 0) {
-    // a thread keeps its row; every round moves on by LOADERS / nrow chunks
-    const int sr = 31 - __clz(nrow), sg = 31 - __clz(rc), cs = LOADERS >> sr;
-    const int row = i & (nrow - 1), in = row & (rc - 1);
-    const float* src = stg + ((row >> sg) * (BK << sg)) + (pair ? 2 * in : in);
-    uint8_t* const dst = sa + row * 128;
-    for (int ch = i >> sr; ch < nch; ch += 2 * cs) {  // two chunks at a time
-      float x[2][8];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int c = min(ch + u * cs, nch - 1);
-        const float* p = src + ((c * 8) << sg);
-        if (pair) {
-#pragma unroll
-          for (int e = 0; e < 8; e += 2) {
-            const float2 v = *reinterpret_cast<const float2*>(p + (e << sg));
-            x[u][e] = v.x;
-            x[u][e + 1] = v.y;
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) x[u][e] = p[e << sg];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-        if (ch + u * cs < nch) put_chunk(dst + (((ch + u * cs) ^ (row & 7)) << 4), x[u]);
-    }
-    return;
-  }
-  for (int t = i; t < nrow * nch; t += LOADERS) {
-    const int ch = t / nrow, row = t - ch * nrow;
+  const int mode = MODE == ANY ? o.mode : MODE, rc = o.rc;
+  const bool runs = mode == ROWRUN || mode == TILERUN, pair = mode == PIECES && o.a.kc == 2;
+  for (int t = i; t < nrow * nch; t += LOADERS) {  // chunk fastest where k is contiguous, else row
+    const int row = runs ? t / nch : t % nrow, ch = runs ? t % nch : t / nrow;
+    const float* src = runs              ? stg + row * (mode == ROWRUN ? BK : nk) + ch * 8
+                       : mode == GENERIC ? stg + (ch * R + row) * 8
+                                         : stg + (row / rc) * (BK * rc) + ch * 8 * rc + (pair ? 2 : 1) * (row % rc);
+    const int step = runs || mode == GENERIC ? 1 : rc;
     float x[8];
-    if (mode == GENERIC) {
-      const float* src = stg + (ch * R + row) * 8;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) x[e] = ch * 8 + e < nk ? src[e] : 0.f;
-    } else {
-      const float* src = stg + (row / rc) * (BK * rc) + (ch * 8) * rc + (pair ? 2 : 1) * (row % rc);
-#pragma unroll
-      for (int e = 0; e < 8; ++e)
-        x[e] = ch * 8 + e < nk ? (pair ? src[(e >> 1) * 2 * rc + (e & 1)] : src[e * rc]) : 0.f;
-    }
+    for (int e = 0; e < 8; ++e)
+      x[e] = ch * 8 + e < nk ? (pair ? src[(e >> 1) * 2 * rc + (e & 1)] : src[e * step]) : 0.f;
     put_chunk(sa + sw128(row, ch * 8), x);
   }
 }
+
+template <int R, int MODE>
+struct Convert {
+  int rounds;            // of LOADERS chunks in a full block; 0: convert_any always
+  int m_full, kb_full;   // full row tiles and K blocks
+  int src, src_step, nk, ch, ch_step, sg;
+  uint32_t dst, dst_step;
+  static constexpr bool RUNS = MODE == ROWRUN || MODE == TILERUN;
+
+  __device__ __forceinline__ void init(const Op& o, long long K, int i) {
+    const int nrow = (int)(o.rows < R ? o.rows : R);
+    nk = (int)(K < BK ? K : BK);
+    const int nch = nk >= BK ? 8 : 2 * ((nk + 15) / 16), total = nrow * nch;
+    m_full = o.rows < R ? 1 : (int)(o.rows / R);
+    kb_full = K < BK ? 1 : (int)(K / BK);
+    rounds = 0;
+    if (MODE == ANY || total % LOADERS != 0) return;
+    if (RUNS) {  // chunk fastest; a round moves on by LOADERS / nch rows, a multiple of 8
+      if (nch == 6) return;
+      const int row = i / nch, ld = MODE == ROWRUN ? BK : nk;
+      ch = i % nch;
+      src = row * ld + ch * 8;
+      src_step = LOADERS / nch * ld;
+      dst = sw128(row, ch * 8);
+      dst_step = (uint32_t)(LOADERS / nch) * 128u;
+    } else {  // row fastest; a thread keeps its row and moves on by LOADERS / nrow chunks
+      if (nk != nch * 8 || (nrow & (nrow - 1)) != 0) return;
+      const int row = i % nrow, rc = o.rc;
+      ch = i / nrow;
+      ch_step = LOADERS / nrow;
+      dst = (uint32_t)row * 128u;
+      dst_step = (uint32_t)(row & 7);
+      if (MODE == GENERIC) {
+        src = (ch * R + row) * 8;
+        src_step = ch_step * R * 8;
+      } else {
+        if ((rc & (rc - 1)) != 0) return;
+        sg = 31 - __clz(rc);
+        const bool pair = MODE == PIECES && o.a.kc == 2;
+        src = (row >> sg) * (BK << sg) + ((ch * 8) << sg) + (pair ? 2 : 1) * (row & (rc - 1));
+        src_step = (ch_step * 8) << sg;
+        if (pair) sg = -sg;  // sign: pairs of neighbouring k
+      }
+    }
+    rounds = total / LOADERS;
+  }
+
+  __device__ __forceinline__ void get(const float* p, int c, float (&x)[8]) const {
+    if (RUNS || MODE == GENERIC) {
+      if (!RUNS || (nk & 15) == 0) {
+        const float4 lo = *reinterpret_cast<const float4*>(p), hi = *reinterpret_cast<const float4*>(p + 4);
+        x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w;
+        x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = c * 8 + e < nk ? p[e] : 0.f;
+      }
+    } else if (MODE == PIECES && sg <= 0) {  // groups of pairs: rc = 2^-sg rows
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        const float2 v = *reinterpret_cast<const float2*>(p + (e << -sg));
+        x[e] = v.x;
+        x[e + 1] = v.y;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = p[e << sg];
+    }
+  }
+  __device__ __forceinline__ uint8_t* at(uint8_t* sa, int u) const {
+    return RUNS ? sa + dst + u * dst_step : sa + dst + ((uint32_t)((ch + u * ch_step) ^ (int)dst_step) << 4);
+  }
+
+  __device__ __forceinline__ void run(uint8_t* sa, const float* stg, const Op& o, long long K, int mt, int kb, int i) {
+    if (rounds == 0 || mt >= m_full || kb >= kb_full) {
+      convert_any<R, MODE>(sa, stg, o, K, (long long)mt * R, kb, i);
+      return;
+    }
+    const float* p = stg + src;
+    constexpr int U = 2;  // chunks read before the first is stored
+    int u = 0;
+#pragma unroll 1
+    for (; u + U <= rounds; u += U, p += U * src_step) {
+      float x[U][8];
+#pragma unroll
+      for (int v = 0; v < U; ++v) get(p + v * src_step, ch, x[v]);
+#pragma unroll
+      for (int v = 0; v < U; ++v) put_chunk(at(sa, u + v), x[v]);
+    }
+    if (u < rounds) {
+      float x[8];
+      get(p, ch, x);
+      put_chunk(at(sa, u), x);
+    }
+  }
+};
 }  // namespace ws
 
 // 16 consecutive accumulator columns of this warp's 32 TMEM lanes (one per lane).
@@ -780,8 +800,8 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
   float* const epi_buf = stgb + D * C::BSLOT_FLOATS;
   __shared__ uint64_t full[ST], bfull[ST], empty[ST], afull[D], accf[2], acce[2], drain;
   __shared__ uint32_t tmem_base;
-  __shared__ long long off_s[ws::EPI_WARPS][32];  // epilogue: per warp, 32 row (or column) offsets
-  __shared__ float bias_s[ws::EPI_WARPS][32];
+  __shared__ long long off_s[2][ws::EPI_WARPS][32];  // epilogue: per warp, 32 row (or column) offsets
+  __shared__ float bias_s[2][ws::EPI_WARPS][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == ws::MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
@@ -833,6 +853,10 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
     auto load = [&](auto form_a, auto form_b) {
       constexpr int MA = decltype(form_a)::value;
       [[maybe_unused]] constexpr int MB = decltype(form_b)::value;
+      ws::Convert<BM, MA> conv_a;
+      conv_a.init(w.a, w.K, i);
+      ws::Convert<C::BROWS, FUSE ? MB : ws::ANY> conv_b;
+      if constexpr (FUSE) conv_b.init(w.b, w.K, i);
       Cur cur, ahead;
       cur.w.start(blockIdx.x, gridDim.x, w.ntiles, mtiles, w.splits);
       open(cur);
@@ -858,14 +882,13 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
         if (ok) {
           uint8_t* st = smem + s * C::STAGE_BYTES;
           if constexpr (FUSE) {
-            ws::convert_op<C::BROWS, MB>(st + A_BYTES, stgb + d * C::BSLOT_FLOATS, w.b, w.K, (long long)cur.w.nt * BN,
-                                         cur.kb, i);
+            conv_b.run(st + A_BYTES, stgb + d * C::BSLOT_FLOATS, w.b, w.K, cur.w.nt, cur.kb, i);
           } else if (i == 0) {
             mbar_expect_tx(&bfull[s], C::B_BYTES);
             bulk_g2s(st + A_BYTES, w.b_img + (((size_t)cur.w.bt * w.ntiles + cur.w.nt) * w.kblocks + cur.kb) * C::B_BYTES,
                      C::B_BYTES, &bfull[s]);
           }
-          ws::convert_op<BM, MA>(st, stg0 + d * ws::SLOT_FLOATS, w.a, w.K, (long long)cur.w.mt * BM, cur.kb, i);
+          conv_a.run(st, stg0 + d * ws::SLOT_FLOATS, w.a, w.K, cur.w.mt, cur.kb, i);
           fence_proxy_async();  // the tensor cores read the stage through the async proxy
           mbar_arrive(&full[s]);
           if (FUSE && i == 0) mbar_arrive(&bfull[s]);
@@ -1023,9 +1046,9 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
           const long long rbase = !row_ok ? -1
                                   : e.out.rc == 1 ? r * e.out.s1
                                                   : (r / e.out.rc) * e.out.s1 + (r % e.out.rc) * e.out.s2;
-          if constexpr (F != OUT_ROWS) off_s[wi][lane] = rbase;
+          if constexpr (F != OUT_ROWS) off_s[0][wi][lane] = rbase;
           __syncwarp();
-          for (int c0 = 0; ok && c0 < BN && nt * BN + c0 < e.N; c0 += 32) {
+          for (int c0 = 0; F != OUT_ROWS && ok && c0 < BN && nt * BN + c0 < e.N; c0 += 32) {
             const int c = nt * BN + c0 + lane;  // this lane's column
             const bool col_ok = c < e.N;
             if constexpr (F == OUT_VEC) {
@@ -1037,24 +1060,30 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
               const int lp = cols > 16 ? 3 : cols > 8 ? 2 : cols > 4 ? 1 : 0;
               const int q4 = (lane & ((1 << lp) - 1)) * 4, c4 = nt * BN + c0 + q4, row0 = lane >> lp, step = 32 >> lp;
               const bool c_ok = c4 < e.N;
-              long long o4[8];  // 1 << lp rounds of `step` rows
-              float4 prev[8];
-#pragma unroll
-              for (int u = 0; u < 8; ++u) {
+              auto offset = [&](int u) -> long long {  // 1 << lp rounds of `step` rows
                 const int row = u * step + row0;
-                const long long rb = off_s[wi][row & 31];
-                o4[u] = row < 32 && rb >= 0 && c_ok ? rb + c4 : -1;
-              }
-              if (have_prev) {
+                const long long rb = off_s[0][wi][row & 31];
+                return row < 32 && rb >= 0 && c_ok ? rb + c4 : -1;
+              };
+              float4 prev[4], next[4];
+              auto fetch = [&](float4 (&f)[4], int h) {
 #pragma unroll
-                for (int u = 0; u < 8; ++u) prev[u] = *reinterpret_cast<const float4*>(p1 + (o4[u] >= 0 ? o4[u] : 0));
+                for (int u = 0; u < 4; ++u) {
+                  const long long o = offset(h + u);
+                  f[u] = *reinterpret_cast<const float4*>(p1 + (o >= 0 ? o : 0));
+                }
                 if (both) {
 #pragma unroll
-                  for (int u = 0; u < 8; ++u) {
-                    const float4 y4 = *reinterpret_cast<const float4*>(ey + (o4[u] >= 0 ? o4[u] : 0));
-                    prev[u] = make_float4(prev[u].x + y4.x, prev[u].y + y4.y, prev[u].z + y4.z, prev[u].w + y4.w);
+                  for (int u = 0; u < 4; ++u) {
+                    const long long o = offset(h + u);
+                    const float4 y4 = *reinterpret_cast<const float4*>(ey + (o >= 0 ? o : 0));
+                    f[u] = make_float4(f[u].x + y4.x, f[u].y + y4.y, f[u].z + y4.z, f[u].w + y4.w);
                   }
                 }
+              };
+              if (have_prev) {
+                fetch(prev, 0);
+                if (lp == 3) fetch(next, 4);
               }
               float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
               if (e.bias && c_ok)
@@ -1063,17 +1092,25 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
               if (!ok) break;
               block_to_smem(c0);
               __syncwarp();
+#pragma unroll 1
+              for (int h = 0; h < (1 << lp); h += 4) {
 #pragma unroll
-              for (int u = 0; u < 8; ++u) {
-                if (o4[u] < 0) continue;
-                const float4 a4 = *reinterpret_cast<const float4*>(blk + (u * step + row0) * ws::EPI_LD + q4);
-                float4 z = make_float4(fmaf(a4.x, e.scale, b4.x), fmaf(a4.y, e.scale, b4.y), fmaf(a4.z, e.scale, b4.z),
-                                       fmaf(a4.w, e.scale, b4.w));
-                if (have_prev) z = make_float4(z.x + prev[u].x, z.y + prev[u].y, z.z + prev[u].z, z.w + prev[u].w);
-                *reinterpret_cast<float4*>(ey + o4[u]) = z;
-                if (eact)
-                  *reinterpret_cast<float4*>(eact + o4[u]) =
-                      make_float4(gelu_t(z.x), gelu_t(z.y), gelu_t(z.z), gelu_t(z.w));
+                for (int u = 0; u < 4; ++u) {
+                  const long long o = offset(h + u);
+                  if (o < 0) continue;
+                  const float4 a4 = *reinterpret_cast<const float4*>(blk + ((h + u) * step + row0) * ws::EPI_LD + q4);
+                  float4 z = make_float4(fmaf(a4.x, e.scale, b4.x), fmaf(a4.y, e.scale, b4.y),
+                                         fmaf(a4.z, e.scale, b4.z), fmaf(a4.w, e.scale, b4.w));
+                  if (have_prev) z = make_float4(z.x + prev[u].x, z.y + prev[u].y, z.z + prev[u].z, z.w + prev[u].w);
+                  *reinterpret_cast<float4*>(ey + o) = z;
+                  if (eact)
+                    *reinterpret_cast<float4*>(eact + o) =
+                        make_float4(gelu_t(z.x), gelu_t(z.y), gelu_t(z.z), gelu_t(z.w));
+                }
+                if (have_prev) {
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) prev[u] = next[u];
+                }
               }
               __syncwarp();
             } else if constexpr (F == OUT_COLS) {
@@ -1090,20 +1127,20 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                 if (have_prev) {
 #pragma unroll
                   for (int j = 0; j < 16; ++j) {
-                    const long long ro = off_s[wi][h + j];
+                    const long long ro = off_s[0][wi][h + j];
                     prev[j] = p1[(ro >= 0 && col_ok) ? ro + c : 0];
                   }
                   if (both) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                      const long long ro = off_s[wi][h + j];
+                      const long long ro = off_s[0][wi][h + j];
                       prev[j] += ey[(ro >= 0 && col_ok) ? ro + c : 0];
                     }
                   }
                 }
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                  const long long ro = off_s[wi][h + j];
+                  const long long ro = off_s[0][wi][h + j];
                   if (ro >= 0 && col_ok) {
                     float z = fmaf(blk[(h + j) * ws::EPI_LD + lane], e.scale, bias_c);
                     if (have_prev) z += prev[j];
@@ -1113,39 +1150,50 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                 }
               }
               __syncwarp();
-            } else {
-              // lanes along rows; the column offsets (this lane's for column c0 + lane) in shared memory
-              off_s[wi][lane] = !col_ok ? -1
-                                : e.out.kc == 1 ? (long long)c * e.out.t1
-                                                : (long long)(c / e.out.kc) * e.out.t1 + (long long)(c % e.out.kc) * e.out.t2;
-              bias_s[wi][lane] = (e.bias && col_ok) ? __ldg(e.bias + c) : 0.f;
+            }
+          }
+          if constexpr (F == OUT_ROWS) {
+            // Lanes along rows; the columns' offsets (this lane's for column c0 + lane) and
+            // biases in shared memory, two blocks deep: block c0 + 32's added values are
+            // requested before block c0 is finished.
+            auto columns = [&](int c0) {
+              const int c = nt * BN + c0 + lane, par = (c0 >> 5) & 1;
+              const bool col_ok = c0 < BN && c < e.N;
+              off_s[par][wi][lane] = !col_ok ? -1
+                                     : e.out.kc == 1
+                                         ? (long long)c * e.out.t1
+                                         : (long long)(c / e.out.kc) * e.out.t1 + (long long)(c % e.out.kc) * e.out.t2;
+              bias_s[par][wi][lane] = (e.bias && col_ok) ? __ldg(e.bias + c) : 0.f;
               __syncwarp();
-              float prev[32];
-              if (have_prev) {
+            };
+            auto fetch = [&](float (&f)[32], int c0) {
+              const long long* const co = off_s[(c0 >> 5) & 1][wi];
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                  const long long cj = off_s[wi][j];
-                  prev[j] = p1[(row_ok && cj >= 0) ? rbase + cj : 0];
-                }
-                if (both) {
+              for (int j = 0; j < 32; ++j) f[j] = p1[(row_ok && co[j] >= 0) ? rbase + co[j] : 0];
+              if (both) {
 #pragma unroll
-                  for (int j = 0; j < 32; ++j) {
-                    const long long cj = off_s[wi][j];
-                    prev[j] += ey[(row_ok && cj >= 0) ? rbase + cj : 0];
-                  }
-                }
+                for (int j = 0; j < 32; ++j) f[j] += ey[(row_ok && co[j] >= 0) ? rbase + co[j] : 0];
               }
-              if (c0 == 0) ok = landed();
-              if (!ok) break;
+            };
+            float prev[32], next[32];
+            columns(0);
+            if (have_prev) fetch(prev, 0);
+            ok = landed();
+#pragma unroll 1
+            for (int c0 = 0; ok && c0 < BN && nt * BN + c0 < e.N; c0 += 32) {
+              columns(c0 + 32);
+              if (have_prev && c0 + 32 < BN && nt * BN + c0 + 32 < e.N) fetch(next, c0 + 32);
+              const long long* const co = off_s[(c0 >> 5) & 1][wi];
+              const float* const bi = bias_s[(c0 >> 5) & 1][wi];
 #pragma unroll
               for (int h = 0; h < 32; h += 16) {
                 uint32_t v[16];
                 tmem_ld16(acc + (uint32_t)(c0 + h), v);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                  const long long cj = off_s[wi][h + j];
+                  const long long cj = co[h + j];
                   if (row_ok && cj >= 0) {
-                    float z = fmaf(__uint_as_float(v[j]), e.scale, bias_s[wi][h + j]);
+                    float z = fmaf(__uint_as_float(v[j]), e.scale, bi[h + j]);
                     if (have_prev) z += prev[h + j];
                     ey[rbase + cj] = z;
                     if (eact) eact[rbase + cj] = gelu_t(z);
@@ -1153,7 +1201,12 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                 }
               }
               __syncwarp();
+              if (have_prev) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) prev[j] = next[j];
+              }
             }
+            __syncwarp();
           }
         }
         if (!ok) break;
@@ -1315,8 +1368,8 @@ int TcGemm::run(const float* a, Addr aa, const float* b, Addr ba, long long M, i
   e.N = N;
   e.ybs = 0;
   tg::WsArgs w{};
-  w.a = tg::ws::Op{a, aa, 0, M, 0, 0};
-  w.b = tg::ws::Op{b, ba, 0, N, 0, 0};
+  w.a = tg::ws::Op{a, aa, 0, M, 0, 0, 0};
+  w.b = tg::ws::Op{b, ba, 0, N, 0, 0, 0};
   w.K = K;
   w.kblocks = kblocks;
   w.ntiles = ntiles;
@@ -1408,7 +1461,7 @@ int TcGemm::run_batched(const float* a, Addr aa, long long a_bs, const float* b,
   const uint8_t* bi = reinterpret_cast<const uint8_t*>(b_img);
   cudaError_t c;
   tg::WsArgs w{};
-  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0};
+  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0};
   w.b_img = bi;
   w.K = K;
   w.kblocks = kblocks;
@@ -1446,7 +1499,7 @@ int TcGemm::run_cplx(const float* a, Addr aa, long long a_bs, const float* src, 
   const uint8_t* bi = reinterpret_cast<const uint8_t*>(b_img);
   cudaError_t c;
   tg::WsArgs w{};
-  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0};
+  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0};
   w.b_img = bi;
   w.K = K;
   w.kblocks = kblocks;
