@@ -65,6 +65,7 @@ __global__ void colsum_part_kernel(const float* __restrict__ x, long long rows, 
   const long long r0 = (long long)blockIdx.x * chunk;
   const long long r1 = r0 + chunk < rows ? r0 + chunk : rows;
   float s = 0.f;
+#pragma unroll 16
   for (long long r = r0 + t / n; r < r1; r += step) s += x[r * n + c];
   red[t] = s;
   __syncthreads();
@@ -80,6 +81,7 @@ __global__ void reduce_parts_kernel(const float* __restrict__ part, int nchunks,
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   float s = 0.f;
+#pragma unroll 32
   for (int k = 0; k < nchunks; ++k) s += part[(size_t)k * n + j];
   out[j] = s;
 }

@@ -776,8 +776,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 // rounded like A.  With part set the epilogue writes raw partial tiles
 // part[((batch * splits + split) * tiles + tile) * 128 * BN + row * BN + col] instead.
 // Forms of the epilogue's output: raw partial tiles; columns contiguous in whole 16-byte
-// pieces; columns contiguous; any other layout, rows along the lanes.
-enum { OUT_PART, OUT_VEC, OUT_COLS, OUT_ROWS };
+// pieces; columns contiguous; any other layout, rows along the lanes; rows contiguous in
+// whole 16-byte pieces.
+enum { OUT_PART, OUT_VEC, OUT_COLS, OUT_ROWS, OUT_RVEC };
 
 struct WsArgs {
   ws::Op a, b;
@@ -786,7 +787,7 @@ struct WsArgs {
   int kblocks, kper, splits, ntiles;
   long long mtiles, items;
   float* part;
-  int vec;  // rows of the output (and of add, act) in whole 16-byte pieces
+  int form;  // of the output (and of add, act)
 };
 
 template <int BN, bool FUSE>
@@ -871,7 +872,7 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                                          (long long)ahead.w.mt * BM, ahead.kb, i);
           if constexpr (FUSE)
             cp |= ws::issue_op<C::BROWS, MB>(stgb + di * C::BSLOT_FLOATS, &afull[di], w.b, ahead.w.bt, w.K,
-                                             (long long)ahead.w.nt * BN, ahead.kb, i);
+                                             (long long)ahead.w.nt * BN, ahead.kb, i ^ 64);  // another warp's bulk copy
           if (cp) ws::cp_arrive(&afull[di]);
           else mbar_arrive(&afull[di]);
           if (++di == D) di = 0;
@@ -883,7 +884,7 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
           uint8_t* st = smem + s * C::STAGE_BYTES;
           if constexpr (FUSE) {
             conv_b.run(st + A_BYTES, stgb + d * C::BSLOT_FLOATS, w.b, w.K, cur.w.nt, cur.kb, i);
-          } else if (i == 0) {
+          } else if (i == 64) {
             mbar_expect_tx(&bfull[s], C::B_BYTES);
             bulk_g2s(st + A_BYTES, w.b_img + (((size_t)cur.w.bt * w.ntiles + cur.w.nt) * w.kblocks + cur.kb) * C::B_BYTES,
                      C::B_BYTES, &bfull[s]);
@@ -909,7 +910,7 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
         mbar_wait_bounded(&afull[d], dp);
         if (++d == D) { d = 0; dp ^= 1u; }
       }
-      if (i == 0 && !FUSE) {
+      if (i == 64 && !FUSE) {
         if (used == ST) sp ^= 1u;  // the last ST stages: s is the oldest of them
         else s = 0;
         for (int j = 0; j < used; ++j) {
@@ -1046,9 +1047,9 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
           const long long rbase = !row_ok ? -1
                                   : e.out.rc == 1 ? r * e.out.s1
                                                   : (r / e.out.rc) * e.out.s1 + (r % e.out.rc) * e.out.s2;
-          if constexpr (F != OUT_ROWS) off_s[0][wi][lane] = rbase;
+          if constexpr (F == OUT_VEC || F == OUT_COLS) off_s[0][wi][lane] = rbase;
           __syncwarp();
-          for (int c0 = 0; F != OUT_ROWS && ok && c0 < BN && nt * BN + c0 < e.N; c0 += 32) {
+          for (int c0 = 0; (F == OUT_VEC || F == OUT_COLS) && ok && c0 < BN && nt * BN + c0 < e.N; c0 += 32) {
             const int c = nt * BN + c0 + lane;  // this lane's column
             const bool col_ok = c < e.N;
             if constexpr (F == OUT_VEC) {
@@ -1152,7 +1153,7 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
               __syncwarp();
             }
           }
-          if constexpr (F == OUT_ROWS) {
+          if constexpr (F == OUT_ROWS || F == OUT_RVEC) {
             // Lanes along rows; the columns' offsets (this lane's for column c0 + lane) and
             // biases in shared memory, two blocks deep: block c0 + 32's added values are
             // requested before block c0 is finished.
@@ -1175,6 +1176,66 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                 for (int j = 0; j < 32; ++j) f[j] += ey[(row_ok && co[j] >= 0) ? rbase + co[j] : 0];
               }
             };
+            if constexpr (F == OUT_RVEC) {
+              // Four rows of a column are 16 bytes: the block goes through shared memory
+              // transposed, lane l takes rows 4 (l % 8) of columns 4 u + l / 8.
+              const int rl = (lane & 7) * 4, cl = lane >> 3;
+              const long long rb = __shfl_sync(0xffffffffu, rbase, rl);
+              auto fetch4 = [&](float4 (&f)[8], int c0) {
+                const long long* const co = off_s[(c0 >> 5) & 1][wi];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                  const long long c = co[u * 4 + cl];
+                  f[u] = *reinterpret_cast<const float4*>(p1 + (rb >= 0 && c >= 0 ? rb + c : 0));
+                }
+                if (both) {
+#pragma unroll
+                  for (int u = 0; u < 8; ++u) {
+                    const long long c = co[u * 4 + cl];
+                    const float4 y4 = *reinterpret_cast<const float4*>(ey + (rb >= 0 && c >= 0 ? rb + c : 0));
+                    f[u] = make_float4(f[u].x + y4.x, f[u].y + y4.y, f[u].z + y4.z, f[u].w + y4.w);
+                  }
+                }
+              };
+              float4 prev[8], next[8];
+              columns(0);
+              if (have_prev) fetch4(prev, 0);
+              ok = landed();
+#pragma unroll 1
+              for (int c0 = 0; ok && c0 < BN && nt * BN + c0 < e.N; c0 += 32) {
+                columns(c0 + 32);
+                if (have_prev && c0 + 32 < BN && nt * BN + c0 + 32 < e.N) fetch4(next, c0 + 32);
+                const long long* const co = off_s[(c0 >> 5) & 1][wi];
+                const float* const bi = bias_s[(c0 >> 5) & 1][wi];
+#pragma unroll
+                for (int h = 0; h < 32; h += 16) {
+                  uint32_t v[16];
+                  tmem_ld16(acc + (uint32_t)(c0 + h), v);
+#pragma unroll
+                  for (int j = 0; j < 16; ++j) blk[(h + j) * ws::EPI_LD + lane] = __uint_as_float(v[j]);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                  const long long c = co[u * 4 + cl];
+                  if (rb < 0 || c < 0) continue;
+                  const float4 a4 = *reinterpret_cast<const float4*>(blk + (u * 4 + cl) * ws::EPI_LD + rl);
+                  const float b = bi[u * 4 + cl];
+                  float4 z = make_float4(fmaf(a4.x, e.scale, b), fmaf(a4.y, e.scale, b), fmaf(a4.z, e.scale, b),
+                                         fmaf(a4.w, e.scale, b));
+                  if (have_prev) z = make_float4(z.x + prev[u].x, z.y + prev[u].y, z.z + prev[u].z, z.w + prev[u].w);
+                  *reinterpret_cast<float4*>(ey + rb + c) = z;
+                  if (eact)
+                    *reinterpret_cast<float4*>(eact + rb + c) =
+                        make_float4(gelu_t(z.x), gelu_t(z.y), gelu_t(z.z), gelu_t(z.w));
+                }
+                __syncwarp();
+                if (have_prev) {
+#pragma unroll
+                  for (int u = 0; u < 8; ++u) prev[u] = next[u];
+                }
+              }
+            } else {
             float prev[32], next[32];
             columns(0);
             if (have_prev) fetch(prev, 0);
@@ -1206,6 +1267,7 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                 for (int j = 0; j < 32; ++j) prev[j] = next[j];
               }
             }
+            }
             __syncwarp();
           }
         }
@@ -1215,10 +1277,13 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
         if (lane == 0) mbar_arrive(&acce[eg]);
       }
     };
-    if (w.part) finish(ws::Tag<OUT_PART>{});
-    else if (w.vec) finish(ws::Tag<OUT_VEC>{});
-    else if (e.out.kc == 1 && e.out.t1 == 1) finish(ws::Tag<OUT_COLS>{});
-    else finish(ws::Tag<OUT_ROWS>{});
+    switch (w.form) {
+      case OUT_PART: finish(ws::Tag<OUT_PART>{}); break;
+      case OUT_VEC: finish(ws::Tag<OUT_VEC>{}); break;
+      case OUT_COLS: finish(ws::Tag<OUT_COLS>{}); break;
+      case OUT_RVEC: finish(ws::Tag<OUT_RVEC>{}); break;
+      default: finish(ws::Tag<OUT_ROWS>{}); break;
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1266,8 +1331,13 @@ cudaError_t launch_ws_bn(WsArgs w, const Epi& e, int* err, cudaStream_t st, long
   ws::op_mode(w.a, BM, w.K);
   if (FUSE) ws::op_mode(w.b, BN, w.K);
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };  // null included
-  w.vec = e.out.kc == 1 && e.out.t1 == 1 && e.N % 4 == 0 && e.out.s1 % 4 == 0 && (e.out.rc == 1 || e.out.s2 % 4 == 0) &&
-          e.ybs % 4 == 0 && al(e.y) && al(e.add) && al(e.act);
+  const Addr& o = e.out;
+  const bool cols = o.kc == 1 && o.t1 == 1, whole = e.ybs % 4 == 0 && al(e.y) && al(e.add) && al(e.act);
+  const bool rows = o.rc == 1 ? o.s1 == 1 : o.s2 == 1 && o.rc % 4 == 0 && o.s1 % 4 == 0;
+  w.form = w.part ? OUT_PART
+           : cols ? (whole && e.N % 4 == 0 && o.s1 % 4 == 0 && (o.rc == 1 || o.s2 % 4 == 0) ? OUT_VEC : OUT_COLS)
+           : rows && whole && e.M % 4 == 0 && o.t1 % 4 == 0 && (o.kc == 1 || o.t2 % 4 == 0) ? OUT_RVEC
+                                                                                         : OUT_ROWS;
   w.items = batch * w.splits * w.mtiles * w.ntiles;
   const unsigned grid = (unsigned)std::min<long long>(w.items, slots);
   gemm_ws_kernel<BN, FUSE><<<grid, ws::THREADS, ws::Cfg<BN>::SMEM, st>>>(w, e, err);
