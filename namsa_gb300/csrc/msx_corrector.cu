@@ -285,11 +285,17 @@ Epi epi(float* y, Addr out) {
 
 // Pixel-major activation (S, H, W, C) as rows (s, y, c) x columns x.
 Addr rows_syc(const msx_corrector* k) { return Addr{(long long)k->W * k->C, 1, k->C, k->C, 0, 1}; }
-// Complex (S, H, C, MX) as rows (s, c, m) x columns (2 y + re/im).
-Addr rows_scm(const msx_corrector* k) {
+// The spectral arrays keep the channels innermost, so that every transform reads and
+// writes runs over the channels and the mixing reads a mode's channels as one run:
+//   U (S, H, MX, C) complex, parts interleaved; X, Y (S, MX, MY, 2, C), parts in planes.
+// U as rows (s, y, c) x columns (2 m + re/im), and as rows (s, m, c) x columns (2 y + re/im).
+Addr u_rows_syc(const msx_corrector* k) { return Addr{2LL * k->MX * k->C, 2, k->C, 2LL * k->C, 1, 2}; }
+Addr u_rows_smc(const msx_corrector* k) {
   const long long cm = (long long)k->C * k->MX;
   return Addr{(long long)k->H * cm * 2, 2, cm, cm * 2, 1, 2};
 }
+// X or Y as rows (s, m, c) x columns (2 n + re/im).
+Addr x_rows_smc(const msx_corrector* k) { return Addr{2LL * k->MY * k->C, 1, k->C, k->C, 0, 1}; }
 
 // out[j] = column sums of x (rows x n), n in {4, 32, 64, ...} dividing 256
 int colsum(msx_corrector* k, const float* x, long long rows, int n, float* out, cudaStream_t st) {
@@ -312,18 +318,13 @@ int wgrad(msx_corrector* k, const float* dY, int n_out, const float* X, int n_in
 
 // Per-mode channel mixing as batched tensor-core GEMMs, one batch per mode m, each
 // complex product as one real GEMM over [real, imaginary] planes (TcGemm::run_cplx).
-//   X, Y: (S, C, NM) complex (float index ((s C + c) NM + m) 2 + e); R: (NM, C, C) complex.
-// Rows s, columns (part, channel) of an (S, C, NM) complex array, for one mode.
-Addr modes_rows_s_parts(const msx_corrector* k) {
-  const long long nm2 = 2LL * k->MX * k->MY;
-  return Addr{(long long)k->C * nm2, 0, 1, 1, nm2, k->C};
-}
+//   X, Y: (S, NM, 2, C), parts in planes; R: (NM, C, C) complex, parts interleaved.
 
 // Y = R X per mode: [Yr, Yi] = [Xr, Xi] against rows [Rr, -Ri] and [Ri, Rr]
 int mix_forward(msx_corrector* k, const float* R, const float* X, int S, float* Y, cudaStream_t st) {
   const int C = k->C, NM = k->MX * k->MY;
-  const Addr xa = modes_rows_s_parts(k);
-  NN_GEMM(k->gemm.run_cplx(X, xa, 2, R, 2LL * C, 2, 2LL * C * C, C, C, 1, S, epi(Y, xa), 2, NM, st));
+  const Addr xa = rowmajor(2LL * NM * C);  // rows s, columns (part, channel)
+  NN_GEMM(k->gemm.run_cplx(X, xa, 2 * C, R, 2LL * C, 2, 1, 2LL * C * C, C, C, 1, S, epi(Y, xa), 2 * C, NM, st));
   return MSX_OK;
 }
 
@@ -332,15 +333,15 @@ int mix_forward(msx_corrector* k, const float* R, const float* X, int S, float* 
 int mix_backward(msx_corrector* k, const float* R, const float* X, const float* dY, int S, float* dX, float* dR,
                  cudaStream_t st) {
   const int C = k->C, NM = k->MX * k->MY;
-  const long long nm2 = 2LL * NM;
-  const Addr xa = modes_rows_s_parts(k);
+  const long long sx = 2LL * NM * C;  // from one sample to the next
+  const Addr xa = rowmajor(sx);
   // dX: rows s, K = (part, o) of dY; B row (part, c), column (part', o) = R[o][c] (xor), - for (1, 0)
-  NN_GEMM(k->gemm.run_cplx(dY, xa, 2, R, 2, 2LL * C, 2LL * C * C, C, C, 2, S, epi(dX, xa), 2, NM, st));
+  NN_GEMM(k->gemm.run_cplx(dY, xa, 2 * C, R, 2, 2LL * C, 1, 2LL * C * C, C, C, 2, S, epi(dX, xa), 2 * C, NM, st));
   // dR: rows o, K = (part, s) of dY; B row (part, c), column (part', s) = X[s][c] (xor), - for (1, 0);
   // out (o, part, c) in R's layout
-  const Addr ya = Addr{nm2, 0, 1, 1, (long long)C * nm2, S};
+  const Addr ya = Addr{1, 0, 1, C, sx, S};
   const Addr ro = Addr{2LL * C, 0, 1, 1, 2, C};
-  NN_GEMM(k->gemm.run_cplx(dY, ya, 2, X, nm2, (long long)C * nm2, 2, C, S, 2, C, epi(dR, ro), 2LL * C * C, NM, st));
+  NN_GEMM(k->gemm.run_cplx(dY, ya, 2 * C, X, 1, sx, C, 2 * C, C, S, 2, C, epi(dR, ro), 2LL * C * C, NM, st));
   return MSX_OK;
 }
 
@@ -360,21 +361,21 @@ int forward(msx_corrector* k, int S, cudaStream_t st) {
     float* aout = k->a + (size_t)(l + 1) * A;
     float* zl = k->z + (size_t)l * A;
     float* Xl = k->Xh + (size_t)l * x_words(k, S);
-    // DFT along x: rows (s, y, c), K = W -> U1 (S, H, C, MX) complex
+    // DFT along x: rows (s, y, c), K = W -> U1
     NN_GEMM(k->gemm.run(ain, rows_syc(k), k->Bdx, rowmajor(W), (long long)S * H * C, 2 * MX, W,
-                        epi(k->U1, rowmajor(2 * MX)), st));
-    // DFT along y: rows (s, c, m), K = 2H -> X (S, C, MX, MY) complex
-    NN_GEMM(k->gemm.run(k->U1, rows_scm(k), k->Bdy, rowmajor(2 * H), (long long)S * C * MX, 2 * MY, 2 * H,
-                        epi(Xl, rowmajor(2 * MY)), st));
+                        epi(k->U1, u_rows_syc(k)), st));
+    // DFT along y: rows (s, m, c), K = 2H -> X
+    NN_GEMM(k->gemm.run(k->U1, u_rows_smc(k), k->Bdy, rowmajor(2 * H), (long long)S * C * MX, 2 * MY, 2 * H,
+                        epi(Xl, x_rows_smc(k)), st));
     {
       const int rc = mix_forward(k, Pm + k->oR[l], Xl, S, k->Yh, st);
       if (rc) return rc;
     }
-    // inverse DFT along y: rows (s, o, m), K = 2 MY -> U2 (S, H, C, MX) complex
-    NN_GEMM(k->gemm.run(k->Yh, rowmajor(2 * MY), k->Biy, rowmajor(2 * MY), (long long)S * C * MX, 2 * H, 2 * MY,
-                        epi(k->U2, rows_scm(k)), st));
+    // inverse DFT along y: rows (s, m, o), K = 2 MY -> U2
+    NN_GEMM(k->gemm.run(k->Yh, x_rows_smc(k), k->Biy, rowmajor(2 * MY), (long long)S * C * MX, 2 * H, 2 * MY,
+                        epi(k->U2, u_rows_smc(k)), st));
     // inverse DFT along x (real part, 1/(H W) folded in): rows (s, y, o), K = 2 MX -> z_l pixel-major
-    NN_GEMM(k->gemm.run(k->U2, rowmajor(2 * MX), k->Bix, rowmajor(2 * MX), (long long)S * H * C, W, 2 * MX,
+    NN_GEMM(k->gemm.run(k->U2, u_rows_syc(k), k->Bix, rowmajor(2 * MX), (long long)S * H * C, W, 2 * MX,
                         epi(zl, rows_syc(k)), st));
     // pointwise layer: z_l += a W_l^T + b_l; a_l = gelu(z_l)
     Epi e = epi(zl, rowmajor(C));
@@ -430,17 +431,17 @@ int backward(msx_corrector* k, const float* dmaps, cudaStream_t st) {
     NN_GEMM(k->gemm.run(k->dz, rowmajor(C), Pm + k->oW[l], colmajor(C), SP, C, C, epi(k->da2, rowmajor(C)), st));
     // spectral part, in reverse: IDFT_x^T, IDFT_y^T, mixing, DFT_y^T, DFT_x^T
     NN_GEMM(k->gemm.run(k->dz, rows_syc(k), k->Bix, colmajor(2 * MX), (long long)S * H * C, 2 * MX, W,
-                        epi(k->U2, rowmajor(2 * MX)), st));
-    NN_GEMM(k->gemm.run(k->U2, rows_scm(k), k->Biy, colmajor(2 * MY), (long long)S * C * MX, 2 * MY, 2 * H,
-                        epi(k->Yh, rowmajor(2 * MY)), st));
-    // dX (S, C, MX, MY) complex into U1's space; dR into the gradients
+                        epi(k->U2, u_rows_syc(k)), st));
+    NN_GEMM(k->gemm.run(k->U2, u_rows_smc(k), k->Biy, colmajor(2 * MY), (long long)S * C * MX, 2 * MY, 2 * H,
+                        epi(k->Yh, x_rows_smc(k)), st));
+    // dX (laid out like X) into U1's space; dR into the gradients
     if ((rc = mix_backward(k, Pm + k->oR[l], Xl, k->Yh, S, k->U1, G + k->oR[l], st))) return rc;
-    // dX -> dU1 (S, H, C, MX): write into U2 (free now)
-    NN_GEMM(k->gemm.run(k->U1, rowmajor(2 * MY), k->Bdy, colmajor(2 * H), (long long)S * C * MX, 2 * H, 2 * MY,
-                        epi(k->U2, rows_scm(k)), st));
+    // dX -> dU1: write into U2 (free now)
+    NN_GEMM(k->gemm.run(k->U1, x_rows_smc(k), k->Bdy, colmajor(2 * H), (long long)S * C * MX, 2 * H, 2 * MY,
+                        epi(k->U2, u_rows_smc(k)), st));
     Epi e = epi(k->da2, rows_syc(k));
     e.accumulate = 1;
-    NN_GEMM(k->gemm.run(k->U2, rowmajor(2 * MX), k->Bdx, colmajor(W), (long long)S * H * C, W, 2 * MX, e, st));
+    NN_GEMM(k->gemm.run(k->U2, u_rows_syc(k), k->Bdx, colmajor(W), (long long)S * H * C, W, 2 * MX, e, st));
     std::swap(k->da, k->da2);
   }
   // lift: a_0 = x W0^T + b0 (no activation)

@@ -114,13 +114,13 @@ __global__ void pack_kernel(const float* __restrict__ src, Addr a, long long row
 
 // Real embedding of a complex product, packed like pack_kernel: B is N x K with
 // N = 2 hn, K = 2 hk; row n = (bn, i) = (n / hn, n % hn), column k = (bk, j); the
-// element is src[i si + j sj + (bn xor bk)] (a complex array, parts interleaved),
+// element is src[i si + j sj + (bn xor bk) sp] (a complex array, its parts sp apart),
 // negated where (bn, bk) = (0, 1) (neg = 1) or (1, 0) (neg = 2).  With the
 // right orientation of src, D = A B^T then gives real and imaginary parts of a
 // complex product in one GEMM: [Re, Im] of x z^T is [xr, xi] against rows
 // [zr, -zi] and [zi, zr].
-__global__ void pack_cplx_kernel(const float* __restrict__ src, long long si, long long sj, long long src_bs, int hn,
-                                 int hk, int neg, int tile_rows, int rows_pad, int kblocks, uint4* __restrict__ img,
+__global__ void pack_cplx_kernel(const float* __restrict__ src, long long si, long long sj, long long sp,
+                                 long long src_bs, int hn, int hk, int neg, int tile_rows, int rows_pad, int kblocks, uint4* __restrict__ img,
                                  int batch) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long chunks = (long long)kblocks * (BK / 8);
@@ -130,8 +130,9 @@ __global__ void pack_cplx_kernel(const float* __restrict__ src, long long si, lo
   i -= bt * per;
   src += bt * src_bs;
   img += bt * (per * 8 * 2 / 16);
-  const int r = (int)(i / chunks);
-  const int ch = (int)(i - (long long)r * chunks);
+  // neighbouring threads along whichever index is nearer in src
+  const int r = si < sj ? (int)(i % rows_pad) : (int)(i / chunks);
+  const int ch = si < sj ? (int)(i / rows_pad) : (int)(i - (long long)r * chunks);
   const int k0 = ch * 8;
   __align__(16) __nv_bfloat16 v[8];
   const int N = 2 * hn, K = 2 * hk;
@@ -142,7 +143,7 @@ __global__ void pack_cplx_kernel(const float* __restrict__ src, long long si, lo
     float x = 0.f;
     if (r < N && k < K) {
       const int bk = k / hk, jj = k - bk * hk;
-      x = __ldg(src + ii * si + jj * sj + (bn ^ bk));
+      x = __ldg(src + ii * si + jj * sj + (bn ^ bk) * sp);
       if ((neg == 1 && bn == 0 && bk == 1) || (neg == 2 && bn == 1 && bk == 0)) x = -x;
     }
     v[j] = __float2bfloat16_rn(x);
@@ -463,10 +464,10 @@ struct Walk {
 //   GROUPRUN rows contiguous in groups of rc with k stride rc (a group's K block is one
 //            run of nk * rc values; rc may be all the operand's rows): thread i < R / rc
 //            copies group i to slot[i * 64 rc ..], element (k, r mod rc) at k rc + r mod rc;
-//   PIECES   rows contiguous in groups of rc at any k stride, each with its kc = 1 or 2
-//            neighbouring k values: 16-byte asynchronous copies dealt over all threads,
-//            group i to slot[i * 64 rc ..], element (k, r mod rc) at
-//            ((k / kc) rc + r mod rc) kc + k mod kc (GROUPRUN's layout for kc = 1);
+//   PIECES   rows contiguous in groups of rc at any k strides, or (pair) with two
+//            neighbouring k values to each row: 16-byte asynchronous copies dealt over all
+//            threads, group i to slot[i * 64 rc ..], element (k, r mod rc) as in GROUPRUN
+//            or (pair) at ((k / 2) rc + r mod rc) 2 + k mod 2;
 //   GENERIC  value by value (4-byte asynchronous copies), a row's values dealt over the
 //            threads that have no row of their own, element (r, k) at ((k / 8) R + i) 8 + k mod 8;
 //   TILERUN  rows of K <= 64 values stored back to back: thread 0 copies the tile's rows
@@ -493,6 +494,7 @@ struct Op {
   long long rows;  // M or N
   int mode, rc;    // rc: rows of a group (GROUPRUN, PIECES)
   int whole;       // TILERUN: every full tile is one 16-byte aligned run
+  int pair;        // PIECES: two neighbouring k values to a row
 };
 
 __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total) {
@@ -500,6 +502,7 @@ __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total)
   o.rc = (int)a.rc;
   o.mode = GENERIC;
   o.whole = 0;
+  o.pair = 0;
   const bool aligned = o.bs % 4 == 0 && (reinterpret_cast<uintptr_t>(o.p) & 15u) == 0;
   if (a.kc == 1 && a.t1 == 1) {
     o.mode = ROWRUN;
@@ -518,15 +521,16 @@ __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total)
     o.rc = (int)g;
     return;
   }
-  // groups that divide the tile or are divided by it
+  // groups of the tile that lie within the operand's
   const bool pair = a.kc == 2 && a.t2 == 1 && a.s2 == 2 && a.rc > 1;
   if (pair) g = a.rc;
-  if (g > 0 && (pair || a.kc == 1) && aligned && a.t1 % 4 == 0 && k_total % a.kc == 0 && o.rows % g == 0 &&
+  if (g > 0 && aligned && a.t1 % 4 == 0 && (pair ? k_total % 2 == 0 : a.kc == 1 || a.t2 % 4 == 0) &&
       (g == o.rows || a.s1 % 4 == 0)) {
-    const long long in = g < tile_rows ? g : tile_rows;
-    if (in * a.kc % 4 == 0 && tile_rows % in == 0 && g % in == 0) {
+    const long long in = (g & -g) < tile_rows ? g & -g : tile_rows;  // a power of two, as the tile
+    if (in * (pair ? 2 : 1) % 4 == 0 && o.rows % in == 0) {
       o.mode = PIECES;
       o.rc = (int)in;
+      o.pair = pair;
     }
   }
 }
@@ -582,21 +586,22 @@ __device__ __forceinline__ bool issue_op(float* stg, uint64_t* bar, const Op& o,
     return false;
   }
   if (mode == PIECES) {
-    const int rc = o.rc, run = (rc * (int)a.kc) >> 2;  // 16-byte pieces of a run
-    const int ks = a.kc == 2 ? 1 : 0;
-    const int pieces = (nk >> ks) * run;               // of a group
-    if ((run & (run - 1)) == 0 && run <= LOADERS) {
-      const int sr = 31 - __clz(run);
-      const long long step = (long long)(LOADERS >> sr) * a.t1;
-      for (int g = 0; g * rc < R && r0 + g * rc < o.rows; ++g) {
-        const float* src = P + row_off(r0 + g * rc) + ((kb0 >> ks) + (i >> sr)) * a.t1 + (i & (run - 1)) * 4;
-        float* dst = stg + g * rc * BK + i * 4;
+    const int rc = o.rc, ks = o.pair ? 1 : 0, run = (rc << ks) >> 2;  // 16-byte pieces of a run, a power of two
+    const int pieces = (nk >> ks) * run;                              // of a group
+    const int sr = 31 - __clz(run);
+    const long long step = (long long)(LOADERS >> sr) * a.t1;
+    for (int g = 0; g * rc < R && r0 + g * rc < o.rows; ++g) {
+      const float* src = P + row_off(r0 + g * rc) + (i & (run - 1)) * 4;
+      float* dst = stg + g * rc * BK + i * 4;
+      if (o.pair || a.kc == 1) {
+        src += ((kb0 >> ks) + (i >> sr)) * a.t1;
         for (int j = i; j < pieces; j += LOADERS, src += step, dst += LOADERS * 4) cp16(dst, src);
+      } else {
+        for (int j = i; j < pieces; j += LOADERS, dst += LOADERS * 4) {
+          const long long k = kb0 + (j >> sr), q = k / a.kc;
+          cp16(dst, src + q * a.t1 + (k - q * a.kc) * a.t2);
+        }
       }
-    } else {
-      for (int g = 0; g * rc < R && r0 + g * rc < o.rows; ++g)
-        for (int j = i; j < pieces; j += LOADERS)
-          cp16(stg + g * rc * BK + j * 4, P + row_off(r0 + g * rc) + ((kb0 >> ks) + j / run) * a.t1 + (j % run) * 4);
     }
     return true;
   }
@@ -646,7 +651,7 @@ __device__ __forceinline__ void convert_any(uint8_t* sa, const float* stg, const
   const int nch = nk >= BK ? 8 : 2 * ((nk + 15) / 16);  // chunks the MMAs read
   const int nrow = (int)(o.rows - r0 < R ? o.rows - r0 : R);  // rows to convert
   const int mode = MODE == ANY ? o.mode : MODE, rc = o.rc;
-  const bool runs = mode == ROWRUN || mode == TILERUN, pair = mode == PIECES && o.a.kc == 2;
+  const bool runs = mode == ROWRUN || mode == TILERUN, pair = mode == PIECES && o.pair;
   for (int t = i; t < nrow * nch; t += LOADERS) {  // chunk fastest where k is contiguous, else row
     const int row = runs ? t / nch : t % nrow, ch = runs ? t % nch : t / nrow;
     const float* src = runs              ? stg + row * (mode == ROWRUN ? BK : nk) + ch * 8
@@ -698,7 +703,7 @@ struct Convert {
       } else {
         if ((rc & (rc - 1)) != 0) return;
         sg = 31 - __clz(rc);
-        const bool pair = MODE == PIECES && o.a.kc == 2;
+        const bool pair = MODE == PIECES && o.pair;
         src = (row >> sg) * (BK << sg) + ((ch * 8) << sg) + (pair ? 2 : 1) * (row & (rc - 1));
         src_step = (ch_step * 8) << sg;
         if (pair) sg = -sg;  // sign: pairs of neighbouring k
@@ -776,9 +781,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 // rounded like A.  With part set the epilogue writes raw partial tiles
 // part[((batch * splits + split) * tiles + tile) * 128 * BN + row * BN + col] instead.
 // Forms of the epilogue's output: raw partial tiles; columns contiguous in whole 16-byte
-// pieces; columns contiguous; any other layout, rows along the lanes; rows contiguous in
-// whole 16-byte pieces.
-enum { OUT_PART, OUT_VEC, OUT_COLS, OUT_ROWS, OUT_RVEC };
+// pieces; columns along the lanes (contiguous, or nearer than rows); any other layout, rows
+// along the lanes; rows contiguous in whole 16-byte pieces; pairs of columns within
+// contiguous rows (complex values).
+enum { OUT_PART, OUT_VEC, OUT_COLS, OUT_ROWS, OUT_RVEC, OUT_PAIR };
 
 struct WsArgs {
   ws::Op a, b;
@@ -1115,8 +1121,10 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
               }
               __syncwarp();
             } else if constexpr (F == OUT_COLS) {
-              // columns contiguous in the output: the block goes through shared memory and
-              // each row is stored with the lanes along its columns
+              // the block goes through shared memory and each row is stored with the lanes
+              // along its columns
+              const long long cc = e.out.kc == 1 ? (long long)c * e.out.t1
+                                                 : (long long)(c / e.out.kc) * e.out.t1 + (long long)(c % e.out.kc) * e.out.t2;
               if (c0 == 0) ok = landed();
               if (!ok) break;
               block_to_smem(c0);
@@ -1129,13 +1137,13 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
 #pragma unroll
                   for (int j = 0; j < 16; ++j) {
                     const long long ro = off_s[0][wi][h + j];
-                    prev[j] = p1[(ro >= 0 && col_ok) ? ro + c : 0];
+                    prev[j] = p1[(ro >= 0 && col_ok) ? ro + cc : 0];
                   }
                   if (both) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                       const long long ro = off_s[0][wi][h + j];
-                      prev[j] += ey[(ro >= 0 && col_ok) ? ro + c : 0];
+                      prev[j] += ey[(ro >= 0 && col_ok) ? ro + cc : 0];
                     }
                   }
                 }
@@ -1145,15 +1153,15 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                   if (ro >= 0 && col_ok) {
                     float z = fmaf(blk[(h + j) * ws::EPI_LD + lane], e.scale, bias_c);
                     if (have_prev) z += prev[j];
-                    ey[ro + c] = z;
-                    if (eact) eact[ro + c] = gelu_t(z);
+                    ey[ro + cc] = z;
+                    if (eact) eact[ro + cc] = gelu_t(z);
                   }
                 }
               }
               __syncwarp();
             }
           }
-          if constexpr (F == OUT_ROWS || F == OUT_RVEC) {
+          if constexpr (F == OUT_ROWS || F == OUT_RVEC || F == OUT_PAIR) {
             // Lanes along rows; the columns' offsets (this lane's for column c0 + lane) and
             // biases in shared memory, two blocks deep: block c0 + 32's added values are
             // requested before block c0 is finished.
@@ -1176,10 +1184,12 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                 for (int j = 0; j < 32; ++j) f[j] += ey[(row_ok && co[j] >= 0) ? rbase + co[j] : 0];
               }
             };
-            if constexpr (F == OUT_RVEC) {
-              // Four rows of a column are 16 bytes: the block goes through shared memory
-              // transposed, lane l takes rows 4 (l % 8) of columns 4 u + l / 8.
-              const int rl = (lane & 7) * 4, cl = lane >> 3;
+            if constexpr (F == OUT_RVEC || F == OUT_PAIR) {
+              // Four rows of a column (two rows of a pair of columns) are 16 bytes: the block
+              // goes through shared memory transposed, lane l takes rows 4 (l % 8) of columns
+              // 4 u + l / 8 (rows 2 (l % 16) of the pairs of columns 2 u + l / 16).
+              constexpr bool PAIR = F == OUT_PAIR;
+              const int rl = PAIR ? (lane & 15) * 2 : (lane & 7) * 4, cl = PAIR ? (lane >> 4) * 2 : lane >> 3;
               const long long rb = __shfl_sync(0xffffffffu, rbase, rl);
               auto fetch4 = [&](float4 (&f)[8], int c0) {
                 const long long* const co = off_s[(c0 >> 5) & 1][wi];
@@ -1219,10 +1229,20 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                 for (int u = 0; u < 8; ++u) {
                   const long long c = co[u * 4 + cl];
                   if (rb < 0 || c < 0) continue;
-                  const float4 a4 = *reinterpret_cast<const float4*>(blk + (u * 4 + cl) * ws::EPI_LD + rl);
+                  const float* const q = blk + (u * 4 + cl) * ws::EPI_LD + rl;
                   const float b = bi[u * 4 + cl];
-                  float4 z = make_float4(fmaf(a4.x, e.scale, b), fmaf(a4.y, e.scale, b), fmaf(a4.z, e.scale, b),
-                                         fmaf(a4.w, e.scale, b));
+                  float4 z;
+                  if (PAIR) {
+                    const float2 x = *reinterpret_cast<const float2*>(q);
+                    const float2 y = *reinterpret_cast<const float2*>(q + ws::EPI_LD);
+                    const float b1 = bi[u * 4 + cl + 1];
+                    z = make_float4(fmaf(x.x, e.scale, b), fmaf(y.x, e.scale, b1), fmaf(x.y, e.scale, b),
+                                    fmaf(y.y, e.scale, b1));
+                  } else {
+                    const float4 x = *reinterpret_cast<const float4*>(q);
+                    z = make_float4(fmaf(x.x, e.scale, b), fmaf(x.y, e.scale, b), fmaf(x.z, e.scale, b),
+                                    fmaf(x.w, e.scale, b));
+                  }
                   if (have_prev) z = make_float4(z.x + prev[u].x, z.y + prev[u].y, z.z + prev[u].z, z.w + prev[u].w);
                   *reinterpret_cast<float4*>(ey + rb + c) = z;
                   if (eact)
@@ -1282,6 +1302,7 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
       case OUT_VEC: finish(ws::Tag<OUT_VEC>{}); break;
       case OUT_COLS: finish(ws::Tag<OUT_COLS>{}); break;
       case OUT_RVEC: finish(ws::Tag<OUT_RVEC>{}); break;
+      case OUT_PAIR: finish(ws::Tag<OUT_PAIR>{}); break;
       default: finish(ws::Tag<OUT_ROWS>{}); break;
     }
   }
@@ -1334,8 +1355,11 @@ cudaError_t launch_ws_bn(WsArgs w, const Epi& e, int* err, cudaStream_t st, long
   const Addr& o = e.out;
   const bool cols = o.kc == 1 && o.t1 == 1, whole = e.ybs % 4 == 0 && al(e.y) && al(e.add) && al(e.act);
   const bool rows = o.rc == 1 ? o.s1 == 1 : o.s2 == 1 && o.rc % 4 == 0 && o.s1 % 4 == 0;
+  const bool pair = o.kc == 2 && o.t2 == 1 && o.s2 == 2 && o.rc > 1 && o.rc % 2 == 0;
   w.form = w.part ? OUT_PART
            : cols ? (whole && e.N % 4 == 0 && o.s1 % 4 == 0 && (o.rc == 1 || o.s2 % 4 == 0) ? OUT_VEC : OUT_COLS)
+           : o.kc >= 32 && o.t2 < (o.rc == 1 ? o.s1 : o.s2) ? OUT_COLS
+           : pair && whole && e.M % 2 == 0 && e.N % 2 == 0 && o.t1 % 4 == 0 && o.s1 % 4 == 0 ? OUT_PAIR
            : rows && whole && e.M % 4 == 0 && o.t1 % 4 == 0 && (o.kc == 1 || o.t2 % 4 == 0) ? OUT_RVEC
                                                                                          : OUT_ROWS;
   w.items = batch * w.splits * w.mtiles * w.ntiles;
@@ -1438,8 +1462,8 @@ int TcGemm::run(const float* a, Addr aa, const float* b, Addr ba, long long M, i
   e.N = N;
   e.ybs = 0;
   tg::WsArgs w{};
-  w.a = tg::ws::Op{a, aa, 0, M, 0, 0, 0};
-  w.b = tg::ws::Op{b, ba, 0, N, 0, 0, 0};
+  w.a = tg::ws::Op{a, aa, 0, M, 0, 0, 0, 0};
+  w.b = tg::ws::Op{b, ba, 0, N, 0, 0, 0, 0};
   w.K = K;
   w.kblocks = kblocks;
   w.ntiles = ntiles;
@@ -1531,7 +1555,7 @@ int TcGemm::run_batched(const float* a, Addr aa, long long a_bs, const float* b,
   const uint8_t* bi = reinterpret_cast<const uint8_t*>(b_img);
   cudaError_t c;
   tg::WsArgs w{};
-  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0};
+  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0, 0};
   w.b_img = bi;
   w.K = K;
   w.kblocks = kblocks;
@@ -1543,7 +1567,7 @@ int TcGemm::run_batched(const float* a, Addr aa, long long a_bs, const float* b,
   return c == cudaSuccess ? MSX_OK : MSX_ERR_CUDA;
 }
 
-int TcGemm::run_cplx(const float* a, Addr aa, long long a_bs, const float* src, long long si, long long sj,
+int TcGemm::run_cplx(const float* a, Addr aa, long long a_bs, const float* src, long long si, long long sj, long long sp,
                      long long src_bs, int hn, int hk, int neg, long long M, const Epi& epi, long long y_bs, int batch,
                      cudaStream_t st) {
   if (batch < 1 || M <= 0 || hn <= 0 || hk <= 0 || 2 * hn > 4096 || neg < 0 || neg > 2) return MSX_ERR_INVALID;
@@ -1559,7 +1583,7 @@ int TcGemm::run_cplx(const float* a, Addr aa, long long a_bs, const float* src, 
   if (rc != MSX_OK) return rc;
   const int b_rows = ntiles * bn;
   const long long b_thr = (long long)b_rows * kblocks * (tg::BK / 8) * batch;
-  tg::pack_cplx_kernel<<<(unsigned)((b_thr + 255) / 256), 256, 0, st>>>(src, si, sj, src_bs, hn, hk, neg, bn, b_rows,
+  tg::pack_cplx_kernel<<<(unsigned)((b_thr + 255) / 256), 256, 0, st>>>(src, si, sj, sp, src_bs, hn, hk, neg, bn, b_rows,
                                                                         kblocks, reinterpret_cast<uint4*>(b_img),
                                                                         batch);
   Epi e = epi;
@@ -1569,7 +1593,7 @@ int TcGemm::run_cplx(const float* a, Addr aa, long long a_bs, const float* src, 
   const uint8_t* bi = reinterpret_cast<const uint8_t*>(b_img);
   cudaError_t c;
   tg::WsArgs w{};
-  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0};
+  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0, 0};
   w.b_img = bi;
   w.K = K;
   w.kblocks = kblocks;
