@@ -368,7 +368,9 @@ namespace ws {
 constexpr int LOADERS = 128;  // warps 0-3
 constexpr int EPI_WARPS = 8;  // warps 4-11
 constexpr int MMA_WARP = 12;
-constexpr int THREADS = 16 * 32;  // warps 13-15 idle: registers move between groups of four warps
+constexpr int COPY_WARP = 13;   // bulk copies of FP32 operands
+constexpr int IMAGE_WARP = 14;  // bulk copies of the packed B
+constexpr int THREADS = 16 * 32;  // warp 15 idle: registers move between groups of four warps
 constexpr int SLOT_FLOATS = BM * BK;  // one FP32 staging slot (32 KB)
 constexpr int EPI_LD = 36;                // row stride of a warp's 32 x 32 block: 16-byte aligned, conflict-free
 constexpr int EPI_BLOCK = 32 * EPI_LD;
@@ -495,6 +497,7 @@ struct Op {
   int mode, rc;    // rc: rows of a group (GROUPRUN, PIECES)
   int whole;       // TILERUN: every full tile is one 16-byte aligned run
   int pair;        // PIECES: two neighbouring k values to a row
+  int bulk;        // every block arrives by bulk copies of one warp (issue_bulk)
 };
 
 __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total) {
@@ -503,11 +506,13 @@ __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total)
   o.mode = GENERIC;
   o.whole = 0;
   o.pair = 0;
+  o.bulk = 0;
   const bool aligned = o.bs % 4 == 0 && (reinterpret_cast<uintptr_t>(o.p) & 15u) == 0;
   if (a.kc == 1 && a.t1 == 1) {
     o.mode = ROWRUN;
     if (a.rc == 1 && k_total <= BK && a.s1 == k_total) o.mode = TILERUN;
     o.whole = aligned;
+    o.bulk = o.mode == TILERUN && aligned && o.rows * k_total % 4 == 0;
     return;
   }
   long long g = -1;
@@ -519,6 +524,7 @@ __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total)
       o.rows % g == 0 && (g == o.rows || a.s1 % 4 == 0) && aligned) {
     o.mode = GROUPRUN;
     o.rc = (int)g;
+    o.bulk = tile_rows / o.rc <= 32;
     return;
   }
   // groups of the tile that lie within the operand's
@@ -533,6 +539,27 @@ __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total)
       o.pair = pair;
     }
   }
+}
+
+// One warp's bulk copies of a block of a `bulk` operand (TILERUN or GROUPRUN): its bytes,
+// or with `go` the copies themselves (lane l the l-th group).
+template <int R>
+__device__ __forceinline__ uint32_t bulk_block(float* stg, uint64_t* bar, const Op& o, int bt, long long K, long long r0,
+                                               int kb, int lane, bool go) {
+  const long long kb0 = (long long)kb * BK, left = o.rows - r0;
+  const int nk = (int)(K - kb0 < BK ? K - kb0 : BK), nrow = (int)(left < R ? left : R);
+  if (nrow <= 0) return 0;
+  const uint32_t bytes = (uint32_t)(nrow * nk) * 4u;
+  if (!go) return bytes;
+  const float* const P = o.p + bt * o.bs;
+  if (o.mode == TILERUN) {
+    if (lane == 0) bulk_g2s(stg, P + r0 * o.a.s1, bytes, bar);
+  } else if (lane * o.rc < nrow) {
+    const long long r = r0 + lane * o.rc;
+    const long long off = o.a.rc == 1 ? r * o.a.s1 : (r / o.a.rc) * o.a.s1 + (r % o.a.rc) * o.a.s2;
+    bulk_g2s(stg + lane * BK * o.rc, P + off + kb0 * o.a.t1, (uint32_t)nk * (uint32_t)o.rc * 4u, bar);
+  }
+  return bytes;
 }
 
 // The loader threads' copies of rows r0 .. r0 + R - 1 of operand o (batch bt) into slot
@@ -805,7 +832,7 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
   float* const stg0 = reinterpret_cast<float*>(smem + ST * C::STAGE_BYTES);
   float* const stgb = stg0 + D * ws::SLOT_FLOATS;  // B staging (BN = 32 only)
   float* const epi_buf = stgb + D * C::BSLOT_FLOATS;
-  __shared__ uint64_t full[ST], bfull[ST], empty[ST], afull[D], accf[2], acce[2], drain;
+  __shared__ uint64_t full[ST], bfull[ST], empty[ST], afull[D], afree[D], accf[2], acce[2], drain;
   __shared__ uint32_t tmem_base;
   __shared__ long long off_s[2][ws::EPI_WARPS][32];  // epilogue: per warp, 32 row (or column) offsets
   __shared__ float bias_s[2][ws::EPI_WARPS][32];
@@ -816,13 +843,17 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  const bool bulk = w.a.bulk && (!FUSE || w.b.bulk);  // every copy a bulk copy: COPY_WARP issues them all
   if (threadIdx.x == 0) {
     for (int s = 0; s < ST; ++s) {
       mbar_init(&full[s], ws::LOADERS);
       mbar_init(&bfull[s], 1);
       mbar_init(&empty[s], 1);
     }
-    for (int d = 0; d < D; ++d) mbar_init(&afull[d], ws::LOADERS);
+    for (int d = 0; d < D; ++d) {
+      mbar_init(&afull[d], bulk ? 1 : ws::LOADERS);
+      mbar_init(&afree[d], 1);
+    }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&accf[b], 1);
       mbar_init(&acce[b], 4);
@@ -838,24 +869,24 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
   const int mtiles = (int)w.mtiles;
   auto k_end = [&](int split) { return min((split + 1) * w.kper, w.kblocks); };
 
+  // blocks of this CTA in order: a cursor over (item, K block)
+  struct Cur {
+    ws::Walk w;
+    int kb, kb1;
+  };
+  auto open = [&](Cur& c) {
+    c.kb = c.w.split * w.kper;
+    c.kb1 = k_end(c.w.split);
+  };
+  auto advance = [&](Cur& c) {
+    if (++c.kb >= c.kb1) {
+      c.w.next(gridDim.x, w.ntiles, mtiles, w.splits);
+      open(c);
+    }
+  };
   if (warp < 4) {  // operand loaders
     asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
     const int i = threadIdx.x;
-    // stages of this CTA in order: a cursor over (item, K block)
-    struct Cur {
-      ws::Walk w;
-      int kb, kb1;
-    };
-    auto open = [&](Cur& c) {
-      c.kb = c.w.split * w.kper;
-      c.kb1 = k_end(c.w.split);
-    };
-    auto advance = [&](Cur& c) {
-      if (++c.kb >= c.kb1) {
-        c.w.next(gridDim.x, w.ntiles, mtiles, w.splits);
-        open(c);
-      }
-    };
     // One loop per operand form: what runs is one form's instructions, without the others between
     auto load = [&](auto form_a, auto form_b) {
       constexpr int MA = decltype(form_a)::value;
@@ -873,7 +904,7 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
       int s = 0, d = 0, used = 0;  // used: stages handed to the MMAs, at most ST
       uint32_t sp = 0, dp = 0;
       while (true) {
-        for (; flight < D && ahead.w.it < w.items; ++flight, advance(ahead)) {
+        for (; !bulk && flight < D && ahead.w.it < w.items; ++flight, advance(ahead)) {
           bool cp = ws::issue_op<BM, MA>(stg0 + di * ws::SLOT_FLOATS, &afull[di], w.a, ahead.w.bt, w.K,
                                          (long long)ahead.w.mt * BM, ahead.kb, i);
           if constexpr (FUSE)
@@ -890,10 +921,6 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
           uint8_t* st = smem + s * C::STAGE_BYTES;
           if constexpr (FUSE) {
             conv_b.run(st + A_BYTES, stgb + d * C::BSLOT_FLOATS, w.b, w.K, cur.w.nt, cur.kb, i);
-          } else if (i == 64) {
-            mbar_expect_tx(&bfull[s], C::B_BYTES);
-            bulk_g2s(st + A_BYTES, w.b_img + (((size_t)cur.w.bt * w.ntiles + cur.w.nt) * w.kblocks + cur.kb) * C::B_BYTES,
-                     C::B_BYTES, &bfull[s]);
           }
           conv_a.run(st, stg0 + d * ws::SLOT_FLOATS, w.a, w.K, cur.w.mt, cur.kb, i);
           fence_proxy_async();  // the tensor cores read the stage through the async proxy
@@ -907,7 +934,11 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
           if (i == 0) atomicOr(err, 2);
           break;
         }
-        --flight;
+        if (bulk) {
+          if (i == 0) mbar_arrive(&afree[d]);
+        } else {
+          --flight;
+        }
         if (++d == D) { d = 0; dp ^= 1u; }
         advance(cur);
       }
@@ -915,14 +946,6 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
       for (; flight > 0; --flight) {
         mbar_wait_bounded(&afull[d], dp);
         if (++d == D) { d = 0; dp ^= 1u; }
-      }
-      if (i == 64 && !FUSE) {
-        if (used == ST) sp ^= 1u;  // the last ST stages: s is the oldest of them
-        else s = 0;
-        for (int j = 0; j < used; ++j) {
-          mbar_wait_bounded(&bfull[s], sp);
-          if (++s == ST) { s = 0; sp ^= 1u; }
-        }
       }
     };
     if constexpr (FUSE) {
@@ -940,7 +963,7 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
       }
     }
   } else if (warp >= ws::MMA_WARP) {  // MMA issuer
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == ws::MMA_WARP && lane == 0) {
       long long n = 0;
       int s = 0;
@@ -991,6 +1014,65 @@ __global__ void __launch_bounds__(ws::THREADS, 1) gemm_ws_kernel(WsArgs w, Epi e
                        smem_u32(&drain))
                    : "memory");
       if (!mbar_wait_bounded(&drain, 0)) atomicOr(err, 32);
+    } else if (warp == ws::COPY_WARP && bulk) {
+      // FP32 operands, up to D blocks ahead of the loaders
+      Cur c;
+      c.w.start(blockIdx.x, gridDim.x, w.ntiles, mtiles, w.splits);
+      open(c);
+      int d = 0, sent = 0;  // sent: blocks in flight or landed, at most D
+      uint32_t dp = 0;
+      for (; c.w.it < w.items; advance(c)) {
+        if (sent == D && !ws::wait_bar(&afree[d], dp ^ 1u)) {
+          if (lane == 0) atomicOr(err, 128);
+          break;
+        }
+        __syncwarp();
+        float* const sa = stg0 + d * ws::SLOT_FLOATS;
+        float* const sb = stgb + d * C::BSLOT_FLOATS;
+        if (lane == 0) {
+          uint32_t bytes = ws::bulk_block<BM>(sa, &afull[d], w.a, c.w.bt, w.K, (long long)c.w.mt * BM, c.kb, 0, false);
+          if constexpr (FUSE)
+            bytes += ws::bulk_block<C::BROWS>(sb, &afull[d], w.b, c.w.bt, w.K, (long long)c.w.nt * BN, c.kb, 0, false);
+          mbar_expect_tx(&afull[d], bytes);
+        }
+        __syncwarp();
+        ws::bulk_block<BM>(sa, &afull[d], w.a, c.w.bt, w.K, (long long)c.w.mt * BM, c.kb, lane, true);
+        if constexpr (FUSE)
+          ws::bulk_block<C::BROWS>(sb, &afull[d], w.b, c.w.bt, w.K, (long long)c.w.nt * BN, c.kb, lane, true);
+        if (sent < D) ++sent;
+        if (++d == D) { d = 0; dp ^= 1u; }
+      }
+      // copies in flight land before the CTA's shared memory is released
+      if (sent == D) dp ^= 1u;  // the last `sent` blocks: d is the oldest of them
+      else d = 0;
+      for (int j = 0; j < sent; ++j) {
+        mbar_wait_bounded(&afull[d], dp);
+        if (++d == D) { d = 0; dp ^= 1u; }
+      }
+    } else if (!FUSE && warp == ws::IMAGE_WARP && lane == 0) {
+      // packed B, into each stage as the MMAs leave it
+      Cur c;
+      c.w.start(blockIdx.x, gridDim.x, w.ntiles, mtiles, w.splits);
+      open(c);
+      int s = 0, sent = 0;
+      uint32_t sp = 0;
+      for (; c.w.it < w.items; advance(c)) {
+        if (sent == ST && !ws::wait_bar(&empty[s], sp ^ 1u)) {
+          atomicOr(err, 256);
+          break;
+        }
+        mbar_expect_tx(&bfull[s], C::B_BYTES);
+        bulk_g2s(smem + s * C::STAGE_BYTES + A_BYTES,
+                 w.b_img + (((size_t)c.w.bt * w.ntiles + c.w.nt) * w.kblocks + c.kb) * C::B_BYTES, C::B_BYTES, &bfull[s]);
+        if (sent < ST) ++sent;
+        if (++s == ST) { s = 0; sp ^= 1u; }
+      }
+      if (sent == ST) sp ^= 1u;
+      else s = 0;
+      for (int j = 0; j < sent; ++j) {
+        mbar_wait_bounded(&bfull[s], sp);
+        if (++s == ST) { s = 0; sp ^= 1u; }
+      }
     }
     __syncwarp();
   } else {  // epilogue, warps 4-11: group eg takes this CTA's tiles n = eg, eg + 2, ... (accumulator eg)
@@ -1462,8 +1544,8 @@ int TcGemm::run(const float* a, Addr aa, const float* b, Addr ba, long long M, i
   e.N = N;
   e.ybs = 0;
   tg::WsArgs w{};
-  w.a = tg::ws::Op{a, aa, 0, M, 0, 0, 0, 0};
-  w.b = tg::ws::Op{b, ba, 0, N, 0, 0, 0, 0};
+  w.a = tg::ws::Op{a, aa, 0, M, 0, 0, 0, 0, 0};
+  w.b = tg::ws::Op{b, ba, 0, N, 0, 0, 0, 0, 0};
   w.K = K;
   w.kblocks = kblocks;
   w.ntiles = ntiles;
@@ -1555,7 +1637,7 @@ int TcGemm::run_batched(const float* a, Addr aa, long long a_bs, const float* b,
   const uint8_t* bi = reinterpret_cast<const uint8_t*>(b_img);
   cudaError_t c;
   tg::WsArgs w{};
-  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0, 0};
+  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0, 0, 0};
   w.b_img = bi;
   w.K = K;
   w.kblocks = kblocks;
@@ -1593,7 +1675,7 @@ int TcGemm::run_cplx(const float* a, Addr aa, long long a_bs, const float* src, 
   const uint8_t* bi = reinterpret_cast<const uint8_t*>(b_img);
   cudaError_t c;
   tg::WsArgs w{};
-  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0, 0};
+  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0, 0, 0};
   w.b_img = bi;
   w.K = K;
   w.kblocks = kblocks;
