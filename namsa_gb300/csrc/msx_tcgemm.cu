@@ -461,8 +461,9 @@ struct Walk {
 
 // How the rows r0 .. r0 + R - 1 of an operand (R = 128 for A, BN for B), K block kb
 // (nk = min(64, K - 64 kb) values), reach a staging slot:
-//   ROWRUN   k contiguous: thread i copies row r0 + i to slot[i][0 .. nk) with one bulk
-//            copy (16-byte aligned runs), else with plain loads;
+//   ROWRUN   k contiguous: row r0 + i to slot[i][0 .. nk) in 16-byte asynchronous copies
+//            dealt over all threads where every row is aligned (one bulk copy a row took
+//            twice as long to issue), else thread i copies its row, in bulk if it can;
 //   GROUPRUN rows contiguous in groups of rc with k stride rc (a group's K block is one
 //            run of nk * rc values; rc may be all the operand's rows): thread i < R / rc
 //            copies group i to slot[i * 64 rc ..], element (k, r mod rc) at k rc + r mod rc;
@@ -495,7 +496,7 @@ struct Op {
   long long bs;    // batch stride (floats)
   long long rows;  // M or N
   int mode, rc;    // rc: rows of a group (GROUPRUN, PIECES)
-  int whole;       // TILERUN: every full tile is one 16-byte aligned run
+  int whole;       // TILERUN: every full tile is one 16-byte aligned run; ROWRUN: every row is aligned
   int pair;        // PIECES: two neighbouring k values to a row
   int bulk;        // every block arrives by bulk copies of one warp (issue_bulk)
 };
@@ -511,7 +512,7 @@ __host__ __device__ inline void op_mode(Op& o, int tile_rows, long long k_total)
   if (a.kc == 1 && a.t1 == 1) {
     o.mode = ROWRUN;
     if (a.rc == 1 && k_total <= BK && a.s1 == k_total) o.mode = TILERUN;
-    o.whole = aligned;
+    o.whole = aligned && (o.mode == TILERUN || ((a.rc == 1 || a.s2 % 4 == 0) && a.s1 % 4 == 0));
     o.bulk = o.mode == TILERUN && aligned && o.rows * k_total % 4 == 0;
     return;
   }
@@ -588,6 +589,14 @@ __device__ __forceinline__ bool issue_op(float* stg, uint64_t* bar, const Op& o,
       for (int j = i; j < n; j += LOADERS) stg[j] = __ldg(src + j);
     }
     return false;
+  }
+  if (mode == ROWRUN && o.whole && (nk & 3) == 0) {
+    const int nrow = (int)(o.rows - r0 < R ? o.rows - r0 : R), pr = nk >> 2;
+    for (int j = i; j < nrow * pr; j += LOADERS) {
+      const int row = nk == BK ? j / (BK / 4) : j / pr, q = j - row * pr;
+      cp16(stg + row * BK + q * 4, P + row_off(r0 + row) + kb0 + q * 4);
+    }
+    return true;
   }
   if (mode == ROWRUN) {
     const long long r = r0 + i;
