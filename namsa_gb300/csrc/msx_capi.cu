@@ -966,7 +966,6 @@ int msx_multislice_detect(msx_plan* p, const float* trans_dev, int num_slices, c
   const size_t need = (size_t)p->group * (p->nx / p->col_ops->col_c) * num_detectors;
   if (need > p->partial_words) {
     if (p->partial) cudaFree(p->partial);
-  if (p->inv_n) cudaFree(p->inv_n);
     p->partial = nullptr;
     p->partial_words = 0;
     if (cudaMalloc(&p->partial, need * sizeof(float)) != cudaSuccess)
