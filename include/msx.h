@@ -138,7 +138,11 @@ MSX_API int msx_build_probe(int ny, int nx, float kmax, double lambda, float k_s
  * wavefunctions kept resident per group (0 = about 1 GiB of waves, 4 to 512);
  * the workspace for it is allocated here.  The plan starts with the schedules
  * the autotuner picks on GB300 for the grid (msx_plan_autotune refines both
- * for given inputs).  Replaces the per-batch cuFFT plans and allocations of
+ * for given inputs), and chooses per call how the slices run: as two passes a
+ * slice; for groups of waves that stay in L2, all slices in one persistent
+ * kernel; for a few positions on grids up to 256 x 256, each wave in the shared
+ * memory of a thread-block cluster.  All three give the same patterns within
+ * float32 rounding.  Replaces the per-batch cuFFT plans and allocations of
  * MSAGPU.multislice (namsa/msa.py:843-881) and plan_simulation's batching
  * (namsa/msa.py:445-461).
  */
@@ -147,7 +151,8 @@ MSX_API int msx_plan_destroy(msx_plan* plan);
 
 /* Selects the FFT schedule of the row (x) and column (y) passes (index into
  * msx_num_schedules of nx / ny) and the group size; group 0 keeps the
- * current one.  The workspace grows when needed. */
+ * current one.  The workspace grows when needed.  Slices then run as two
+ * passes with these schedules. */
 MSX_API int msx_plan_set_schedule(msx_plan* plan, int row_schedule, int col_schedule, int group);
 
 /* Reports the current row/column schedule indices and group size. */
@@ -463,7 +468,9 @@ MSX_API int msx_corrector_residual(const float* psi_dev, const float* target_dev
  * plan's grid on the given inputs -- `iters` slices of row + column passes
  * per candidate, CUDA events on `stream` -- and keeps the fastest.  Group
  * sizes range over resident sets of 8 MiB to 1 GiB of waves (capped by
- * num_probes and max_workspace_bytes, 0 = 1 GiB).  Writes the best time per
+ * num_probes and max_workspace_bytes, 0 = 1 GiB).  Where the one-kernel form
+ * of all slices exists for the grid it is timed against them, and the plan
+ * keeps whichever is faster.  Writes the best time per
  * wave and slice (ns) to *best_ns_per_wave_slice when non-NULL.  Synchronises
  * `stream`.  No counterpart in the reference (its batch size comes from a
  * free-memory heuristic, namsa/msa.py:445-461).

@@ -122,7 +122,8 @@ struct msx_plan {
   int row_ctas = 0, col_ctas = 0, sms = 0;
   // all slices of a group in one kernel (msx_stream.cuh); off while schedules are set by hand
   const StreamOps* stream = nullptr;
-  bool use_stream = false;       // may take `stream` and `resident`
+  bool use_stream = false;       // may take `stream`
+  bool use_resident = false;     // may take `resident`
   // a wave in the shared memory of a cluster (msx_resident.cuh), small grids
   const ResidentOps* resident = nullptr;
   float2* rtw_row = nullptr;     // in `tables`
@@ -240,6 +241,7 @@ int create_tables(msx_plan* p) {
     MSX_CUDA(p->resident->configure(), "configuring the cluster-resident kernel");
   }
   p->use_stream = true;
+  p->use_resident = true;
   return MSX_OK;
 }
 
@@ -500,7 +502,7 @@ int stream_group(const msx_plan* p, const MsArgs& a) {
 // to two rounds of clusters of four.
 constexpr int kResidentSizes[3] = {16, 8, 4};
 int resident_cluster(msx_plan* p, const MsArgs& a) {
-  if (!p->use_stream || !p->resident || !p->use_tma || !p->map_ok || a.det || a.num_slices < 2 || a.num_probes < 1 ||
+  if (!p->use_resident || !p->resident || !p->use_tma || !p->map_ok || a.det || a.num_slices < 2 || a.num_probes < 1 ||
       a.num_probes > a.group || !aligned(a.trans, 16))
     return 0;
   int lo = 0, hi = 0;
@@ -827,7 +829,7 @@ int msx_plan_set_schedule(msx_plan* p, int row_schedule, int col_schedule, int g
     rc = upload_twiddles(cops[col_schedule], &p->tw_col);
     if (rc != MSX_OK) return rc;
   }
-  p->use_stream = false;  // schedules set by hand are the passes that run
+  p->use_stream = p->use_resident = false;  // schedules set by hand are the passes that run
   p->row_sched = row_schedule;
   p->col_sched = col_schedule;
   p->row_ops = &rops[row_schedule];
@@ -1118,7 +1120,7 @@ int msx_multislice_host(msx_plan* p, const float* trans_host, int num_slices, co
   hk.d_cbed = p->io_cbed; hk.normalization = normalization; hk.lambda = lambda; hk.slice_t = slice_t;
   hk.kmax = kmax; hk.k_band = k_band; hk.num_slices = num_slices; hk.num_probes = num_probes; hk.crop_y = crop_y;
   hk.crop_x = crop_x; hk.group = p->group; hk.row_sched = p->row_sched; hk.col_sched = p->col_sched;
-  hk.tma = (p->use_tma ? 1 : 0) + (p->use_stream ? 2 : 0);
+  hk.tma = (p->use_tma ? 1 : 0) + (p->use_stream ? 2 : 0) + (p->use_resident ? 4 : 0);
   std::vector<unsigned char> key(sizeof(hk));
   std::memcpy(key.data(), &hk, sizeof(hk));
   // everything here follows the caller's earlier work and this plan's earlier calls
@@ -1363,9 +1365,8 @@ int msx_plan_autotune(msx_plan* p, const float* trans_dev, int num_slices, const
     std::memset(&a, 0, sizeof(a));
     a.trans = trans_dev; a.num_slices = num_slices; a.num_probes = num_probes; a.kmax = kmax; a.lambda = lambda;
     a.slice_t = slice_t; a.k_band = k_band; a.group = p->group;
-    p->use_stream = p->stream != nullptr;
+    p->use_stream = p->use_resident = true;  // per call, unless the timing below is against the former
     const int g = stream_group(p, a), s = num_slices < iters ? num_slices : iters;
-    p->use_stream = false;
     if (g > 0 && workspace_holds(p, g)) {
       ColArgs c{};
       c.psi = p->psi; c.psik = reinterpret_cast<const float2*>(psi_k_dev); c.pos_yx = positions_dev; c.tw = p->tw_col;
@@ -1382,10 +1383,8 @@ int msx_plan_autotune(msx_plan* p, const float* trans_dev, int num_slices, const
         float ms = 0;
         MSX_CUDA(cudaEventElapsedTime(&ms, e0, e1), "cudaEventElapsedTime");
         const float ns = ms * 1e6f / ((float)s * (float)g);
-        if (ns < best) {
-          best = ns;
-          p->use_stream = true;
-        }
+        if (ns < best) best = ns;
+        else p->use_stream = false;
         return MSX_OK;
       }();
     }
@@ -1416,10 +1415,16 @@ struct msx_batch {
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
   cudaGraphExec_t gexec = nullptr;
   std::vector<unsigned char> gkey;
-  std::vector<std::pair<long long, std::array<int, 4>>> sched;  // (ny<<32|nx) -> row, col, group, all-slices kernel
+  std::vector<std::pair<long long, std::array<int, 4>>> sched;  // (ny<<32|nx) -> row, col, group, forms
 };
 
 namespace {
+
+// Forms besides the two passes that a plan with given schedules may take: 1 the all-slices kernel, 2 clusters.
+void allow_forms(msx_plan* p, int forms) {
+  p->use_stream = (forms & 1) != 0;
+  p->use_resident = (forms & 2) != 0;
+}
 
 msx_plan* batch_plan(msx_batch* b, int branch, int ny, int nx, int* rc) {
   const long long key = ((long long)ny << 32) | (unsigned)nx;
@@ -1430,10 +1435,11 @@ msx_plan* batch_plan(msx_batch* b, int branch, int ny, int nx, int* rc) {
   int group = (int)(((size_t)1 << 30) / (sizeof(float2) * (size_t)ny * nx));
   if (group < 2) group = 2;
   int r = 0, c = 0;
-  bool tuned = false, stream = false;  // schedules set for this grid (else the plan's defaults)
+  bool tuned = false;  // schedules set for this grid (else the plan's defaults)
+  int forms = 0;
   for (auto& kv : b->sched)
     if (kv.first == key) {
-      r = kv.second[0]; c = kv.second[1]; tuned = true; stream = kv.second[3] != 0;
+      r = kv.second[0]; c = kv.second[1]; tuned = true; forms = kv.second[3];
       if (kv.second[2] > 0) group = kv.second[2];
     }
   msx_plan* p = nullptr;
@@ -1442,13 +1448,13 @@ msx_plan* batch_plan(msx_batch* b, int branch, int ny, int nx, int* rc) {
   if (tuned) {
     *rc = msx_plan_set_schedule(p, r, c, group);
     if (*rc != MSX_OK) { msx_plan_destroy(p); return nullptr; }
-    p->use_stream = stream && p->stream;
+    allow_forms(p, forms);
   }
   b->plans[branch].push_back({key, p});
   return p;
 }
 
-int batch_set_schedule(msx_batch* b, int ny, int nx, int row_schedule, int col_schedule, int group, bool stream) {
+int batch_set_schedule(msx_batch* b, int ny, int nx, int row_schedule, int col_schedule, int group, int forms) {
   if (!b) return fail(MSX_ERR_INVALID, "null batch");
   if (!msx_supported_size(ny) || !msx_supported_size(nx)) return fail(MSX_ERR_UNSUPPORTED, "grid %d x %d", ny, nx);
   if (row_schedule < 0 || row_schedule >= msx_num_schedules(nx) || col_schedule < 0 ||
@@ -1457,14 +1463,14 @@ int batch_set_schedule(msx_batch* b, int ny, int nx, int row_schedule, int col_s
   const long long key = ((long long)ny << 32) | (unsigned)nx;
   bool found = false;
   for (auto& kv : b->sched)
-    if (kv.first == key) { kv.second = {row_schedule, col_schedule, group, stream}; found = true; }
-  if (!found) b->sched.push_back({key, {row_schedule, col_schedule, group, stream}});
+    if (kv.first == key) { kv.second = {row_schedule, col_schedule, group, forms}; found = true; }
+  if (!found) b->sched.push_back({key, {row_schedule, col_schedule, group, forms}});
   for (auto& br : b->plans)
     for (auto& kv : br)
       if (kv.first == key) {
         const int rc = msx_plan_set_schedule(kv.second, row_schedule, col_schedule, group);
         if (rc != MSX_OK) return rc;
-        kv.second->use_stream = stream && kv.second->stream;
+        allow_forms(kv.second, forms);
       }
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
   b->gexec = nullptr;
@@ -1517,7 +1523,7 @@ int msx_batch_destroy(msx_batch* b) {
 }
 
 int msx_batch_set_schedule(msx_batch* b, int ny, int nx, int row_schedule, int col_schedule, int group) {
-  return batch_set_schedule(b, ny, nx, row_schedule, col_schedule, group, false);
+  return batch_set_schedule(b, ny, nx, row_schedule, col_schedule, group, 0);
 }
 
 int msx_batch_autotune(msx_batch* b, const msx_job* jobs, int njobs, int iters, void* stream) {
@@ -1546,9 +1552,9 @@ int msx_batch_autotune(msx_batch* b, const msx_job* jobs, int njobs, int iters, 
                            stream);
     int row = 0, col = 0, group = 0;
     if (rc == MSX_OK) rc = msx_plan_get_schedule(p, &row, &col, &group);
-    const bool stream = rc == MSX_OK && p->use_stream;
+    const int forms = rc == MSX_OK ? (p->use_stream ? 1 : 0) + (p->use_resident ? 2 : 0) : 0;
     msx_plan_destroy(p);
-    if (rc == MSX_OK) rc = batch_set_schedule(b, j.ny, j.nx, row, col, group, stream);
+    if (rc == MSX_OK) rc = batch_set_schedule(b, j.ny, j.nx, row, col, group, forms);
     if (rc != MSX_OK) return rc;
   }
   return MSX_OK;

@@ -19,7 +19,25 @@
 // shared memory, B comes from a small packed image (pack_kernel, or
 // pack_cplx_kernel for the real embedding of a complex product) or, for the
 // long-K weight gradients (N <= 32), is staged and rounded like A while K is
-// split over the CTAs.  The per-tile kernel (gemm_kernel, both operands packed)
+// split over the CTAs.
+//
+// What bounds it: the products here are narrow (32 to 256 columns), so each is a
+// stream over one or two activations and the tensor cores are idle most of the
+// time; what is left above the memory time is the instruction chain of a block
+// (one warp per scheduler and role).  Hence the roles: four warps that only round,
+// one that issues the bulk copies, one that moves the packed B, one that issues
+// the MMAs, eight that finish tiles; registers moved from the former to the
+// latter (128 at launch -> 120 / 56 / 168), for a spill costs a trip to L2 once
+// shared memory has taken the L1; one loop per operand and output form, because
+// a quarter of the stalls were instruction fetch when the forms shared one; and
+// no division between one block and the next.  At 32 x 256^2 pixels, 32 channels
+// (us, before these -> now, memory time at the measured copy rate):
+//   pointwise + add + gelu    384 -> 199 (158)   weight gradient   456 -> 160 (79)
+//   pointwise, plain          241 ->  95  (79)   x transform       109 ->  69 (49)
+//   inverse x                 101 ->  72  (49)   inverse x, added  194 -> 130 (89)
+//   y transform                75 ->  28  (12)   inverse y          45 ->  31 (12)
+//   mixing                     70 ->  25   (5)
+// The per-tile kernel (gemm_kernel, both operands packed)
 // remains for split-K products with N > 32.
 #include "msx.h"
 #include "msx_internal.h"

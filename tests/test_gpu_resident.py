@@ -70,3 +70,17 @@ def test_streams_host_buffers_and_capture():
     assert torch.equal(out, wy)
     plan.check()
     plan.close()
+
+
+def test_autotuned_plan_keeps_the_clusters():
+    """Tuning chooses among the passes; calls that the clusters take still go there, same bits.
+    Schedules set by hand are the passes that run."""
+    torch.cuda.set_device(0)
+    x = case(128, 128, 5, 4, 7)
+    plan = engine.Plan(128, 128)
+    want = plan.multislice(*x).clone()
+    plan.autotune(*x, iters=2)
+    assert torch.equal(plan.multislice(*x), want)
+    plan.set_schedule(*plan.schedule[:2])
+    assert rel(plan.multislice(*x), want) < 1e-6
+    plan.close()
