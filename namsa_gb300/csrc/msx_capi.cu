@@ -120,6 +120,14 @@ struct msx_plan {
   CUtensorMap map{};             // workspace as (psi_waves*ny) x nx 8-byte elements, box col_c x col_boxr
   bool map_ok = false;
   int row_ctas = 0, col_ctas = 0, sms = 0;
+  // the passes of calls of a few lines (few_lines); off while schedules are set by hand
+  struct FewPass {
+    const SchedOps* ops = nullptr;
+    float2* tw = nullptr;        // in `tables`
+    int ctas = 0;
+  } few_row, few_col;
+  CUtensorMap fmap{};            // the workspace with few_col's tile as box
+  bool use_few = false;
   // all slices of a group in one kernel (msx_stream.cuh); off while schedules are set by hand
   const StreamOps* stream = nullptr;
   bool use_stream = false;       // may take `stream`
@@ -212,7 +220,9 @@ int create_tables(msx_plan* p) {
     std::memcpy(h.data() + (off - twiddles), t.data(), sizeof(float2) * words);
     return off;
   };
-  size_t srow = 0, scol = 0, rrow = 0, rcol = 0;
+  size_t srow = 0, scol = 0, rrow = 0, rcol = 0, frow = 0, fcol = 0;
+  if (p->few_row.ops) frow = table(p->few_row.ops->tw_words, p->few_row.ops->host_twiddles);
+  if (p->few_col.ops) fcol = table(p->few_col.ops->tw_words, p->few_col.ops->host_twiddles);
   if (p->stream) {
     srow = table(p->stream->twr_words, p->stream->tw_row);
     scol = table(p->stream->twc_words, p->stream->tw_col);
@@ -240,6 +250,9 @@ int create_tables(msx_plan* p) {
     p->rtw_col = reinterpret_cast<float2*>(base + rcol);
     MSX_CUDA(p->resident->configure(), "configuring the cluster-resident kernel");
   }
+  p->few_row.tw = reinterpret_cast<float2*>(base + frow);
+  p->few_col.tw = reinterpret_cast<float2*>(base + fcol);
+  p->use_few = true;
   p->use_stream = true;
   p->use_resident = true;
   return MSX_OK;
@@ -296,12 +309,20 @@ int prepare_tma(msx_plan* p) {
   };
   CUresult r = encode(&p->map, p->col_ops->col_c, p->col_ops->col_boxr);
   if (r == CUDA_SUCCESS && p->stream) r = encode(&p->smap, p->stream->col_c, p->stream->col_boxr);
+  if (r == CUDA_SUCCESS && p->few_col.ops) r = encode(&p->fmap, p->few_col.ops->col_c, p->few_col.ops->col_boxr);
   if (r != CUDA_SUCCESS) return fail(MSX_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
   int sms = 0, rr = 0, cr = 0, dummy = 0;
   MSX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device), "SM count");
   MSX_CUDA(p->row_ops->occupancy(&rr, &dummy), "occupancy");
   MSX_CUDA(p->col_ops->occupancy(&dummy, &cr), "occupancy");
   if (rr < 1 || cr < 1) return fail(MSX_ERR_CUDA, "persistent passes do not fit on an SM");
+  for (msx_plan::FewPass* f : {&p->few_row, &p->few_col})
+    if (f->ops) {
+      int fr = 0, fc = 0;
+      MSX_CUDA(f->ops->occupancy(&fr, &fc), "occupancy");
+      f->ctas = sms * (f == &p->few_row ? fr : fc);
+      if (f->ctas < 1) return fail(MSX_ERR_CUDA, "persistent passes do not fit on an SM");
+    }
   p->sms = sms;
   p->row_ctas = sms * rr;
   p->col_ctas = sms * cr;
@@ -360,6 +381,19 @@ int default_col_schedule(int ny) {
   return ny == 768 ? schedule_index(768, "t16_r48x16") : ny == 384 ? schedule_index(384, "t8_r48x8") : 0;
 }
 
+// Schedules of calls whose passes do not fill the GPU, where the shortest line counts
+// and not the most lines: the radices above win by fewer operations and exchanges
+// per line but are a longer chain.  -1: the default serves them too.
+int few_row_schedule(int nx) {
+  switch (nx) {
+    case 384: return schedule_index(384, "t16_r8x8x6");
+    case 512: return schedule_index(512, "t32_r16x2x16_pair");
+    case 768: return schedule_index(768, "t32_r8x8x12");
+    default: return -1;
+  }
+}
+int few_col_schedule(int ny) { return ny == 384 || ny == 768 ? few_row_schedule(ny) : -1; }
+
 struct MsArgs {
   const float* trans; int num_slices; const float* psik; const double* norm; const float* pos; int num_probes;
   float kmax; double lambda, slice_t; float k_band; float* cbed; int crop_y, crop_x;
@@ -394,18 +428,47 @@ void band_columns(int nx, float kmax, float k_band, int C, int* x_lo, int* x_hi)
   *x_hi = (hi / C + 1) * C < nx ? (hi / C + 1) * C : nx;
 }
 
+// Whether the row (column) pass over gn waves runs with the schedule for few lines:
+// while its tiles are at most one to an SM; at 768 also for one tile a row, since the
+// default's CTAs are alone on their SM.  Event timings on GB300, us per slice of both
+// passes, default / few:
+//   rows     64 x 384   P 1 9.9/9.0   32 12.2/11.5  64 14.4/16.0     256 x 384  P 4 12.6/14.3
+//           128 x 384   P 4 11.7/10.9 16 12.6/11.9  24 14.7/16.5
+//            64 x 768   P 1 11.2/9.6  16 13.2/11.0  24 13.9/15.0
+//           384 x 768   P 1 25.3/21.0  8 27.3/23.5  12 31.8/36.5
+//            64 x 512   P 1 8.8/8.2   16 9.9/9.2    24 10.6/10.7
+//   columns 384 x 128   P 1 14.4/13.0 24 15.9/14.7  32 17.4/17.8
+//           384 x 384   P 1 19.5/18.2  8 20.2/18.9  12 21.6/21.8
+//           768 x 64    P 1 16.1/14.1 24 18.5/16.6  32 19.5/20.9
+//           768 x 256   P 1 16.5/14.3  4 16.7/14.5   8 17.4/19.0
+bool few_rows(const msx_plan* p, int gn) {
+  if (!p->use_few || !p->few_row.ops) return false;
+  const int tiles = (gn + p->few_row.ops->row_lines - 1) / p->few_row.ops->row_lines;
+  return tiles * p->ny <= p->sms || (p->nx == 768 && tiles == 1);
+}
+bool few_cols(const msx_plan* p, int gn, float kmax, float k_band, int* x_lo, int* x_hi) {
+  if (p->use_few && p->few_col.ops) {
+    band_columns(p->nx, kmax, k_band, p->few_col.ops->col_c, x_lo, x_hi);
+    if ((*x_hi - *x_lo) / p->few_col.ops->col_c * gn <= p->sms) return true;
+  }
+  band_columns(p->nx, kmax, k_band, p->col_ops->col_c, x_lo, x_hi);
+  return false;
+}
+
 // x_lo, x_hi: the column range of the TMA passes (0, 0 = all columns); the
-// plain passes always cover every column.
+// plain passes always cover every column.  fr, fc: the row, column pass with the
+// schedule for few lines.
 int slice_passes(msx_plan* p, const float2* trans_s, int gn, const ColArgs& c, bool with_col, cudaStream_t st,
-                 int x_lo, int x_hi, bool tma) {
+                 int x_lo, int x_hi, bool tma, bool fr = false, bool fc = false) {
   if (tma) {
     TmaPassArgs ta{};
-    ta.psi = p->psi; ta.trans = trans_s; ta.tw = p->tw_row; ta.pyx = p->pyx; ta.band = p->band; ta.err = p->err;
-    ta.G = gn; ta.Ny = p->ny; ta.Nx = p->nx; ta.x_lo = x_lo; ta.x_hi = x_hi;
-    MSX_CUDA(p->row_ops->row_tma(ta, p->row_ctas, st), "row pass");
+    ta.psi = p->psi; ta.trans = trans_s; ta.tw = fr ? p->few_row.tw : p->tw_row; ta.pyx = p->pyx; ta.band = p->band;
+    ta.err = p->err; ta.G = gn; ta.Ny = p->ny; ta.Nx = p->nx; ta.x_lo = x_lo; ta.x_hi = x_hi;
+    MSX_CUDA((fr ? p->few_row.ops : p->row_ops)->row_tma(ta, fr ? p->few_row.ctas : p->row_ctas, st), "row pass");
     if (with_col) {
-      ta.tw = p->tw_col;
-      MSX_CUDA(p->col_ops->col_tma(p->map, ta, p->col_ctas, st), "column pass");
+      ta.tw = fc ? p->few_col.tw : p->tw_col;
+      MSX_CUDA(fc ? p->few_col.ops->col_tma(p->fmap, ta, p->few_col.ctas, st)
+                  : p->col_ops->col_tma(p->map, ta, p->col_ctas, st), "column pass");
     }
   } else {
     MSX_CUDA(p->row_ops->row(p->psi, trans_s, p->tw_row, gn, p->ny, st), "row pass");
@@ -468,9 +531,9 @@ struct StreamRange {
 };
 constexpr StreamRange kStreamRange[4][4] = {  // [ny][nx], lines of 256, 384, 512, 768
     {{12, 180}, {24, 130}, {12, 60}, {1, 130}},
-    {{24, 36}, {16, 400}, {12, 130}, {1, 300}},
+    {{24, 36}, {16, 400}, {12, 130}, {12, 300}},
     {{8, 60}, {1, 500}, {1, 360}, {1, 500}},
-    {{1, 36}, {1, 300}, {1, 380}, {1, 310}}};
+    {{8, 36}, {1, 300}, {1, 380}, {1, 310}}};
 int stream_group(const msx_plan* p, const MsArgs& a) {
   if (!p->use_stream || !p->stream || !p->use_tma || !p->map_ok || a.num_slices < 2 || a.num_probes < 1 ||
       !aligned(a.trans, 16))
@@ -519,7 +582,9 @@ int resident_cluster(msx_plan* p, const MsArgs& a) {
   if (area > 128 * 128 && a.num_probes <= p->rclusters[0]) return kResidentSizes[0];
   if (area >= 256 * 256) return 0;
   if (a.num_probes <= p->rclusters[1]) return kResidentSizes[1];
-  if (a.num_probes <= (area <= 128 * 128 ? 2 : 1) * p->rclusters[2]) return kResidentSizes[2];
+  if (p->nx > p->ny && area > 128 * 128 && a.num_probes < 24) return 0;  // 128 x 256: P 16 9.0 / 9.7, 24 9.8 / 9.7
+  const int rounds = area <= 128 * 128 && p->nx <= 128 ? 2 : 1;  // 64 x 256: P 64 10.9 / 11.1 in two
+  if (a.num_probes <= rounds * p->rclusters[2]) return kResidentSizes[2];
   return 0;
 }
 
@@ -574,8 +639,6 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
   const size_t wave = (size_t)ny * nx;
   const int y0 = ny / 2 - a.crop_y / 2, x0 = nx / 2 - a.crop_x / 2;
   const float2* trans = reinterpret_cast<const float2*>(a.trans);
-  int bx_lo = 0, bx_hi = 0;
-  band_columns(nx, a.kmax, a.k_band, p->col_ops->col_c, &bx_lo, &bx_hi);
   // group done: hand its CBED block to the copy stream (host-buffer calls)
   auto hand_off = [&](int gi, int g0, int gn) -> int {
     if (!hp) return MSX_OK;
@@ -631,6 +694,8 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
       if (rc != MSX_OK) return rc;
       continue;
     }
+    int bx_lo = 0, bx_hi = 0;
+    const bool fr = few_rows(p, gn), fc = few_cols(p, gn, a.kmax, a.k_band, &bx_lo, &bx_hi);
     for (int s = 0; s < a.num_slices; ++s) {
       if (hp && gi == 0 && s % hp->chunk == 0)
         MSX_CUDA(cudaStreamWaitEvent(st, (*hp->chunk_ev)[s / hp->chunk], 0), "cudaStreamWaitEvent");
@@ -642,7 +707,7 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
       } else {
         // the first slice covers every column (the probe may reach beyond the band)
         rc = slice_passes(p, trans + (size_t)s * wave, gn, c, s + 1 < a.num_slices, st, s > 0 ? bx_lo : 0,
-                          s > 0 ? bx_hi : 0, tma);
+                          s > 0 ? bx_hi : 0, tma, fr, fc);
       }
       if (rc != MSX_OK) return rc;
       if (s + 1 == a.num_slices) {
@@ -773,8 +838,22 @@ int msx_plan_create(int ny, int nx, int group, msx_plan** out) {
   p->device = device;
   p->stream = stream_ops(ny, nx);
   p->resident = resident_ops(ny, nx);
-  int rc = msx_plan_set_schedule(p, default_row_schedule(nx), default_col_schedule(ny),
-                                 group > 0 ? group : auto_group(ny, nx));
+  int rc = MSX_OK;
+  const SchedOps *rops, *cops;
+  schedule_table(nx, &rops);
+  schedule_table(ny, &cops);
+  const int fr = few_row_schedule(nx), fc = few_col_schedule(ny);
+  if (fr >= 0) {
+    p->few_row.ops = &rops[fr];
+    rc = ensure_configured(device, nx, fr, rops[fr]);
+  }
+  if (rc == MSX_OK && fc >= 0) {
+    p->few_col.ops = &cops[fc];
+    rc = ensure_configured(device, ny, fc, cops[fc]);
+  }
+  if (rc == MSX_OK)
+    rc = msx_plan_set_schedule(p, default_row_schedule(nx), default_col_schedule(ny),
+                               group > 0 ? group : auto_group(ny, nx));
   if (rc == MSX_OK) rc = create_tables(p);
   if (rc == MSX_OK) {
     cudaError_t e = cudaStreamCreateWithFlags(&p->work, cudaStreamNonBlocking);
@@ -829,7 +908,7 @@ int msx_plan_set_schedule(msx_plan* p, int row_schedule, int col_schedule, int g
     rc = upload_twiddles(cops[col_schedule], &p->tw_col);
     if (rc != MSX_OK) return rc;
   }
-  p->use_stream = p->use_resident = false;  // schedules set by hand are the passes that run
+  p->use_stream = p->use_resident = p->use_few = false;  // schedules set by hand are the passes that run
   p->row_sched = row_schedule;
   p->col_sched = col_schedule;
   p->row_ops = &rops[row_schedule];
@@ -1120,7 +1199,7 @@ int msx_multislice_host(msx_plan* p, const float* trans_host, int num_slices, co
   hk.d_cbed = p->io_cbed; hk.normalization = normalization; hk.lambda = lambda; hk.slice_t = slice_t;
   hk.kmax = kmax; hk.k_band = k_band; hk.num_slices = num_slices; hk.num_probes = num_probes; hk.crop_y = crop_y;
   hk.crop_x = crop_x; hk.group = p->group; hk.row_sched = p->row_sched; hk.col_sched = p->col_sched;
-  hk.tma = (p->use_tma ? 1 : 0) + (p->use_stream ? 2 : 0) + (p->use_resident ? 4 : 0);
+  hk.tma = (p->use_tma ? 1 : 0) + (p->use_stream ? 2 : 0) + (p->use_resident ? 4 : 0) + (p->use_few ? 8 : 0);
   std::vector<unsigned char> key(sizeof(hk));
   std::memcpy(key.data(), &hk, sizeof(hk));
   // everything here follows the caller's earlier work and this plan's earlier calls

@@ -16,6 +16,7 @@ struct SchedOps {
   int tw_words;
   int col_c;                  // columns per column-pass tile
   int col_boxr;               // rows per tensor-map box of the column tile
+  int row_lines;              // waves per row-pass tile
   void (*host_twiddles)(float2*);
   cudaError_t (*configure)();
   cudaError_t (*row)(float2* psi, const float2* trans, const float2* tw, int G, int Ny, cudaStream_t st);
@@ -98,7 +99,7 @@ template <class S> struct SchedImpl {
     return cudaGetLastError();
   }
   static SchedOps ops(const char* name) {
-    return SchedOps{S::N, name, S::TW, S::C, ColTma<S>::BOXR, &host_twiddles, &configure, &row, &col,
+    return SchedOps{S::N, name, S::TW, S::C, ColTma<S>::BOXR, S::ROW_LINES, &host_twiddles, &configure, &row, &col,
                     &row_tma, &col_tma, &occupancy, &row_mode};
   }
 };

@@ -123,3 +123,18 @@ def test_slices_at_an_odd_address_run_through_the_plain_passes():
     plan.check()
     plan.close()
     assert rel(got, want) < 1e-6
+
+
+@pytest.mark.parametrize('ny,nx,P', [(64, 384, 1), (64, 384, 33), (128, 384, 17), (256, 384, 3), (64, 512, 32), (64, 768, 17),
+                                     (128, 768, 9), (384, 768, 8), (384, 64, 5), (384, 128, 30), (768, 64, 25),
+                                     (768, 128, 13), (768, 256, 7), (384, 384, 9)])
+def test_schedules_of_few_lines(ny, nx, P):
+    """Either side of the lines between the schedules of few and of many lines, and groups that
+    fall on different sides of one."""
+    torch.cuda.set_device(0)
+    x = case(ny, nx, 4, P, ny + nx + P)
+    a, b = both(ny, nx, x, lambda plan, y: plan.multislice(*y))
+    assert rel(a, b) < 1e-6
+    plan = engine.Plan(ny, nx, 4)
+    assert rel(plan.multislice(*x), b) < 1e-6
+    plan.close()
