@@ -40,19 +40,57 @@ __device__ __forceinline__ float gelu_d(float z) {
   return 0.5f * (1.f + th) + 0.5f * z * (1.f - th * th) * k * (1.f + 3.f * 0.044715f * z * z);
 }
 
-// V = 4: four values per thread in 16-byte accesses (n / 4 threads; aligned arrays).
-// Memory-bound: 805 MB at 32 x 256^2 x 32 in 115 us (7.0 TB/s), 224 us one value a thread.
-template <int V>
 __global__ void gelu_bwd_kernel(const float* da, const float* z, long long n, float* dz) {  // dz may be da
-  const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * V;
-  if (i >= n) return;
-  if constexpr (V == 4) {
-    const float4 d = *reinterpret_cast<const float4*>(da + i), v = *reinterpret_cast<const float4*>(z + i);
-    *reinterpret_cast<float4*>(dz + i) =
-        make_float4(d.x * gelu_d(v.x), d.y * gelu_d(v.y), d.z * gelu_d(v.z), d.w * gelu_d(v.w));
-  } else {
-    dz[i] = da[i] * gelu_d(z[i]);
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) dz[i] = da[i] * gelu_d(z[i]);
+}
+
+// The same with the column sums of dz (rows x n, n a power of two from 4 on) on the
+// way, part[chunk][c] over the chunk's rows: thread t of 256 takes the four columns
+// 4 (t mod n / 4) of rows t / (n / 4), + 1024 / n, ...; the partial sums of a column are
+// then added in a fixed tree (in a row they had up to twice the error of the separate
+// kernel below).  Memory-bound: 805 MB at 32 x 256^2 x 32 in 127 us (6.3 TB/s), against
+// 224 us one value a thread and 75 us for reading dz again.
+__global__ void __launch_bounds__(256) gelu_bwd_sum_kernel(const float* da, const float* z, long long rows, int n,
+                                                           long long chunk, float* dz, float* __restrict__ part) {
+  __shared__ float4 red[256];
+  const int t = threadIdx.x, q = n >> 2;
+  const long long r0 = (long long)blockIdx.x * chunk, r1 = r0 + chunk < rows ? r0 + chunk : rows;
+  const float4* a4 = reinterpret_cast<const float4*>(da);
+  const float4* z4 = reinterpret_cast<const float4*>(z);
+  float4* d4 = reinterpret_cast<float4*>(dz);
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  const long long end = r1 * q;
+  long long i = r0 * q + t;  // row r0 + t / q, columns 4 (t mod q): 256 values on is `step` rows on
+  for (; i + 3 * 256 < end; i += 4 * 256) {
+    float4 d[4], v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      d[u] = a4[i + u * 256];
+      v[u] = z4[i + u * 256];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      d[u] = make_float4(d[u].x * gelu_d(v[u].x), d[u].y * gelu_d(v[u].y), d[u].z * gelu_d(v[u].z),
+                         d[u].w * gelu_d(v[u].w));
+      d4[i + u * 256] = d[u];
+      s = make_float4(s.x + d[u].x, s.y + d[u].y, s.z + d[u].z, s.w + d[u].w);
+    }
   }
+  for (; i < end; i += 256) {
+    const float4 e = a4[i], v = z4[i];
+    const float4 d = make_float4(e.x * gelu_d(v.x), e.y * gelu_d(v.y), e.z * gelu_d(v.z), e.w * gelu_d(v.w));
+    d4[i] = d;
+    s = make_float4(s.x + d.x, s.y + d.y, s.z + d.z, s.w + d.w);
+  }
+  red[t] = s;
+  __syncthreads();
+  for (int h = 128; h >= q; h >>= 1) {  // t and t + h hold the same columns: q divides h
+    if (t < h) red[t] = make_float4(red[t].x + red[t + h].x, red[t].y + red[t + h].y, red[t].z + red[t + h].z,
+                                    red[t].w + red[t + h].w);
+    __syncthreads();
+  }
+  if (t < n) part[(size_t)blockIdx.x * n + t] = reinterpret_cast<const float*>(red)[t];
 }
 
 // Column sums of a (rows x n) row-major matrix, first stage: part[chunk][c] over
@@ -76,14 +114,17 @@ __global__ void colsum_part_kernel(const float* __restrict__ x, long long rows, 
   }
 }
 
-// out[j] = sum over chunks k (in order) of part[k][j]
+// out[j] = sum over chunks k of part[k][j], one warp per column: a lane adds chunks lane,
+// lane + 32, ... in order, then the lanes add up in a fixed tree.  (One thread per column
+// took 14 us for 512 chunks.)
 __global__ void reduce_parts_kernel(const float* __restrict__ part, int nchunks, int n, float* __restrict__ out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
+  const int j = blockIdx.x, lane = threadIdx.x;
   float s = 0.f;
-#pragma unroll 32
-  for (int k = 0; k < nchunks; ++k) s += part[(size_t)k * n + j];
-  out[j] = s;
+#pragma unroll 8
+  for (int k = lane; k < nchunks; k += 32) s += part[(size_t)k * n + j];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) out[j] = s;
 }
 
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
@@ -297,13 +338,35 @@ Addr u_rows_smc(const msx_corrector* k) {
 // X or Y as rows (s, m, c) x columns (2 n + re/im).
 Addr x_rows_smc(const msx_corrector* k) { return Addr{2LL * k->MY * k->C, 1, k->C, k->C, 0, 1}; }
 
+constexpr long long kSumChunk = 4096;  // rows of a partial column sum
+
+int sum_chunks(msx_corrector* k, long long rows, int n) {
+  const int nchunks = (int)((rows + kSumChunk - 1) / kSumChunk);
+  return (size_t)nchunks * n > k->part_words ? -1 : nchunks;
+}
+
 // out[j] = column sums of x (rows x n), n in {4, 32, 64, ...} dividing 256
 int colsum(msx_corrector* k, const float* x, long long rows, int n, float* out, cudaStream_t st) {
-  const long long chunk = 4096;
-  const int nchunks = (int)((rows + chunk - 1) / chunk);
-  if ((size_t)nchunks * n > k->part_words) return cfail(MSX_ERR_INVALID, "corrector: reduction buffer too small");
-  colsum_part_kernel<<<nchunks, 256, 0, st>>>(x, rows, n, chunk, k->part);
-  reduce_parts_kernel<<<blocks_for(n, 128), 128, 0, st>>>(k->part, nchunks, n, out);
+  const int nchunks = sum_chunks(k, rows, n);
+  if (nchunks < 0) return cfail(MSX_ERR_INVALID, "corrector: reduction buffer too small");
+  colsum_part_kernel<<<nchunks, 256, 0, st>>>(x, rows, n, kSumChunk, k->part);
+  reduce_parts_kernel<<<n, 32, 0, st>>>(k->part, nchunks, n, out);
+  NN_CUDA(cudaGetLastError());
+  return MSX_OK;
+}
+
+// dz = da * gelu'(z) over rows x n values, and its column sums.  Layers lie rows * n values
+// apart, so fewer than 4 channels may leave them unaligned: value by value then.
+int gelu_bwd(msx_corrector* k, const float* da, const float* z, long long rows, int n, float* dz, float* sums,
+             cudaStream_t st) {
+  if (n % 4 != 0) {
+    gelu_bwd_kernel<<<blocks_for(rows * n, 256), 256, 0, st>>>(da, z, rows * n, dz);
+    return colsum(k, dz, rows, n, sums, st);
+  }
+  const int nchunks = sum_chunks(k, rows, n);
+  if (nchunks < 0) return cfail(MSX_ERR_INVALID, "corrector: reduction buffer too small");
+  gelu_bwd_sum_kernel<<<nchunks, 256, 0, st>>>(da, z, rows, n, kSumChunk, dz, k->part);
+  reduce_parts_kernel<<<n, 32, 0, st>>>(k->part, nchunks, n, sums);
   NN_CUDA(cudaGetLastError());
   return MSX_OK;
 }
@@ -396,13 +459,6 @@ int forward(msx_corrector* k, int S, cudaStream_t st) {
   return MSX_OK;
 }
 
-// dz = da * gelu'(z) over n values.  Layers lie n values apart, so an n that is no
-// multiple of 4 (odd grids with few channels) leaves them unaligned.
-void gelu_bwd(const float* da, const float* z, size_t n, float* dz, cudaStream_t st) {
-  if (n % 4 == 0) gelu_bwd_kernel<4><<<blocks_for((long long)(n / 4), 256), 256, 0, st>>>(da, z, (long long)n, dz);
-  else gelu_bwd_kernel<1><<<blocks_for((long long)n, 256), 256, 0, st>>>(da, z, (long long)n, dz);
-}
-
 int backward(msx_corrector* k, const float* dmaps, cudaStream_t st) {
   const int S = k->S_last;
   const long long SP = (long long)S * k->P;
@@ -415,18 +471,15 @@ int backward(msx_corrector* k, const float* dmaps, cudaStream_t st) {
   if ((rc = wgrad(k, dmaps, 4, k->h, C, S, G + k->oP2, st))) return rc;
   if ((rc = colsum(k, dmaps, SP, 4, G + k->oc2, st))) return rc;
   NN_GEMM(k->gemm.run(dmaps, rowmajor(4), Pm + k->oP2, colmajor(C), SP, C, 4, epi(k->dz, rowmajor(C)), st));
-  gelu_bwd(k->dz, k->zh, A, k->dz, st);
+  if ((rc = gelu_bwd(k, k->dz, k->zh, SP, C, k->dz, G + k->oc1, st))) return rc;
   if ((rc = wgrad(k, k->dz, C, k->a + (size_t)k->L * A, C, S, G + k->oP1, st))) return rc;
-  if ((rc = colsum(k, k->dz, SP, C, G + k->oc1, st))) return rc;
   NN_GEMM(k->gemm.run(k->dz, rowmajor(C), Pm + k->oP1, colmajor(C), SP, C, C, epi(k->da, rowmajor(C)), st));
   for (int l = k->L - 1; l >= 0; --l) {
     const float* ain = k->a + (size_t)l * A;
     const float* zl = k->z + (size_t)l * A;
     const float* Xl = k->Xh + (size_t)l * x_words(k, S);
-    gelu_bwd(k->da, zl, A, k->dz, st);
-    NN_CUDA(cudaGetLastError());
+    if ((rc = gelu_bwd(k, k->da, zl, SP, C, k->dz, G + k->ob[l], st))) return rc;
     if ((rc = wgrad(k, k->dz, C, ain, C, S, G + k->oW[l], st))) return rc;
-    if ((rc = colsum(k, k->dz, SP, C, G + k->ob[l], st))) return rc;
     // pointwise part: da2 = dz W_l
     NN_GEMM(k->gemm.run(k->dz, rowmajor(C), Pm + k->oW[l], colmajor(C), SP, C, C, epi(k->da2, rowmajor(C)), st));
     // spectral part, in reverse: IDFT_x^T, IDFT_y^T, mixing, DFT_y^T, DFT_x^T
