@@ -440,6 +440,11 @@ struct StreamImpl {
       const cudaError_t e = StreamImpl<LR, LC, 2>::configure();
       if (e != cudaSuccess) return e;
     }
+    // the registers the roles take must be there at launch, or setmaxnreg waits for good
+    cudaFuncAttributes fa{};
+    const cudaError_t e = cudaFuncGetAttributes(&fa, stream_kernel<LR, LC, MINB>);
+    if (e != cudaSuccess) return e;
+    if (fa.numRegs * K::THREADS < (MINB == 2 ? 256 * 104 + 128 * 32 : 256 * 232 + 128 * 40)) return cudaErrorInvalidConfiguration;
     return cudaFuncSetAttribute(stream_kernel<LR, LC, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::smem());
   }
   static cudaError_t launch(const CUtensorMap& map, const StreamArgs& a, int sms, cudaStream_t st) {

@@ -1433,6 +1433,11 @@ cudaError_t ws_slots(int& slots) {
   const int d = dev & 63;
   int v = cache[d].load(std::memory_order_acquire);
   if (v <= 0) {
+    // the registers the roles take must be there at launch, or setmaxnreg waits for good
+    cudaFuncAttributes fa{};
+    c = cudaFuncGetAttributes(&fa, gemm_ws_kernel<BN, FUSE>);
+    if (c != cudaSuccess) return c;
+    if (fa.numRegs * ws::THREADS < 128 * (120 + 56 + 2 * 168)) return cudaErrorInvalidConfiguration;
     c = cudaFuncSetAttribute(gemm_ws_kernel<BN, FUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws::Cfg<BN>::SMEM);
     if (c != cudaSuccess) return c;
     // all of the unified L1 as shared memory
