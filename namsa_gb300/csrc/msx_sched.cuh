@@ -110,6 +110,7 @@ int schedules_128(const SchedOps** out);
 int schedules_256(const SchedOps** out);
 int schedules_384(const SchedOps** out);
 int schedules_512(const SchedOps** out);
+SchedOps schedule_512_c8();  // in a module of its own: one of 12 MB took 10 ms to load, these take 2
 int schedules_768(const SchedOps** out);
 int schedules_1024(const SchedOps** out);
 
