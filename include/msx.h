@@ -18,7 +18,10 @@
  *    pairs.  Nothing is synchronised: work is ordered on `stream`
  *    (a cudaStream_t, NULL = the legacy default stream).
  *  - A plan owns its workspace and is not re-entrant; distinct plans may be
- *    used from distinct threads.
+ *    used from distinct threads.  Multislice and detector calls of one plan
+ *    from different streams run one after another.  A call under a stream
+ *    capture is recorded on the capturing stream: its replays must not overlap
+ *    other calls of the plan.
  *  - Supported grid line lengths (msx_supported_size): 64, 128, 256, 384,
  *    512, 768, 1024 on each axis.
  */

@@ -615,6 +615,33 @@ bool few_launches(msx_plan* p, const MsArgs& a) {
   return g > 0 && a.num_probes <= 2 * g;
 }
 
+// Runs enqueue(stream) on the plan's stream, ordered after and before the caller's: calls
+// of one plan share its waves, tables, partial sums and counters, whichever streams they
+// come from.  Under a capture it joins the caller's stream, and the caller keeps the
+// captured work apart from the plan's other calls.
+template <class F>
+int on_plan_stream(msx_plan* p, cudaStream_t caller, F enqueue) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  MSX_CUDA(cudaStreamIsCapturing(caller, &cap), "cudaStreamIsCapturing");
+  if (cap != cudaStreamCaptureStatusNone) return enqueue(caller, true);
+  MSX_CUDA(cudaEventRecord(p->ev_in, caller), "cudaEventRecord");
+  MSX_CUDA(cudaStreamWaitEvent(p->work, p->ev_in, 0), "cudaStreamWaitEvent");
+  const int rc = enqueue(p->work, false);
+  const std::string msg = g_err;
+  // also after a failure: what was enqueued before it still uses the caller's buffers
+  MSX_CUDA(cudaEventRecord(p->ev_out, p->work), "cudaEventRecord");
+  MSX_CUDA(cudaStreamWaitEvent(caller, p->ev_out, 0), "cudaStreamWaitEvent");
+  if (rc != MSX_OK) g_err = msg;
+  return rc;
+}
+
+// Orders `st`, on which a tuning or timing call is about to use the plan, after the plan's own work.
+int after_plan_stream(msx_plan* p, cudaStream_t st) {
+  MSX_CUDA(cudaEventRecord(p->ev_out, p->work), "cudaEventRecord");
+  MSX_CUDA(cudaStreamWaitEvent(st, p->ev_out, 0), "cudaStreamWaitEvent");
+  return MSX_OK;
+}
+
 int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const HostPipe* hp = nullptr) {
   const int ny = p->ny, nx = p->nx;
   const int cluster = resident_cluster(p, a);
@@ -989,46 +1016,32 @@ int msx_multislice(msx_plan* p, const float* trans_dev, int num_slices, const fl
   a.pos = positions_dev; a.num_probes = num_probes; a.kmax = kmax; a.lambda = lambda; a.slice_t = slice_t;
   a.k_band = k_band; a.cbed = cbed_out_dev; a.crop_y = crop_y; a.crop_x = crop_x;
   a.group = p->group; a.row_sched = p->row_sched; a.col_sched = p->col_sched;
-  cudaStream_t caller = (cudaStream_t)stream;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  MSX_CUDA(cudaStreamIsCapturing(caller, &cap), "cudaStreamIsCapturing");
-  if (cap != cudaStreamCaptureStatusNone || !p->use_graph) return enqueue_multislice(p, a, caller);
-
-  // Run on the plan's stream, ordered after and before the caller's stream.
-  MSX_CUDA(cudaEventRecord(p->ev_in, caller), "cudaEventRecord");
-  MSX_CUDA(cudaStreamWaitEvent(p->work, p->ev_in, 0), "cudaStreamWaitEvent");
-  if (few_launches(p, a)) {
-    const int rc = enqueue_multislice(p, a, p->work);
-    if (rc != MSX_OK) return rc;
-    MSX_CUDA(cudaEventRecord(p->ev_out, p->work), "cudaEventRecord");
-    MSX_CUDA(cudaStreamWaitEvent(caller, p->ev_out, 0), "cudaStreamWaitEvent");
+  return on_plan_stream(p, (cudaStream_t)stream, [&](cudaStream_t st, bool captured) -> int {
+    if (captured || !p->use_graph || few_launches(p, a)) return enqueue_multislice(p, a, st);
+    std::vector<unsigned char> key(sizeof(MsArgs));
+    std::memcpy(key.data(), &a, sizeof(MsArgs));
+    if (!p->gexec || key != p->gkey) {
+      drop_graph(p);
+      cudaGraph_t graph = nullptr;
+      MSX_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
+      const int rc = enqueue_multislice(p, a, st);
+      cudaError_t e = cudaStreamEndCapture(st, &graph);
+      if (rc != MSX_OK) {
+        if (graph) cudaGraphDestroy(graph);
+        return rc;
+      }
+      if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
+      e = cudaGraphInstantiate(&p->gexec, graph, 0);
+      cudaGraphDestroy(graph);
+      if (e != cudaSuccess) {
+        p->gexec = nullptr;
+        return cuda_fail(e, "cudaGraphInstantiate");
+      }
+      p->gkey = key;
+    }
+    MSX_CUDA(cudaGraphLaunch(p->gexec, st), "cudaGraphLaunch");
     return MSX_OK;
-  }
-  std::vector<unsigned char> key(sizeof(MsArgs));
-  std::memcpy(key.data(), &a, sizeof(MsArgs));
-  if (!p->gexec || key != p->gkey) {
-    drop_graph(p);
-    cudaGraph_t graph = nullptr;
-    MSX_CUDA(cudaStreamBeginCapture(p->work, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-    const int rc = enqueue_multislice(p, a, p->work);
-    cudaError_t e = cudaStreamEndCapture(p->work, &graph);
-    if (rc != MSX_OK) {
-      if (graph) cudaGraphDestroy(graph);
-      return rc;
-    }
-    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
-    e = cudaGraphInstantiate(&p->gexec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) {
-      p->gexec = nullptr;
-      return cuda_fail(e, "cudaGraphInstantiate");
-    }
-    p->gkey = key;
-  }
-  MSX_CUDA(cudaGraphLaunch(p->gexec, p->work), "cudaGraphLaunch");
-  MSX_CUDA(cudaEventRecord(p->ev_out, p->work), "cudaEventRecord");
-  MSX_CUDA(cudaStreamWaitEvent(caller, p->ev_out, 0), "cudaStreamWaitEvent");
-  return MSX_OK;
+  });
 }
 
 int msx_multislice_detect(msx_plan* p, const float* trans_dev, int num_slices, const float* psi_k_dev,
@@ -1060,7 +1073,8 @@ int msx_multislice_detect(msx_plan* p, const float* trans_dev, int num_slices, c
   a.k_band = k_band; a.crop_y = p->ny; a.crop_x = p->nx; a.group = p->group; a.row_sched = p->row_sched;
   a.col_sched = p->col_sched; a.det = detectors_dev; a.ndet = num_detectors; a.signals = signals_out_dev;
   drop_graph(p);  // the detector sequence is launched directly
-  return enqueue_multislice(p, a, (cudaStream_t)stream);
+  return on_plan_stream(p, (cudaStream_t)stream,
+                        [&](cudaStream_t st, bool) -> int { return enqueue_multislice(p, a, st); });
 }
 
 int msx_propagator_table(int ny, int nx, float kmax, double lambda, double slice_t, float k_band, float* ptab_out_dev,
@@ -1305,7 +1319,8 @@ int msx_plan_profile(msx_plan* p, const float* trans_dev, int num_slices, const 
     return fail(MSX_ERR_ALLOC, "the plan's workspace does not hold %d waves (an earlier allocation failed)", gn);
   const size_t wave = (size_t)ny * nx;
   cudaStream_t st = (cudaStream_t)stream;
-  const int rcp = ensure_ptab(p);
+  int rcp = ensure_ptab(p);
+  if (rcp == MSX_OK) rcp = after_plan_stream(p, st);
   if (rcp != MSX_OK) return rcp;
   cudaEvent_t ev[4];
   for (auto& e : ev) MSX_CUDA(cudaEventCreate(&e), "cudaEventCreate");
@@ -1357,7 +1372,8 @@ int msx_plan_autotune(msx_plan* p, const float* trans_dev, int num_slices, const
   if (!p) return fail(MSX_ERR_INVALID, "null plan");
   if (iters <= 0 || num_slices <= 0 || num_probes <= 0 || !trans_dev || !psi_k_dev || !normalization_dev || !positions_dev)
     return fail(MSX_ERR_INVALID, "autotune needs slices, probes, inputs and iters > 0");
-  const int rcp = ensure_ptab(p);
+  int rcp = ensure_ptab(p);
+  if (rcp == MSX_OK) rcp = after_plan_stream(p, (cudaStream_t)stream);
   if (rcp != MSX_OK) return rcp;
   const SchedOps *rops, *cops;
   const int nr = schedule_table(p->nx, &rops), nc = schedule_table(p->ny, &cops);
