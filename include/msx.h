@@ -370,7 +370,8 @@ MSX_API int msx_batch_check(msx_batch* batch);
  *  msx_tc_set_compensation: 1 (default) / 0 turns the norm compensation on / off
  *                     for the calling host thread
  *  msx_tc_check:      synchronises; MSX_ERR_TIMEOUT if a bounded wait gave up
- * Scratch is held per host thread and grows with the largest call.
+ * Scratch is held per host thread and device and grows with the largest call; a
+ * thread's calls from different streams run one after another.
  */
 MSX_API int msx_tc_dft(const float* x_dev, int lines, int n, int sign, float* z_dev, void* stream);
 MSX_API int msx_step_waves_tc(float* waves_dev, int num_waves, int n, const float* trans_dev, const float* ptab_dev,
@@ -384,7 +385,8 @@ MSX_API int msx_tc_check(void);
  * with a and b rounded to bfloat16 and FP32 accumulation on tcgen05; with
  * accumulate = 1 the product is added to c.  a, b, c are FP32 row-major with
  * leading dimensions lda, ldb, ldc (elements); n <= 4096.  Operand images are
- * held per host thread and grow with the largest call.  msx_gemm_check
+ * held per host thread and device and grow with the largest call; a thread's
+ * calls from different streams run one after another.  msx_gemm_check
  * synchronises and reports MSX_ERR_TIMEOUT if a bounded wait gave up.
  */
 MSX_API int msx_gemm_bf16(const float* a_dev, int lda, const float* b_dev, int ldb, int m, int n, int k, float* c_dev,

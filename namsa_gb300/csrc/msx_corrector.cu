@@ -755,20 +755,30 @@ int msx_corrector_residual(const float* psi_dev, const float* target_dev, int nu
     return cfail(MSX_ERR_INVALID, "corrector residual: bad arguments");
   const long long n = (long long)num * ny * nx;
   const unsigned nb = blocks_for(n, 256);
-  thread_local double* sums = nullptr;
-  thread_local size_t cap = 0;
-  if (nb > cap) {
-    if (sums) cudaFree(sums);
-    sums = nullptr;
-    cap = 0;
-    if (cudaMalloc(&sums, nb * sizeof(double)) != cudaSuccess) return cfail(MSX_ERR_ALLOC, "loss partials");
-    cap = nb;
+  struct Scratch {
+    double* sums = nullptr;
+    size_t cap = 0;
+    ScratchOrder order;
+  };
+  thread_local PerDevice<Scratch> scratch;
+  Scratch* k = scratch.here();
+  if (!k) return cfail(MSX_ERR_CUDA, "corrector residual: no device");
+  if (nb > k->cap) {
+    if (k->sums) cudaFree(k->sums);
+    k->sums = nullptr;
+    k->cap = 0;
+    if (cudaMalloc(&k->sums, nb * sizeof(double)) != cudaSuccess) return cfail(MSX_ERR_ALLOC, "loss partials");
+    k->cap = nb;
   }
   cudaStream_t st = (cudaStream_t)stream;
+  double* const sums = k->sums;
+  NN_CUDA(k->order.enter(st));
   resid_kernel<<<nb, 256, 0, st>>>(reinterpret_cast<const float2*>(psi_dev), reinterpret_cast<const float2*>(target_dev),
                                    n, weight, accumulate ? 1 : 0, reinterpret_cast<float2*>(adjoint_dev), sums);
   sum_blocks_kernel<<<1, 256, 0, st>>>(sums, (int)nb, loss_out_dev);
-  NN_CUDA(cudaGetLastError());
+  const cudaError_t launched = cudaGetLastError();
+  NN_CUDA(k->order.leave(st));
+  NN_CUDA(launched);
   return MSX_OK;
 }
 

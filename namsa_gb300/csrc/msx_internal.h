@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <map>
+
 #include "msx_sched.cuh"
 #include "msx_resident.cuh"
 #include "msx_stream.cuh"
@@ -24,6 +26,42 @@ cudaError_t launch_pfac(int Ny, int Nx, float kmax, double lambda, double slice_
                         int2* band, cudaStream_t st);
 cudaError_t launch_ptab(int Ny, int Nx, float kmax, double lambda, double slice_t, float k_band, float2* ptab,
                         cudaStream_t st);
+
+// Order of the calls that use one piece of scratch, from whichever streams.  Under a
+// capture nothing is recorded: the caller orders the replays with the other calls.
+struct ScratchOrder {
+  cudaEvent_t last = nullptr;  // after the last use; null before the first
+  cudaError_t enter(cudaStream_t st) {  // st follows the last call
+    const int c = captured(st);
+    return c < 0 ? cudaErrorInvalidValue : c || !last ? cudaSuccess : cudaStreamWaitEvent(st, last, 0);
+  }
+  cudaError_t leave(cudaStream_t st) {  // also where a launch in between failed
+    const int c = captured(st);
+    if (c) return c < 0 ? cudaErrorInvalidValue : cudaSuccess;
+    if (!last) {
+      const cudaError_t e = cudaEventCreateWithFlags(&last, cudaEventDisableTiming);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaEventRecord(last, st);
+  }
+
+ private:
+  static int captured(cudaStream_t st) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) return -1;
+    return cap != cudaStreamCaptureStatusNone ? 1 : 0;
+  }
+};
+
+// A host thread's scratch T on the current device (its allocations belong to that device).
+template <class T>
+struct PerDevice {
+  std::map<int, T> of;  // its elements stay where they are
+  T* here() {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess ? &of[dev] : nullptr;
+  }
+};
 
 // Strided addressing of a matrix element (r, k):
 //   (r / rc) * s1 + (r % rc) * s2 + (k / kc) * t1 + (k % kc) * t2.

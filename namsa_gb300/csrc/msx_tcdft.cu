@@ -288,12 +288,17 @@ struct TcState {
   int* err = nullptr;
   size_t lines_cap = 0;
   bool configured = false;
+  ScratchOrder order;
 };
-thread_local TcState g_tc;  // one per host thread; sized by the largest call
+thread_local PerDevice<TcState> g_tc;  // per host thread and device; sized by the largest call
 thread_local bool g_tc_compensate = true;
 
-int tc_prepare(int N, size_t lines) {
-  TcState& s = g_tc;
+// The scratch for calls of this size on `st`, after the last call that used it; null on failure.
+int tc_prepare(int N, size_t lines, cudaStream_t st, TcState** out) {
+  TcState* const here = g_tc.here();
+  if (!here) return tfail(MSX_ERR_CUDA, "tensor-core DFT: no device");
+  TcState& s = *here;
+  *out = here;
   if (s.N != N) {
     for (void* p : {(void*)s.fwd_hi, (void*)s.fwd_lo, (void*)s.inv_hi, (void*)s.inv_lo})
       if (p) cudaFree(p);
@@ -330,12 +335,18 @@ int tc_prepare(int N, size_t lines) {
       return tfail(MSX_ERR_CUDA, "tensor-core GEMM: shared memory attribute");
     s.configured = true;
   }
+  if (s.order.enter(st) != cudaSuccess) return tfail(MSX_ERR_CUDA, "tensor-core DFT: stream order");
   return MSX_OK;
 }
 
+int tc_leave(TcState& s, cudaStream_t st, int rc) {
+  if (s.order.leave(st) != cudaSuccess && rc == MSX_OK) return tfail(MSX_ERR_CUDA, "tensor-core DFT: stream order");
+  return rc;
+}
+
 // Z (lines x N complex) = DFT of sign `sign` of X (lines x N) (X * mult when mult != null)
-int tc_dft(const float2* X, size_t lines, int N, const float2* mult, int lm, int sign, float2* Z, cudaStream_t st) {
-  TcState& s = g_tc;
+int tc_dft(TcState& s, const float2* X, size_t lines, int N, const float2* mult, int lm, int sign, float2* Z,
+           cudaStream_t st) {
   const bool comp = g_tc_compensate;
   tc_split_kernel<<<(unsigned)lines, 256, 0, st>>>(X, N, mult, lm, s.a_hi, s.a_lo, comp ? s.nin : nullptr);
   const int kblocks = 2 * N / BK, ntn = 2 * N / BN;
@@ -358,10 +369,12 @@ extern "C" {
 int msx_tc_dft(const float* x_dev, int lines, int n, int sign, float* z_dev, void* stream) {
   if (!x_dev || !z_dev || (n != 256 && n != 512) || lines <= 0 || lines % BM || (sign != 1 && sign != -1))
     return tfail(MSX_ERR_INVALID, "tc_dft: n must be 256 or 512, lines a positive multiple of 128, sign +-1");
-  int rc = tc_prepare(n, (size_t)lines);
+  cudaStream_t st = (cudaStream_t)stream;
+  TcState* s = nullptr;
+  const int rc = tc_prepare(n, (size_t)lines, st, &s);
   if (rc) return rc;
-  return tc_dft(reinterpret_cast<const float2*>(x_dev), (size_t)lines, n, nullptr, 1, sign,
-                reinterpret_cast<float2*>(z_dev), (cudaStream_t)stream);
+  return tc_leave(*s, st, tc_dft(*s, reinterpret_cast<const float2*>(x_dev), (size_t)lines, n, nullptr, 1, sign,
+                                 reinterpret_cast<float2*>(z_dev), st));
 }
 
 int msx_step_waves_tc(float* waves_dev, int num_waves, int n, const float* trans_dev, const float* ptab_dev,
@@ -369,23 +382,28 @@ int msx_step_waves_tc(float* waves_dev, int num_waves, int n, const float* trans
   if (!waves_dev || !trans_dev || !ptab_dev || num_waves <= 0 || (n != 256 && n != 512))
     return tfail(MSX_ERR_INVALID, "step_waves_tc: square grids of 256 or 512 only");
   const size_t lines = (size_t)num_waves * n;
-  int rc = tc_prepare(n, lines);
-  if (rc) return rc;
-  TcState& s = g_tc;
   cudaStream_t st = (cudaStream_t)stream;
+  TcState* scratch = nullptr;
+  const int prepared = tc_prepare(n, lines, st, &scratch);
+  if (prepared) return prepared;
+  TcState& s = *scratch;
   float2* w = reinterpret_cast<float2*>(waves_dev);
   const dim3 tb(32, 8), tg(n / 32, n / 32, num_waves), tg1(n / 32, n / 32, 1);
-  // P^T once per call: rows kx, columns ky
-  transpose_kernel<<<tg1, tb, 0, st>>>(reinterpret_cast<const float2*>(ptab_dev), n, s.ptab_t);
-  // psi (rows y, cols x) -> t psi -> DFT_x
-  if ((rc = tc_dft(w, lines, n, reinterpret_cast<const float2*>(trans_dev), n, -1, s.z0, st))) return rc;
-  transpose_kernel<<<tg, tb, 0, st>>>(s.z0, n, s.z1);                      // rows kx, cols y
-  if ((rc = tc_dft(s.z1, lines, n, nullptr, 1, -1, s.z0, st))) return rc;  // DFT_y: rows kx, cols ky
-  if ((rc = tc_dft(s.z0, lines, n, s.ptab_t, n, +1, s.z1, st))) return rc; // * P/N, inverse DFT_y
-  transpose_kernel<<<tg, tb, 0, st>>>(s.z1, n, s.z0);                      // rows y, cols kx
-  if ((rc = tc_dft(s.z0, lines, n, nullptr, 1, +1, w, st))) return rc;     // inverse DFT_x
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? MSX_OK : tfail(MSX_ERR_CUDA, cudaGetErrorString(e));
+  auto step = [&]() -> int {
+    int rc;
+    // P^T once per call: rows kx, columns ky
+    transpose_kernel<<<tg1, tb, 0, st>>>(reinterpret_cast<const float2*>(ptab_dev), n, s.ptab_t);
+    // psi (rows y, cols x) -> t psi -> DFT_x
+    if ((rc = tc_dft(s, w, lines, n, reinterpret_cast<const float2*>(trans_dev), n, -1, s.z0, st))) return rc;
+    transpose_kernel<<<tg, tb, 0, st>>>(s.z0, n, s.z1);                      // rows kx, cols y
+    if ((rc = tc_dft(s, s.z1, lines, n, nullptr, 1, -1, s.z0, st))) return rc;  // DFT_y: rows kx, cols ky
+    if ((rc = tc_dft(s, s.z0, lines, n, s.ptab_t, n, +1, s.z1, st))) return rc; // * P/N, inverse DFT_y
+    transpose_kernel<<<tg, tb, 0, st>>>(s.z1, n, s.z0);                      // rows y, cols kx
+    if ((rc = tc_dft(s, s.z0, lines, n, nullptr, 1, +1, w, st))) return rc;     // inverse DFT_x
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? MSX_OK : tfail(MSX_ERR_CUDA, cudaGetErrorString(e));
+  };
+  return tc_leave(s, st, step());
 }
 
 int msx_tc_set_compensation(int enable) {
@@ -394,12 +412,14 @@ int msx_tc_set_compensation(int enable) {
 }
 
 int msx_tc_check(void) {
-  if (!g_tc.err) return MSX_OK;
+  TcState* s = g_tc.here();
+  if (!s) return tfail(MSX_ERR_CUDA, "tensor-core DFT: no device");
+  if (!s->err) return MSX_OK;
   int h = 0;
-  if (cudaMemcpy(&h, g_tc.err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+  if (cudaMemcpy(&h, s->err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
     return tfail(MSX_ERR_CUDA, "reading the tensor-core error word");
   if (h) {
-    cudaMemset(g_tc.err, 0, sizeof(int));
+    cudaMemset(s->err, 0, sizeof(int));
     return tfail(MSX_ERR_TIMEOUT, "a tensor-core DFT wait gave up");
   }
   return MSX_OK;

@@ -1733,8 +1733,13 @@ int TcGemm::check() {
 }  // namespace msx
 
 namespace {
-thread_local msx::TcGemm g_gemm;  // scratch of msx_gemm_bf16, one per host thread
-}
+// scratch of msx_gemm_bf16, per host thread and device
+struct GemmScratch {
+  msx::TcGemm gemm;
+  msx::ScratchOrder order;
+};
+thread_local msx::PerDevice<GemmScratch> g_gemm;
+}  // namespace
 
 extern "C" int msx_gemm_bf16(const float* a_dev, int lda, const float* b_dev, int ldb, int m, int n, int k,
                              float* c_dev, int ldc, const float* bias_dev, int accumulate, void* stream) {
@@ -1751,8 +1756,14 @@ extern "C" int msx_gemm_bf16(const float* a_dev, int lda, const float* b_dev, in
   // long K with few output tiles: split K over CTAs
   const long long tiles = ((m + 127) / 128) * (long long)((n + 255) / 256);
   const int ksplit = (k >= 4096 && tiles < 64) ? (int)((k / 2048) < 64 ? (k / 2048) : 64) : 1;
-  const int rc = g_gemm.run(a_dev, msx::rowmajor(lda), b_dev, msx::rowmajor(ldb), m, n, k, e, (cudaStream_t)stream,
-                            ksplit);
+  const cudaStream_t st = (cudaStream_t)stream;
+  GemmScratch* g = g_gemm.here();
+  if (!g || g->order.enter(st) != cudaSuccess) {
+    msx::set_last_error("gemm_bf16: no device, or its stream is unusable");
+    return MSX_ERR_CUDA;
+  }
+  int rc = g->gemm.run(a_dev, msx::rowmajor(lda), b_dev, msx::rowmajor(ldb), m, n, k, e, st, ksplit);
+  if (g->order.leave(st) != cudaSuccess && rc == MSX_OK) rc = MSX_ERR_CUDA;
   if (rc == MSX_ERR_ALLOC) msx::set_last_error("gemm_bf16: operand image allocation failed");
   else if (rc == MSX_ERR_CUDA) msx::set_last_error("gemm_bf16: launch failed");
   else if (rc != MSX_OK) msx::set_last_error("gemm_bf16: bad sizes");
@@ -1760,7 +1771,8 @@ extern "C" int msx_gemm_bf16(const float* a_dev, int lda, const float* b_dev, in
 }
 
 extern "C" int msx_gemm_check(void) {
-  const int rc = g_gemm.check();
+  GemmScratch* g = g_gemm.here();
+  const int rc = g ? g->gemm.check() : MSX_ERR_CUDA;
   if (rc == MSX_ERR_TIMEOUT) msx::set_last_error("a tensor-core GEMM wait gave up");
   return rc;
 }
