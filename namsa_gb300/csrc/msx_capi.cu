@@ -455,6 +455,10 @@ bool few_cols(const msx_plan* p, int gn, float kmax, float k_band, int* x_lo, in
   return false;
 }
 
+// Whether the passes run as persistent kernels: their bulk copies of transmission rows
+// start on 16-byte boundaries.
+bool tma_passes(const msx_plan* p, const void* trans) { return p->use_tma && p->map_ok && aligned(trans, 16); }
+
 // x_lo, x_hi: the column range of the TMA passes (0, 0 = all columns); the
 // plain passes always cover every column.  fr, fc: the row, column pass with the
 // schedule for few lines.
@@ -653,7 +657,7 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
   // the persistent passes form the propagator from its factors and the mask band;
   // the table of N values (26 us of double precision at 512^2, 89 us at 1024^2)
   // serves the plain passes
-  const bool tma = p->use_tma && p->map_ok && aligned(a.trans, 16);  // bulk copies start on 16-byte boundaries
+  const bool tma = tma_passes(p, a.trans);
   const bool factors = tma;
   if (!factors) {
     const int rc = ensure_ptab(p);
@@ -1336,13 +1340,14 @@ int msx_plan_profile(msx_plan* p, const float* trans_dev, int num_slices, const 
   // the steady-state passes of multislice: the band-limited column range
   int bx_lo = 0, bx_hi = 0;
   band_columns(nx, kmax, k_band, p->col_ops->col_c, &bx_lo, &bx_hi);
+  const bool tma = tma_passes(p, trans_dev);
   for (int i = 0; i < iters; ++i) {
     const int s = i % num_slices;
     MSX_CUDA(cudaEventRecord(ev[0], st), "cudaEventRecord");
-    int rc = slice_passes(p, trans + (size_t)s * wave, gn, c, false, st, bx_lo, bx_hi, p->use_tma && p->map_ok);
+    int rc = slice_passes(p, trans + (size_t)s * wave, gn, c, false, st, bx_lo, bx_hi, tma);
     if (rc != MSX_OK) return rc;
     MSX_CUDA(cudaEventRecord(ev[1], st), "cudaEventRecord");
-    if (p->use_tma && p->map_ok) {
+    if (tma) {
       TmaPassArgs ta{};
       ta.psi = p->psi; ta.tw = p->tw_col; ta.pyx = p->pyx; ta.band = p->band; ta.err = p->err;
       ta.G = gn; ta.Ny = ny; ta.Nx = nx; ta.x_lo = bx_lo; ta.x_hi = bx_hi;
@@ -1412,9 +1417,9 @@ int msx_plan_autotune(msx_plan* p, const float* trans_dev, int num_slices, const
       for (int i = 0; i < iters; ++i) {
         if (row_pass) {
           const int r2 = slice_passes(p, trans + (size_t)(i % num_slices) * wave, g, c, false, st, bx_lo, bx_hi,
-                                       p->use_tma && p->map_ok);
+                                       tma_passes(p, trans));
           if (r2 != MSX_OK) return r2;
-        } else if (p->use_tma && p->map_ok) {
+        } else if (tma_passes(p, trans)) {
           TmaPassArgs ta{};
           ta.psi = p->psi; ta.tw = p->tw_col; ta.pyx = p->pyx; ta.band = p->band; ta.err = p->err;
           ta.G = g; ta.Ny = p->ny; ta.Nx = p->nx; ta.x_lo = bx_lo; ta.x_hi = bx_hi;
