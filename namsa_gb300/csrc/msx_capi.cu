@@ -10,6 +10,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -88,6 +89,13 @@ int ensure_configured(int device, int n, int idx, const SchedOps& op) {
 }
 
 bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
+// Every pointer on an 8-byte boundary (null is): complex values and position pairs are loaded whole.
+bool aligned8(std::initializer_list<const void*> ps) {
+  for (const void* p : ps)
+    if (!aligned(p, 8)) return false;
+  return true;
+}
+constexpr const char* kAlign8 = "complex inputs, positions and the normalisation must be 8-byte aligned";
 
 }  // namespace
 
@@ -1006,8 +1014,7 @@ int msx_multislice(msx_plan* p, const float* trans_dev, int num_slices, const fl
     return fail(MSX_ERR_INVALID, "crop %d x %d outside the %d x %d grid", crop_y, crop_x, p->ny, p->nx);
   if (!psi_k_dev || !normalization_dev || !positions_dev || !cbed_out_dev || (num_slices > 0 && !trans_dev))
     return fail(MSX_ERR_INVALID, "null pointer");
-  if (!aligned(trans_dev, 8) || !aligned(psi_k_dev, 8) || !aligned(positions_dev, 8) || !aligned(normalization_dev, 8))
-    return fail(MSX_ERR_INVALID, "complex inputs, positions and the normalisation must be 8-byte aligned");
+  if (!aligned8({trans_dev, psi_k_dev, positions_dev, normalization_dev})) return fail(MSX_ERR_INVALID, kAlign8);
   if (!(kmax > 0) || !(lambda > 0) || !(slice_t >= 0) || !(k_band >= 0))
     return fail(MSX_ERR_INVALID, "kmax, lambda must be positive; slice thickness and k_band non-negative");
   int dev = 0;
@@ -1059,6 +1066,7 @@ int msx_multislice_detect(msx_plan* p, const float* trans_dev, int num_slices, c
     return fail(MSX_ERR_INVALID, "1..%d detectors supported, got %d", kMaxDetectors, num_detectors);
   if (!trans_dev || !psi_k_dev || !normalization_dev || !positions_dev || !detectors_dev || !signals_out_dev)
     return fail(MSX_ERR_INVALID, "null pointer");
+  if (!aligned8({trans_dev, psi_k_dev, positions_dev, normalization_dev})) return fail(MSX_ERR_INVALID, kAlign8);
   if (!(kmax > 0) || !(lambda > 0) || !(slice_t >= 0) || !(k_band >= 0))
     return fail(MSX_ERR_INVALID, "kmax, lambda must be positive; slice thickness and k_band non-negative");
   const size_t need = (size_t)p->group * (p->nx / p->col_ops->col_c) * num_detectors;
@@ -1094,6 +1102,7 @@ int msx_plan_probe_waves(msx_plan* p, const float* psi_k_dev, const float* posit
                          float* waves_out_dev, void* stream) {
   if (!p || num_probes < 0 || !psi_k_dev || !positions_dev || !waves_out_dev || !(kmax > 0))
     return fail(MSX_ERR_INVALID, "probe waves: bad arguments");
+  if (!aligned8({psi_k_dev, positions_dev, waves_out_dev})) return fail(MSX_ERR_INVALID, kAlign8);
   if (num_probes == 0) return MSX_OK;
   cudaStream_t st = (cudaStream_t)stream;
   ColArgs c{};
@@ -1109,8 +1118,7 @@ int msx_plan_probe_stack(msx_plan* p, const float* psi_k_dev, const double* norm
                          const float* positions_dev, int num_probes, float kmax, float* probes_out_dev, void* stream) {
   if (!p || num_probes < 0 || !psi_k_dev || !normalization_dev || !positions_dev || !probes_out_dev || !(kmax > 0))
     return fail(MSX_ERR_INVALID, "probe stack: bad arguments");
-  if (!aligned(psi_k_dev, 8) || !aligned(normalization_dev, 8) || !aligned(positions_dev, 8) ||
-      !aligned(probes_out_dev, 8))
+  if (!aligned8({psi_k_dev, normalization_dev, positions_dev, probes_out_dev}))
     return fail(MSX_ERR_INVALID, "probe stack: arrays must be 8-byte aligned");
   if (num_probes == 0) return MSX_OK;
   cudaStream_t st = (cudaStream_t)stream;
@@ -1126,6 +1134,7 @@ int msx_plan_probe_stack(msx_plan* p, const float* psi_k_dev, const double* norm
 int msx_plan_step_waves(msx_plan* p, float* waves_dev, int num_waves, const float* trans_dev, const float* ptab_dev,
                         void* stream) {
   if (!p || num_waves < 0 || !waves_dev || !trans_dev || !ptab_dev) return fail(MSX_ERR_INVALID, "step waves: bad arguments");
+  if (!aligned8({waves_dev, trans_dev, ptab_dev})) return fail(MSX_ERR_INVALID, kAlign8);
   if (num_waves == 0) return MSX_OK;
   cudaStream_t st = (cudaStream_t)stream;
   float2* w = reinterpret_cast<float2*>(waves_dev);
@@ -1144,6 +1153,7 @@ int msx_plan_cbed_waves(msx_plan* p, float* waves_dev, int num_waves, const doub
   if (!p || num_waves < 0 || !waves_dev || !normalization_dev || !cbed_out_dev || crop_y <= 0 || crop_x <= 0 ||
       crop_y > p->ny || crop_x > p->nx)
     return fail(MSX_ERR_INVALID, "cbed of waves: bad arguments");
+  if (!aligned8({waves_dev, normalization_dev})) return fail(MSX_ERR_INVALID, kAlign8);
   if (num_waves == 0) return MSX_OK;
   cudaStream_t st = (cudaStream_t)stream;
   if (!p->inv_n) {
@@ -1317,6 +1327,7 @@ int msx_plan_profile(msx_plan* p, const float* trans_dev, int num_slices, const 
   if (!p || !ms_out) return fail(MSX_ERR_INVALID, "null plan or output");
   if (iters <= 0 || num_slices <= 0 || num_probes <= 0 || !trans_dev || !psi_k_dev || !normalization_dev || !positions_dev)
     return fail(MSX_ERR_INVALID, "profile needs slices, probes, inputs and iters > 0");
+  if (!aligned8({trans_dev, psi_k_dev, positions_dev, normalization_dev})) return fail(MSX_ERR_INVALID, kAlign8);
   const int ny = p->ny, nx = p->nx;
   const int gn = num_probes < p->group ? num_probes : p->group;
   if (!workspace_holds(p, gn))
@@ -1377,6 +1388,7 @@ int msx_plan_autotune(msx_plan* p, const float* trans_dev, int num_slices, const
   if (!p) return fail(MSX_ERR_INVALID, "null plan");
   if (iters <= 0 || num_slices <= 0 || num_probes <= 0 || !trans_dev || !psi_k_dev || !normalization_dev || !positions_dev)
     return fail(MSX_ERR_INVALID, "autotune needs slices, probes, inputs and iters > 0");
+  if (!aligned8({trans_dev, psi_k_dev, positions_dev, normalization_dev})) return fail(MSX_ERR_INVALID, kAlign8);
   int rcp = ensure_ptab(p);
   if (rcp == MSX_OK) rcp = after_plan_stream(p, (cudaStream_t)stream);
   if (rcp != MSX_OK) return rcp;
@@ -1676,6 +1688,8 @@ int msx_batch_run(msx_batch* b, const msx_job* jobs, int njobs, void* stream) {
     if (j.num_probes > 0 && (!j.psi_k_dev || !j.normalization_dev || !j.positions_dev || !j.cbed_out_dev ||
                              (j.num_slices > 0 && !j.trans_dev)))
       return fail(MSX_ERR_INVALID, "job %d: null pointer", i);
+    if (j.num_probes > 0 && !aligned8({j.trans_dev, j.psi_k_dev, j.positions_dev, j.normalization_dev}))
+      return fail(MSX_ERR_INVALID, "job %d: %s", i, kAlign8);
     if (!(j.kmax > 0) || !(j.lambda > 0) || !(j.slice_t >= 0) || !(j.k_band >= 0))
       return fail(MSX_ERR_INVALID, "job %d: kmax, lambda must be positive", i);
   }
