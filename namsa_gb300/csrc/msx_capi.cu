@@ -986,6 +986,7 @@ int msx_plan_set_tma(msx_plan* p, int enable) {
 int msx_plan_check(msx_plan* p) {
   if (!p) return fail(MSX_ERR_INVALID, "null plan");
   int h = 0;
+  MSX_CUDA(cudaDeviceSynchronize(), "synchronising the device");  // a copy alone does not wait for non-blocking streams
   MSX_CUDA(cudaMemcpy(&h, p->err, sizeof(int), cudaMemcpyDeviceToHost), "reading the plan error word");
   if (h) {
     MSX_CUDA(cudaMemset(p->err, 0, sizeof(int)), "clearing the plan error word");

@@ -416,6 +416,8 @@ int msx_tc_check(void) {
   if (!s) return tfail(MSX_ERR_CUDA, "tensor-core DFT: no device");
   if (!s->err) return MSX_OK;
   int h = 0;
+  // a copy alone does not wait for non-blocking streams
+  if (cudaDeviceSynchronize() != cudaSuccess) return tfail(MSX_ERR_CUDA, "synchronising the device");
   if (cudaMemcpy(&h, s->err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
     return tfail(MSX_ERR_CUDA, "reading the tensor-core error word");
   if (h) {

@@ -1722,6 +1722,7 @@ int TcGemm::run_cplx(const float* a, Addr aa, long long a_bs, const float* src, 
 int TcGemm::check() {
   if (!err) return MSX_OK;
   int h = 0;
+  if (cudaDeviceSynchronize() != cudaSuccess) return MSX_ERR_CUDA;  // a copy alone does not wait for non-blocking streams
   if (cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return MSX_ERR_CUDA;
   if (h) {
     cudaMemset(err, 0, sizeof(int));
