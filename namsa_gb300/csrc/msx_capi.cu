@@ -211,6 +211,28 @@ int ensure_ptab(msx_plan* p) {
   return MSX_OK;
 }
 
+// The constant (1/N, 0) table, filled before the first call that reads it goes on: later
+// calls may come from any stream, and the first one may be under a capture.
+int ensure_inv_n(msx_plan* p) {
+  if (p->inv_n) return MSX_OK;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  MSX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+  float2* t = nullptr;
+  cudaError_t e = cudaMalloc(&t, sizeof(float2) * (size_t)p->ny * p->nx);
+  const bool allocated = e == cudaSuccess;
+  // P = 1 everywhere, k_band beyond every |k|: zero thickness gives (1/N, 0)
+  if (e == cudaSuccess) e = launch_ptab(p->ny, p->nx, 1.0f, 1.0, 0.0, 3.0e38f, t, p->work);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(p->work);
+  MSX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (t) cudaFree(t);
+    return allocated ? cuda_fail(e, "constant table") : fail(MSX_ERR_ALLOC, "constant table allocation failed");
+  }
+  p->inv_n = t;
+  return MSX_OK;
+}
+
 // The plan's small tables in one allocation: propagator factors, mask bands, the
 // error word, and the all-slices kernel's counters and twiddles.
 int create_tables(msx_plan* p) {
@@ -1157,12 +1179,8 @@ int msx_plan_cbed_waves(msx_plan* p, float* waves_dev, int num_waves, const doub
   if (!aligned8({waves_dev, normalization_dev})) return fail(MSX_ERR_INVALID, kAlign8);
   if (num_waves == 0) return MSX_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (!p->inv_n) {
-    if (cudaMalloc(&p->inv_n, sizeof(float2) * (size_t)p->ny * p->nx) != cudaSuccess)
-      return fail(MSX_ERR_ALLOC, "constant table allocation failed");
-    // P = 1 everywhere, k_band beyond every |k|: launch_ptab with zero thickness gives (1/N, 0)
-    MSX_CUDA(launch_ptab(p->ny, p->nx, 1.0f, 1.0, 0.0, 3.0e38f, p->inv_n, st), "constant table");
-  }
+  const int rc = ensure_inv_n(p);
+  if (rc != MSX_OK) return rc;
   float2* w = reinterpret_cast<float2*>(waves_dev);
   MSX_CUDA(p->row_ops->row_mode(ROW_F, w, nullptr, p->tw_row, num_waves, p->ny, st), "forward row transform");
   ColArgs c{};

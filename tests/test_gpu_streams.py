@@ -38,3 +38,36 @@ def test_detector_graph_free_and_recorded_calls_of_one_plan(n, S, P):
         assert torch.equal(a, want) and torch.equal(b, signals) and torch.equal(c, plain)
     plan.check()
     plan.close()
+
+
+def test_first_use_of_the_constant_table_from_two_streams():
+    """The table of cbed_waves is there before the first call goes on, whatever its stream waits
+    for; a first call under a capture has it too."""
+    torch.cuda.set_device(0)
+    n, P = 128, 2
+    g = torch.Generator(DEV).manual_seed(9)
+    waves = torch.view_as_complex(torch.randn((P, n, n, 2), generator=g, device=DEV))
+    norm = torch.tensor([float(n * n)], dtype=torch.float64, device=DEV)
+    want = torch.fft.fft2(waves.to(torch.complex128) / n).abs().square() * (1.0 / (n * n))
+    plan = engine.Plan(n, n)
+    a, b = waves.clone(), waves.clone()
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s1):
+        torch.cuda._sleep(100_000_000)
+        first = plan.cbed_waves(a, norm)
+    with torch.cuda.stream(s2):
+        second = plan.cbed_waves(b, norm)
+    torch.cuda.synchronize()
+    assert torch.equal(first, second) and float((first - want).norm() / want.norm()) < 1e-6
+    plan.close()
+    plan = engine.Plan(n, n)
+    c = waves.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = plan.cbed_waves(c, norm)
+    c.copy_(waves)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, first)
+    plan.close()
