@@ -246,6 +246,7 @@ __global__ void __launch_bounds__(384, MINB) stream_kernel(const __grid_constant
           if (!ok) atomicOr(a.err, 1);
         }
         if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+        __syncwarp();             // lane 0's acquire before what follows in the other lanes (a shuffle orders nothing)
         fence_proxy_async_all();  // in every lane that issues copies: the awaited data before its own copies
         float2* const dst = stage + s * STAGE;
         if (t.row) {
