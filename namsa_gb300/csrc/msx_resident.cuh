@@ -20,9 +20,15 @@
 // o and only after that has received the block sent from there, and it sends a
 // column block only after its last read of those columns.
 //
-// Waits are bounded as in msx_tma.cuh; when one runs out, bit 0 of *err is set,
-// later waits are skipped (the phases then see incomplete values) and the kernel
-// runs to its end.
+// Waits are bounded as in msx_tma.cuh.  When one runs out, bit 0 of *err is set, the CTA
+// ends its phase on incomplete values, waits for the next phase's blocks (bounded, as
+// ever) and stops there; the others then miss its blocks, time out and stop the
+// same way.  So a CTA leaves only after a wait, complete or a second long, that
+// followed every block sent to it, and after one for its own transmission rows: no
+// copy is in flight when the shared memory is released.  The flag is read
+// ahead of a wait, one word per kind of phase (a word is written in one phase and
+// read in the next, on the other side of a barrier), which costs nothing measurable; a barrier
+// with a reduction in either phase took 3 % of a slice at 256^2.
 #pragma once
 #include "msx_tma.cuh"
 
@@ -69,7 +75,7 @@ struct Resident {
            + (size_t)live * NX             // exchange lines of a row round
            + 2 * (size_t)NY * cols(w, cl) + TWR + TWC + NY;  // the row blocks, the columns, tables
   }
-  static __host__ size_t bytes(int w, int cl, int tbufs) { return sizeof(float2) * words(w, cl, tbufs) + 64; }
+  static __host__ size_t bytes(int w, int cl, int tbufs) { return sizeof(float2) * words(w, cl, tbufs) + 64; }  // + barriers, flags
   // two transmission buffers where they fit
   static __host__ int tbufs(int w, int cl) { return bytes(w, cl, 2) <= 232448 ? 2 : 1; }
   static __host__ size_t smem(int w, int cl) { return bytes(w, cl, tbufs(w, cl)); }
@@ -135,6 +141,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Res
   uint64_t* const tfull = reinterpret_cast<uint64_t*>(py + NY);  // one per transmission buffer
   uint64_t* const rfull = tfull + 2;
   uint64_t* const cfull = tfull + 3;
+  volatile int* const failed = reinterpret_cast<volatile int*>(tfull + 4);  // a wait ran out: in a row phase, in a column phase
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int mycols = min(wc, max(0, W - rank * wc));
   const uint32_t tbytes = (uint32_t)(rows * NX * sizeof(float2));
@@ -146,6 +153,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Res
   };
   if (tid == 0) {
     for (int i = 0; i < 4; ++i) mbar_init(&tfull[i], 1);
+    failed[0] = failed[1] = 0;
     fence_mbar_init();
     for (int s = 0; s < a.tbufs && s < a.slices; ++s) fetch(s);
   }
@@ -162,20 +170,25 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Res
   const uint32_t rbuf_s = smem_u32(rbuf), cbuf_s = smem_u32(cbuf);
   const uint32_t rfull_s = smem_u32(rfull), cfull_s = smem_u32(cfull);
   const uint32_t winv = (65536u + wc - 1) / wc;  // v / wc == (v winv) >> 16 for v < W <= 256 (checked on the host)
-  bool dead = false;
+  int stopped = -1;  // the slice in which the CTA stopped
 
   for (int s = 0; s < a.slices; ++s) {
     // ------------------------------------------------------------------ row phase
     const int tb = s % a.tbufs;
     const float2* const trow = tbuf + tb * rows * NX;
-    bool ok = dead || mbar_wait_bounded(&tfull[tb], (uint32_t)((s / a.tbufs) & 1));
-    if (s > 0 && !dead) {
+    const int failed_before = failed[1];
+    bool ok = mbar_wait_bounded(&tfull[tb], (uint32_t)((s / a.tbufs) & 1));
+    if (s > 0) {
       if (tid == 0) mbar_expect_tx(rfull, phase_bytes);  // the values may have been arriving before
-      ok = ok && wait_cluster(rfull, (uint32_t)((s - 1) & 1));
+      ok = wait_cluster(rfull, (uint32_t)((s - 1) & 1)) && ok;
     }
-    if (!__all_sync(0xffffffffu, ok)) {
-      dead = true;
-      if (lane == 0) atomicOr(a.err, 1);
+    if (!__all_sync(0xffffffffu, ok) && lane == 0) {
+      failed[0] = 1;
+      atomicOr(a.err, 1);
+    }
+    if (failed_before) {  // the same for every thread
+      stopped = s;
+      break;
     }
     {
       constexpr int T = LR::T, E = LR::E;
@@ -227,12 +240,15 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Res
     if (tid < cl)
       bulk_s2s(map_rank(cbuf_s + rank * bbytes, (uint32_t)tid), rbuf_s + tid * bbytes, bbytes, map_rank(cfull_s, (uint32_t)tid));
     // --------------------------------------------------------------- column phase
-    if (!dead) {
-      if (tid == 0) mbar_expect_tx(cfull, phase_bytes);
-      if (!__all_sync(0xffffffffu, wait_cluster(cfull, (uint32_t)(s & 1)) ? 1 : 0)) {
-        dead = true;
-        if (lane == 0) atomicOr(a.err, 1);
-      }
+    const int failed_rows = failed[0];
+    if (tid == 0) mbar_expect_tx(cfull, phase_bytes);
+    if (!__all_sync(0xffffffffu, wait_cluster(cfull, (uint32_t)(s & 1)) ? 1 : 0) && lane == 0) {
+      failed[1] = 1;
+      atomicOr(a.err, 1);
+    }
+    if (failed_rows) {
+      stopped = s;
+      break;
     }
     {
       constexpr int T = LC::T, E = LC::E, C = K::CPR;
@@ -310,8 +326,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Res
       }
     }
   }
-  if (dead && tid == 0)  // copies that had not landed in time land before the shared memory is released
-    for (int s = a.slices > a.tbufs ? a.slices - a.tbufs : 0; s < a.slices; ++s)
+  if (stopped >= 0 && tid == 0)  // rows asked for: those of the slices before stopped + tbufs
+    for (int s = stopped; s < stopped + a.tbufs && s < a.slices; ++s)
       mbar_wait_bounded(&tfull[s % a.tbufs], (uint32_t)((s / a.tbufs) & 1));
   cluster_sync_all();  // no CTA leaves while another may still write to it
 }
