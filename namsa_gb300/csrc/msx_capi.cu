@@ -133,11 +133,13 @@ struct msx_plan {
     const SchedOps* ops = nullptr;
     float2* tw = nullptr;        // in `tables`
     int ctas = 0;
+    FormState form;
   } few_row, few_col;
   CUtensorMap fmap{};            // the workspace with few_col's tile as box
   bool use_few = false;
   // all slices of a group in one kernel (msx_stream.cuh); off while schedules are set by hand
   const StreamOps* stream = nullptr;
+  FormState stream_form, resident_form;
   bool use_stream = false;       // may take `stream`
   bool use_resident = false;     // may take `resident`
   // a wave in the shared memory of a cluster (msx_resident.cuh), small grids
@@ -233,6 +235,25 @@ int ensure_inv_n(msx_plan* p) {
   return MSX_OK;
 }
 
+// Whether the device takes the plan's optional forms; where it refuses one (no room for
+// its CTAs, its clusters or its registers) the two passes with the plan's schedules run.
+bool stream_ready(msx_plan* p) {
+  return p->stream && p->stream_form.ready([&] { return p->stream->configure(); });
+}
+bool resident_ready(msx_plan* p) {
+  return p->resident && p->resident_form.ready([&] { return p->resident->configure(); });
+}
+bool few_ready(msx_plan* p, msx_plan::FewPass& f) {
+  return f.ops && f.form.ready([&] {
+    cudaError_t e = f.ops->configure();
+    int sms = 0, rows = 0, cols = 0;
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    if (e == cudaSuccess) e = f.ops->occupancy(&rows, &cols);
+    f.ctas = sms * (&f == &p->few_row ? rows : cols);
+    return e == cudaSuccess && f.ctas < 1 ? cudaErrorInvalidConfiguration : e;
+  });
+}
+
 // The plan's small tables in one allocation: propagator factors, mask bands, the
 // error word, and the all-slices kernel's counters and twiddles.
 int create_tables(msx_plan* p) {
@@ -273,12 +294,10 @@ int create_tables(msx_plan* p) {
     p->counters = reinterpret_cast<int*>(base + counters);
     p->stw_row = reinterpret_cast<float2*>(base + srow);
     p->stw_col = reinterpret_cast<float2*>(base + scol);
-    MSX_CUDA(p->stream->configure(), "configuring the all-slices kernel");
   }
   if (p->resident) {
     p->rtw_row = reinterpret_cast<float2*>(base + rrow);
     p->rtw_col = reinterpret_cast<float2*>(base + rcol);
-    MSX_CUDA(p->resident->configure(), "configuring the cluster-resident kernel");
   }
   p->few_row.tw = reinterpret_cast<float2*>(base + frow);
   p->few_col.tw = reinterpret_cast<float2*>(base + fcol);
@@ -346,13 +365,6 @@ int prepare_tma(msx_plan* p) {
   MSX_CUDA(p->row_ops->occupancy(&rr, &dummy), "occupancy");
   MSX_CUDA(p->col_ops->occupancy(&dummy, &cr), "occupancy");
   if (rr < 1 || cr < 1) return fail(MSX_ERR_CUDA, "persistent passes do not fit on an SM");
-  for (msx_plan::FewPass* f : {&p->few_row, &p->few_col})
-    if (f->ops) {
-      int fr = 0, fc = 0;
-      MSX_CUDA(f->ops->occupancy(&fr, &fc), "occupancy");
-      f->ctas = sms * (f == &p->few_row ? fr : fc);
-      if (f->ctas < 1) return fail(MSX_ERR_CUDA, "persistent passes do not fit on an SM");
-    }
   p->sms = sms;
   p->row_ctas = sms * rr;
   p->col_ctas = sms * cr;
@@ -471,15 +483,15 @@ void band_columns(int nx, float kmax, float k_band, int C, int* x_lo, int* x_hi)
 //           384 x 384   P 1 19.5/18.2  8 20.2/18.9  12 21.6/21.8
 //           768 x 64    P 1 16.1/14.1 24 18.5/16.6  32 19.5/20.9
 //           768 x 256   P 1 16.5/14.3  4 16.7/14.5   8 17.4/19.0
-bool few_rows(const msx_plan* p, int gn) {
+bool few_rows(msx_plan* p, int gn) {
   if (!p->use_few || !p->few_row.ops) return false;
   const int tiles = (gn + p->few_row.ops->row_lines - 1) / p->few_row.ops->row_lines;
-  return tiles * p->ny <= p->sms || (p->nx == 768 && tiles == 1);
+  return (tiles * p->ny <= p->sms || (p->nx == 768 && tiles == 1)) && few_ready(p, p->few_row);
 }
-bool few_cols(const msx_plan* p, int gn, float kmax, float k_band, int* x_lo, int* x_hi) {
+bool few_cols(msx_plan* p, int gn, float kmax, float k_band, int* x_lo, int* x_hi) {
   if (p->use_few && p->few_col.ops) {
     band_columns(p->nx, kmax, k_band, p->few_col.ops->col_c, x_lo, x_hi);
-    if ((*x_hi - *x_lo) / p->few_col.ops->col_c * gn <= p->sms) return true;
+    if ((*x_hi - *x_lo) / p->few_col.ops->col_c * gn <= p->sms && few_ready(p, p->few_col)) return true;
   }
   band_columns(p->nx, kmax, k_band, p->col_ops->col_c, x_lo, x_hi);
   return false;
@@ -568,7 +580,7 @@ constexpr StreamRange kStreamRange[4][4] = {  // [ny][nx], lines of 256, 384, 51
     {{24, 36}, {16, 400}, {12, 130}, {12, 300}},
     {{8, 60}, {1, 500}, {1, 360}, {1, 500}},
     {{8, 36}, {1, 300}, {1, 380}, {1, 310}}};
-int stream_group(const msx_plan* p, const MsArgs& a) {
+int stream_group(msx_plan* p, const MsArgs& a) {
   if (!p->use_stream || !p->stream || !p->use_tma || !p->map_ok || a.num_slices < 2 || a.num_probes < 1 ||
       !aligned(a.trans, 16))
     return 0;
@@ -585,7 +597,7 @@ int stream_group(const msx_plan* p, const MsArgs& a) {
   const int groups = (int)((a.num_probes + most - 1) / most);
   int g = ((a.num_probes + groups - 1) / groups + unit - 1) / unit * unit;
   if (g > a.num_probes) g = a.num_probes;
-  return g <= a.group ? g : 0;
+  return g <= a.group && stream_ready(p) ? g : 0;
 }
 
 // Whether a call keeps each wave in a cluster, and the CTAs of a cluster: as many as
@@ -600,7 +612,7 @@ int stream_group(const msx_plan* p, const MsArgs& a) {
 constexpr int kResidentSizes[3] = {16, 8, 4};
 int resident_cluster(msx_plan* p, const MsArgs& a) {
   if (!p->use_resident || !p->resident || !p->use_tma || !p->map_ok || a.det || a.num_slices < 2 || a.num_probes < 1 ||
-      a.num_probes > a.group || !aligned(a.trans, 16))
+      a.num_probes > a.group || !aligned(a.trans, 16) || !resident_ready(p))
     return 0;
   int lo = 0, hi = 0;
   band_columns(p->nx, a.kmax, a.k_band, 1, &lo, &hi);
@@ -904,18 +916,17 @@ int msx_plan_create(int ny, int nx, int group, msx_plan** out) {
   schedule_table(nx, &rops);
   schedule_table(ny, &cops);
   const int fr = few_row_schedule(nx), fc = few_col_schedule(ny);
-  if (fr >= 0) {
-    p->few_row.ops = &rops[fr];
-    rc = ensure_configured(device, nx, fr, rops[fr]);
-  }
-  if (rc == MSX_OK && fc >= 0) {
-    p->few_col.ops = &cops[fc];
-    rc = ensure_configured(device, ny, fc, cops[fc]);
-  }
-  if (rc == MSX_OK)
-    rc = msx_plan_set_schedule(p, default_row_schedule(nx), default_col_schedule(ny),
-                               group > 0 ? group : auto_group(ny, nx));
+  if (fr >= 0) p->few_row.ops = &rops[fr];
+  if (fc >= 0) p->few_col.ops = &cops[fc];
+  rc = msx_plan_set_schedule(p, default_row_schedule(nx), default_col_schedule(ny),
+                             group > 0 ? group : auto_group(ny, nx));
   if (rc == MSX_OK) rc = create_tables(p);
+  if (rc == MSX_OK) {
+    stream_ready(p);
+    resident_ready(p);
+    few_ready(p, p->few_row);
+    few_ready(p, p->few_col);
+  }
   if (rc == MSX_OK) {
     cudaError_t e = cudaStreamCreateWithFlags(&p->work, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->ev_in, cudaEventDisableTiming);

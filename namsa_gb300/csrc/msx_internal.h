@@ -4,6 +4,7 @@
 
 #include <map>
 
+#include "msx_form.h"
 #include "msx_sched.cuh"
 #include "msx_resident.cuh"
 #include "msx_stream.cuh"

@@ -443,10 +443,18 @@ struct StreamImpl {
     }
     // the registers the roles take must be there at launch, or setmaxnreg waits for good
     cudaFuncAttributes fa{};
-    const cudaError_t e = cudaFuncGetAttributes(&fa, stream_kernel<LR, LC, MINB>);
+    cudaError_t e = cudaFuncGetAttributes(&fa, stream_kernel<LR, LC, MINB>);
     if (e != cudaSuccess) return e;
     if (fa.numRegs * K::THREADS < (MINB == 2 ? 256 * 104 + 128 * 32 : 256 * 232 + 128 * 40)) return cudaErrorInvalidConfiguration;
-    return cudaFuncSetAttribute(stream_kernel<LR, LC, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::smem());
+    e = cudaFuncSetAttribute(stream_kernel<LR, LC, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::smem());
+    if (e != cudaSuccess) return e;
+    // every CTA of a launch resident, MINB to an SM
+    int dev = 0, cooperative = 0, ctas = 0;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, stream_kernel<LR, LC, MINB>, K::THREADS, K::smem());
+    return e == cudaSuccess && (!cooperative || ctas < MINB) ? cudaErrorInvalidConfiguration : e;
   }
   static cudaError_t launch(const CUtensorMap& map, const StreamArgs& a, int sms, cudaStream_t st) {
     const long long tasks = a.sh.tasks();
