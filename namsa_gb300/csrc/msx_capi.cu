@@ -139,7 +139,7 @@ struct msx_plan {
   bool use_few = false;
   // all slices of a group in one kernel (msx_stream.cuh); off while schedules are set by hand
   const StreamOps* stream = nullptr;
-  FormState stream_form, resident_form;
+  FormState stream_form, resident_form;  // asked by the first call that would take the form
   bool use_stream = false;       // may take `stream`
   bool use_resident = false;     // may take `resident`
   // a wave in the shared memory of a cluster (msx_resident.cuh), small grids
@@ -235,23 +235,38 @@ int ensure_inv_n(msx_plan* p) {
   return MSX_OK;
 }
 
+// Asks the device, also under a stream capture.
+template <class F>
+cudaError_t ask_device(F ask) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return e;
+  const cudaError_t asked = ask();
+  e = cudaThreadExchangeStreamCaptureMode(&mode);
+  return asked != cudaSuccess ? asked : e;
+}
+
 // Whether the device takes the plan's optional forms; where it refuses one (no room for
 // its CTAs, its clusters or its registers) the two passes with the plan's schedules run.
+// Asked by the first call whose rules choose the form: the answer loads the form's
+// module, and many plans never come to it (first plan of a process: 256^2 2.8 ms
+// configuring every form at once, 2.3 so; 512^2 2.6, 2.2; 384 x 768 2.9, 2.3).
 bool stream_ready(msx_plan* p) {
-  return p->stream && p->stream_form.ready([&] { return p->stream->configure(); });
+  return p->stream && p->stream_form.ready([&] { return ask_device([&] { return p->stream->configure(); }); });
 }
 bool resident_ready(msx_plan* p) {
-  return p->resident && p->resident_form.ready([&] { return p->resident->configure(); });
+  return p->resident && p->resident_form.ready([&] { return ask_device([&] { return p->resident->configure(); }); });
 }
 bool few_ready(msx_plan* p, msx_plan::FewPass& f) {
-  return f.ops && f.form.ready([&] {
+  auto configure = [&] {
     cudaError_t e = f.ops->configure();
     int sms = 0, rows = 0, cols = 0;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
     if (e == cudaSuccess) e = f.ops->occupancy(&rows, &cols);
     f.ctas = sms * (&f == &p->few_row ? rows : cols);
     return e == cudaSuccess && f.ctas < 1 ? cudaErrorInvalidConfiguration : e;
-  });
+  };
+  return f.ops && f.form.ready([&] { return ask_device(configure); });
 }
 
 // The plan's small tables in one allocation: propagator factors, mask bands, the
@@ -612,25 +627,34 @@ int stream_group(msx_plan* p, const MsArgs& a) {
 constexpr int kResidentSizes[3] = {16, 8, 4};
 int resident_cluster(msx_plan* p, const MsArgs& a) {
   if (!p->use_resident || !p->resident || !p->use_tma || !p->map_ok || a.det || a.num_slices < 2 || a.num_probes < 1 ||
-      a.num_probes > a.group || !aligned(a.trans, 16) || !resident_ready(p))
+      a.num_probes > a.group || !aligned(a.trans, 16))
     return 0;
   int lo = 0, hi = 0;
   band_columns(p->nx, a.kmax, a.k_band, 1, &lo, &hi);
-  if (p->rclusters_w != hi - lo) {
-    for (int i = 0; i < 3; ++i)
-      if (p->resident->clusters(hi - lo, kResidentSizes[i], &p->rclusters[i]) != cudaSuccess) {
-        cudaGetLastError();
-        p->rclusters[i] = 0;
-      }
-    p->rclusters_w = hi - lo;
-  }
+  const int w = hi - lo;
+  // whether all positions run in `rounds` rounds of clusters of kResidentSizes[i]; the
+  // device is asked where the shared memory alone does not rule it out
+  auto fits = [&](int i, int rounds) -> bool {
+    const int cl = kResidentSizes[i];
+    if (a.num_probes > rounds * p->resident->most(w, cl, p->sms) || !resident_ready(p)) return false;
+    if (p->rclusters_w != w) {
+      for (int& n : p->rclusters) n = -1;
+      p->rclusters_w = w;
+    }
+    int& n = p->rclusters[i];
+    if (n < 0 && ask_device([&] { return p->resident->clusters(w, cl, &n); }) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+    return a.num_probes <= rounds * n;
+  };
   const int area = p->ny * p->nx;
-  if (area > 128 * 128 && a.num_probes <= p->rclusters[0]) return kResidentSizes[0];
+  if (area > 128 * 128 && fits(0, 1)) return kResidentSizes[0];
   if (area >= 256 * 256) return 0;
-  if (a.num_probes <= p->rclusters[1]) return kResidentSizes[1];
+  if (fits(1, 1)) return kResidentSizes[1];
   if (p->nx > p->ny && area > 128 * 128 && a.num_probes < 24) return 0;  // 128 x 256: P 16 9.0 / 9.7, 24 9.8 / 9.7
   const int rounds = area <= 128 * 128 && p->nx <= 128 ? 2 : 1;  // 64 x 256: P 64 10.9 / 11.1 in two
-  if (a.num_probes <= rounds * p->rclusters[2]) return kResidentSizes[2];
+  if (fits(2, rounds)) return kResidentSizes[2];
   return 0;
 }
 
@@ -921,12 +945,6 @@ int msx_plan_create(int ny, int nx, int group, msx_plan** out) {
   rc = msx_plan_set_schedule(p, default_row_schedule(nx), default_col_schedule(ny),
                              group > 0 ? group : auto_group(ny, nx));
   if (rc == MSX_OK) rc = create_tables(p);
-  if (rc == MSX_OK) {
-    stream_ready(p);
-    resident_ready(p);
-    few_ready(p, p->few_row);
-    few_ready(p, p->few_col);
-  }
   if (rc == MSX_OK) {
     cudaError_t e = cudaStreamCreateWithFlags(&p->work, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->ev_in, cudaEventDisableTiming);

@@ -25,6 +25,11 @@ struct ResidentImpl {
       e = cudaFuncSetAttribute(resident_kernel<LR, LC>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
   }
+  static int most(int w, int cl, int sms) {
+    if (K::smem(w, cl) > 232448 || cl > K::NY) return 0;
+    const size_t by_smem = 233472 / (K::smem(w, cl) + 1024), by_threads = 2048 / kResidentThreads;
+    return (int)(by_smem < by_threads ? by_smem : by_threads) * sms / cl;
+  }
   static cudaError_t clusters(int w, int cl, int* n) {
     *n = 0;
     if (K::smem(w, cl) > 232448 || cl > K::NY) return cudaSuccess;
@@ -40,7 +45,7 @@ struct ResidentImpl {
   }
   static ResidentOps ops() {
     return ResidentOps{LR::FFT::tw_words(), LC::FFT::tw_words(), &LR::FFT::host_twiddles, &LC::FFT::host_twiddles,
-                       &configure, &clusters, &launch};
+                       &configure, &most, &clusters, &launch};
   }
 };
 

@@ -337,6 +337,8 @@ struct ResidentOps {
   void (*tw_row)(float2*);
   void (*tw_col)(float2*);
   cudaError_t (*configure)();
+  // no more clusters of `cl` CTAs than this run at the same time, by shared memory and threads alone
+  int (*most)(int w, int cl, int sms);
   // clusters of `cl` CTAs that run at the same time with `w` band columns (0: does not fit)
   cudaError_t (*clusters)(int w, int cl, int* n);
   cudaError_t (*launch)(ResidentArgs a, int waves, int cl, cudaStream_t st);
