@@ -161,6 +161,19 @@ MSX_API int msx_plan_set_schedule(msx_plan* plan, int row_schedule, int col_sche
 /* Reports the current row/column schedule indices and group size. */
 MSX_API int msx_plan_get_schedule(const msx_plan* plan, int* row_schedule, int* col_schedule, int* group);
 
+/*
+ * How a call with these sizes (slices and complex inputs 16-byte aligned) would
+ * run its slices: *form is one of MSX_FORM_*, *size the waves of its first group
+ * (clusters: the CTAs of a cluster), and *few tells whether the first group's
+ * passes take the schedules for few lines (1 rows, 2 columns, 3 both).
+ * `detector` 1 asks for msx_multislice_detect.  The outputs may be NULL.
+ */
+#define MSX_FORM_PASSES 0
+#define MSX_FORM_ALL_SLICES 1
+#define MSX_FORM_CLUSTER 2
+MSX_API int msx_plan_route(msx_plan* plan, int num_slices, int num_probes, float kmax, float k_band, int detector,
+                           int* form, int* size, int* few);
+
 /* 1 = run the per-slice passes as persistent, TMA-pipelined kernels (default);
  * 0 = one CTA per tile, plain loads.  Both give the same results. */
 MSX_API int msx_plan_set_tma(msx_plan* plan, int enable);

@@ -40,6 +40,7 @@ SIGNATURES = [
     ('msx_plan_destroy', _c.c_int, [_vp]),
     ('msx_plan_set_schedule', _c.c_int, [_vp, _c.c_int, _c.c_int, _c.c_int]),
     ('msx_plan_get_schedule', _c.c_int, [_vp, _c.POINTER(_c.c_int), _c.POINTER(_c.c_int), _c.POINTER(_c.c_int)]),
+    ('msx_plan_route', _c.c_int, [_vp, _c.c_int, _c.c_int, _c.c_float, _c.c_float, _c.c_int] + [_c.POINTER(_c.c_int)] * 3),
     ('msx_plan_set_graph', _c.c_int, [_vp, _c.c_int]),
     ('msx_plan_set_tma', _c.c_int, [_vp, _c.c_int]),
     ('msx_plan_check', _c.c_int, [_vp]),

@@ -1027,6 +1027,29 @@ int msx_plan_get_schedule(const msx_plan* p, int* row_schedule, int* col_schedul
   return MSX_OK;
 }
 
+int msx_plan_route(msx_plan* p, int num_slices, int num_probes, float kmax, float k_band, int detector, int* form,
+                   int* size, int* few) {
+  if (!p) return fail(MSX_ERR_INVALID, "null plan");
+  if (num_slices < 0 || num_probes < 1 || !(kmax > 0) || !(k_band >= 0))
+    return fail(MSX_ERR_INVALID, "route: needs probes, kmax > 0, non-negative slices and k_band");
+  MsArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.num_slices = num_slices; a.num_probes = num_probes; a.kmax = kmax; a.k_band = k_band; a.group = p->group;
+  const float any = 0.f;
+  a.det = detector ? &any : nullptr;
+  const int cluster = resident_cluster(p, a), streamed = cluster ? 0 : stream_group(p, a);
+  const int waves = num_probes < p->group ? num_probes : p->group;
+  int lo = 0, hi = 0;
+  if (form) *form = cluster ? MSX_FORM_CLUSTER : streamed ? MSX_FORM_ALL_SLICES : MSX_FORM_PASSES;
+  if (size) *size = cluster ? cluster : streamed ? streamed : waves;
+  if (few) {
+    *few = 0;
+    if (!cluster && !streamed && num_slices > 0 && p->use_tma && p->map_ok)
+      *few = (few_rows(p, waves) ? 1 : 0) + (few_cols(p, waves, kmax, k_band, &lo, &hi) ? 2 : 0);
+  }
+  return MSX_OK;
+}
+
 int msx_plan_set_tma(msx_plan* p, int enable) {
   if (!p) return fail(MSX_ERR_INVALID, "null plan");
   p->use_tma = enable != 0;

@@ -275,6 +275,15 @@ class Plan:
         _lib.check(lib().msx_plan_get_schedule(self.handle, ctypes.byref(r), ctypes.byref(c), ctypes.byref(g)))
         return r.value, c.value, g.value
 
+    def route(self, num_slices, num_probes, kmax, k_band, detector=False):
+        """How a call of these sizes runs its slices: ('passes', waves of a group), ('all_slices',
+        waves of a group) or ('cluster', CTAs of a cluster), and whether the row and the column
+        pass take the schedules for few lines."""
+        form, size, few = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+        _lib.check(lib().msx_plan_route(self.handle, int(num_slices), int(num_probes), float(kmax), float(k_band),
+                                        int(bool(detector)), ctypes.byref(form), ctypes.byref(size), ctypes.byref(few)))
+        return ('passes', 'all_slices', 'cluster')[form.value], size.value, bool(few.value & 1), bool(few.value & 2)
+
     def set_graph(self, enable):
         _lib.check(lib().msx_plan_set_graph(self.handle, int(bool(enable))))
 
