@@ -486,9 +486,11 @@ MSX_API int msx_corrector_residual(const float* psi_dev, const float* target_dev
  * plan's grid on the given inputs -- `iters` slices of row + column passes
  * per candidate, CUDA events on `stream` -- and keeps the fastest.  Group
  * sizes range over resident sets of 8 MiB to 1 GiB of waves (capped by
- * num_probes and max_workspace_bytes, 0 = 1 GiB).  Where the one-kernel form
- * of all slices exists for the grid it is timed against them, and the plan
- * keeps whichever is faster.  Writes the best time per
+ * num_probes and max_workspace_bytes, 0 = 1 GiB).  Where the plan would run
+ * these inputs in the one-kernel form of all slices, that is timed against them,
+ * and the plan keeps whichever is faster.  The other forms stay as they were:
+ * small calls take clusters and, unless these inputs are themselves of few lines,
+ * the schedules for few lines.  Writes the best time per
  * wave and slice (ns) to *best_ns_per_wave_slice when non-NULL.  Synchronises
  * `stream`.  No counterpart in the reference (its batch size comes from a
  * free-memory heuristic, namsa/msa.py:445-461).

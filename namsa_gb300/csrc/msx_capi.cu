@@ -612,7 +612,7 @@ int stream_group(msx_plan* p, const MsArgs& a) {
   const int groups = (int)((a.num_probes + most - 1) / most);
   int g = ((a.num_probes + groups - 1) / groups + unit - 1) / unit * unit;
   if (g > a.num_probes) g = a.num_probes;
-  return g <= a.group && stream_ready(p) ? g : 0;
+  return workspace_holds(p, g) && stream_ready(p) ? g : 0;
 }
 
 // Whether a call keeps each wave in a cluster, and the CTAs of a cluster: as many as
@@ -627,7 +627,7 @@ int stream_group(msx_plan* p, const MsArgs& a) {
 constexpr int kResidentSizes[3] = {16, 8, 4};
 int resident_cluster(msx_plan* p, const MsArgs& a) {
   if (!p->use_resident || !p->resident || !p->use_tma || !p->map_ok || a.det || a.num_slices < 2 || a.num_probes < 1 ||
-      a.num_probes > a.group || !aligned(a.trans, 16))
+      !workspace_holds(p, a.num_probes) || !aligned(a.trans, 16))
     return 0;
   int lo = 0, hi = 0;
   band_columns(p->nx, a.kmax, a.k_band, 1, &lo, &hi);
@@ -1144,7 +1144,14 @@ int msx_multislice_detect(msx_plan* p, const float* trans_dev, int num_slices, c
   if (!aligned8({trans_dev, psi_k_dev, positions_dev, normalization_dev})) return fail(MSX_ERR_INVALID, kAlign8);
   if (!(kmax > 0) || !(lambda > 0) || !(slice_t >= 0) || !(k_band >= 0))
     return fail(MSX_ERR_INVALID, "kmax, lambda must be positive; slice thickness and k_band non-negative");
-  const size_t need = (size_t)p->group * (p->nx / p->col_ops->col_c) * num_detectors;
+  MsArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.trans = trans_dev; a.num_slices = num_slices; a.psik = psi_k_dev; a.norm = normalization_dev;
+  a.pos = positions_dev; a.num_probes = num_probes; a.kmax = kmax; a.lambda = lambda; a.slice_t = slice_t;
+  a.k_band = k_band; a.crop_y = p->ny; a.crop_x = p->nx; a.group = p->group; a.row_sched = p->row_sched;
+  a.col_sched = p->col_sched; a.det = detectors_dev; a.ndet = num_detectors; a.signals = signals_out_dev;
+  const int waves = std::max(p->group, stream_group(p, a));  // of a group, whichever form runs
+  const size_t need = (size_t)waves * (p->nx / p->col_ops->col_c) * num_detectors;
   if (need > p->partial_words) {
     if (p->partial) cudaFree(p->partial);
     p->partial = nullptr;
@@ -1153,12 +1160,6 @@ int msx_multislice_detect(msx_plan* p, const float* trans_dev, int num_slices, c
       return fail(MSX_ERR_ALLOC, "detector partial sums allocation failed");
     p->partial_words = need;
   }
-  MsArgs a;
-  std::memset(&a, 0, sizeof(a));
-  a.trans = trans_dev; a.num_slices = num_slices; a.psik = psi_k_dev; a.norm = normalization_dev;
-  a.pos = positions_dev; a.num_probes = num_probes; a.kmax = kmax; a.lambda = lambda; a.slice_t = slice_t;
-  a.k_band = k_band; a.crop_y = p->ny; a.crop_x = p->nx; a.group = p->group; a.row_sched = p->row_sched;
-  a.col_sched = p->col_sched; a.det = detectors_dev; a.ndet = num_detectors; a.signals = signals_out_dev;
   drop_graph(p);  // the detector sequence is launched directly
   return on_plan_stream(p, (cudaStream_t)stream,
                         [&](cudaStream_t st, bool) -> int { return enqueue_multislice(p, a, st); });
@@ -1571,6 +1572,11 @@ int msx_plan_autotune(msx_plan* p, const float* trans_dev, int num_slices, const
         return MSX_OK;
       }();
     }
+    // the winners stand for groups of bg waves: calls of few lines keep their schedules
+    // unless the timing was of few lines itself
+    int lo = 0, hi = 0;
+    p->use_few = true;
+    if (few_rows(p, bg) || few_cols(p, bg, kmax, k_band, &lo, &hi)) p->use_few = false;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -1603,20 +1609,29 @@ struct msx_batch {
 
 namespace {
 
-// Forms besides the two passes that a plan with given schedules may take: 1 the all-slices kernel, 2 clusters.
+// Forms besides the two passes with the given schedules that a plan may take: 1 the
+// all-slices kernel, 2 clusters, 4 the schedules of few lines.
 void allow_forms(msx_plan* p, int forms) {
   p->use_stream = (forms & 1) != 0;
   p->use_resident = (forms & 2) != 0;
+  p->use_few = (forms & 4) != 0;
+}
+int allowed_forms(const msx_plan* p) {
+  return (p->use_stream ? 1 : 0) + (p->use_resident ? 2 : 0) + (p->use_few ? 4 : 0);
+}
+
+// Persistent passes amortise their start-up over large groups: up to 1 GiB of
+// waves per branch (the jobs of a branch run one after another).
+int batch_waves(int ny, int nx) {
+  const int g = (int)(((size_t)1 << 30) / (sizeof(float2) * (size_t)ny * nx));
+  return g < 2 ? 2 : g;
 }
 
 msx_plan* batch_plan(msx_batch* b, int branch, int ny, int nx, int* rc) {
   const long long key = ((long long)ny << 32) | (unsigned)nx;
   for (auto& kv : b->plans[branch])
     if (kv.first == key) return kv.second;
-  // Persistent passes amortise their start-up over large groups: up to 1 GiB
-  // of waves per branch (the jobs of a branch run one after another).
-  int group = (int)(((size_t)1 << 30) / (sizeof(float2) * (size_t)ny * nx));
-  if (group < 2) group = 2;
+  int group = batch_waves(ny, nx), waves = group;
   int r = 0, c = 0;
   bool tuned = false;  // schedules set for this grid (else the plan's defaults)
   int forms = 0;
@@ -1624,9 +1639,11 @@ msx_plan* batch_plan(msx_batch* b, int branch, int ny, int nx, int* rc) {
     if (kv.first == key) {
       r = kv.second[0]; c = kv.second[1]; tuned = true; forms = kv.second[3];
       if (kv.second[2] > 0) group = kv.second[2];
+      // forms that choose their own groups need the room that the tuned plan had
+      if (!(forms & 3) || waves < group) waves = group;
     }
   msx_plan* p = nullptr;
-  *rc = msx_plan_create(ny, nx, group, &p);
+  *rc = msx_plan_create(ny, nx, waves, &p);
   if (*rc != MSX_OK) return nullptr;
   if (tuned) {
     *rc = msx_plan_set_schedule(p, r, c, group);
@@ -1651,9 +1668,14 @@ int batch_set_schedule(msx_batch* b, int ny, int nx, int row_schedule, int col_s
   for (auto& br : b->plans)
     for (auto& kv : br)
       if (kv.first == key) {
-        const int rc = msx_plan_set_schedule(kv.second, row_schedule, col_schedule, group);
+        int rc = msx_plan_set_schedule(kv.second, row_schedule, col_schedule, group);
         if (rc != MSX_OK) return rc;
         allow_forms(kv.second, forms);
+        if (forms & 3) {
+          rc = ensure_workspace(kv.second, (size_t)batch_waves(ny, nx));
+          if (rc == MSX_OK) rc = prepare_tma(kv.second);
+          if (rc != MSX_OK) return rc;
+        }
       }
   if (b->gexec) cudaGraphExecDestroy(b->gexec);
   b->gexec = nullptr;
@@ -1735,7 +1757,7 @@ int msx_batch_autotune(msx_batch* b, const msx_job* jobs, int njobs, int iters, 
                            stream);
     int row = 0, col = 0, group = 0;
     if (rc == MSX_OK) rc = msx_plan_get_schedule(p, &row, &col, &group);
-    const int forms = rc == MSX_OK ? (p->use_stream ? 1 : 0) + (p->use_resident ? 2 : 0) : 0;
+    const int forms = rc == MSX_OK ? allowed_forms(p) : 0;
     msx_plan_destroy(p);
     if (rc == MSX_OK) rc = batch_set_schedule(b, j.ny, j.nx, row, col, group, forms);
     if (rc != MSX_OK) return rc;
