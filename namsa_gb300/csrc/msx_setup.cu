@@ -87,7 +87,7 @@ __device__ double window_row(const double* c, int i, int j, int a, int os, doubl
   return accr / os;
 }
 
-// Grid: (species, blocks of bins of the quadrant).  `rows` threads share a bin
+// Grid: blocks of bins of the quadrant, species after species.  `rows` threads share a bin
 // (the oversampled rows a, a + rows, ...); slot 0 is the corner bin, slots
 // 1 .. bins are the block's own.  numpy's order: mean over the last axis, then
 // over the second-to-last.
@@ -98,10 +98,12 @@ atom_window_kernel(const double* __restrict__ coeff, int n0, int n1, int os, int
   __shared__ double val[kWinThreads];
   const int h0 = n0 / os, h1 = n1 / os;
   const int q1 = (h1 + 1) / 2, quad = ((h0 + 1) / 2) * q1;
-  const double* c = coeff + 12 * blockIdx.x;
+  const int blocks = (quad + bins - 1) / bins;  // of a species
+  const int species = blockIdx.x / blocks, block = blockIdx.x - species * blocks;
+  const double* c = coeff + 12 * species;
   const double start = -range / 2, sx = range / (double)(n0 - 1), sy = range / (double)(n1 - 1);
   const int slot = threadIdx.x / rows, a0 = threadIdx.x % rows;
-  const int bin = slot == 0 ? 0 : blockIdx.y * bins + slot - 1;  // bin 0 is the corner
+  const int bin = slot == 0 ? 0 : block * bins + slot - 1;  // bin 0 is the corner
   const bool live = slot <= bins && bin < quad;
   double acc = 0;
   for (int base = 0; base < os; base += rows) {
@@ -120,7 +122,7 @@ atom_window_kernel(const double* __restrict__ coeff, int n0, int n1, int os, int
   if (live && slot > 0 && a0 == 0) {
     const float v = (float)(val[slot] - val[0]);
     const int i = bin / q1, j = bin % q1;
-    float* o = out + (size_t)blockIdx.x * h0 * h1;
+    float* o = out + (size_t)species * h0 * h1;
     o[(size_t)i * h1 + j] = v;
     o[(size_t)(h0 - 1 - i) * h1 + j] = v;
     o[(size_t)i * h1 + h1 - 1 - j] = v;
@@ -463,8 +465,9 @@ cudaError_t launch_atom_windows(const double* coeff, int nspecies, int n0, int n
   const int rows = os < kWinThreads / 2 ? os : kWinThreads / 2;  // threads per bin
   const int bins = kWinThreads / rows - 1;                       // a block's own bins; one slot is the corner
   const int quad = ((n0 / os + 1) / 2) * ((n1 / os + 1) / 2);
-  const dim3 grid(nspecies, (quad + bins - 1) / bins);
-  atom_window_kernel<<<grid, kWinThreads, 0, st>>>(coeff, n0, n1, os, rows, bins, range, out);
+  const long long grid = (long long)nspecies * ((quad + bins - 1) / bins);
+  if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  atom_window_kernel<<<(unsigned)grid, kWinThreads, 0, st>>>(coeff, n0, n1, os, rows, bins, range, out);
   return cudaGetLastError();
 }
 
