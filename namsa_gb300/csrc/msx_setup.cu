@@ -1,6 +1,7 @@
 // Device kernels that prepare the multislice inputs: Kirkland atom windows,
 // the transmission slices exp(i sigma V), the k-space probe and its
 // normalisation, and the propagator table.
+#include "msx_bessel.cuh"
 #include "msx_internal.h"
 
 #include <cooperative_groups.h>
@@ -10,41 +11,7 @@
 
 namespace msx {
 
-// ------------------------------------------------------------------ Bessel K0
-// K0(x) = int_0^inf exp(-x cosh u) du (x > 0).  The integrand is analytic and
-// decays double-exponentially in the strip |Im u| < pi/2, so the trapezoidal
-// rule with step h converges like exp(-pi^2 / h) while the peak at u = 0, of
-// width 1/sqrt(x), is wide against h: h = 1/4 is within 7e-15 of the limit for
-// x < 6 (measured against h = 1/16 on [0.1, 6.5]), h = 1/8 serves the larger x,
-// whose sums are short.  The sum stops once a term falls below 1e-18 of the
-// running sum: cosh(u) < 1 + 42 / x, so u < 7 for every x >= 0.1.
-constexpr int kCoshTable = 64;  // cosh(k / 8)
-struct CoshTable {
-  double v[kCoshTable];
-  constexpr CoshTable() : v() {
-    for (int k = 0; k < kCoshTable; ++k) {
-      const double x = k / 8.0;
-      double term = 1.0, sum = 1.0;  // all terms positive: x < 8 needs 30 of them
-      for (int n = 1; n < 40; ++n) {
-        term *= x * x / double((2 * n - 1) * (2 * n));
-        sum += term;
-      }
-      v[k] = sum;
-    }
-  }
-};
 __constant__ CoshTable kCosh{};
-
-__device__ double bessel_k0(double x) {
-  const int step = x < 6.0 ? 2 : 1;  // in units of 1/8
-  double sum = 0.5 * exp(-x);
-  for (int k = step; k < kCoshTable; k += step) {
-    const double term = exp(-x * kCosh.v[k]);
-    sum += term;
-    if (term < 1e-18 * sum) break;
-  }
-  return 0.125 * step * sum;
-}
 
 // ------------------------------------------------------------------ atom windows
 // Follows _get_potential (namsa/msa.py:180-196) and bin_2d_array
@@ -79,7 +46,7 @@ __device__ double window_row(const double* c, int i, int j, int a, int os, doubl
     double v = 0;
     for (int k = 0; k < 3; ++k) {
       const double ak = c[k], bk = c[3 + k], ck = c[6 + k], dk = c[9 + k];
-      const double term = pre * ak * bessel_k0(2 * pi * r * sqrt(bk) + 0.1) + pre / 2. * ck / dk * exp(-pi * pi * r * r / dk);
+      const double term = pre * ak * bessel_k0(2 * pi * r * sqrt(bk) + 0.1, kCosh.v) + pre / 2. * ck / dk * exp(-pi * pi * r * r / dk);
       v = (k == 0) ? term : v + term;
     }
     accr = (b == 0) ? v : accr + v;
