@@ -106,10 +106,6 @@ struct TcGemm {
   // Partial tiles are summed in a fixed order before the epilogue.
   int run(const float* a, Addr aa, const float* b, Addr ba, long long M, int N, long long K, const Epi& e,
           cudaStream_t st, int ksplit = 1);
-  // `batch` independent GEMMs of the same shape; batch b reads A at a + b * a_bs, B at
-  // b_ptr + b * b_bs and writes at e.y + b * y_bs (floats); no K split.
-  int run_batched(const float* a, Addr aa, long long a_bs, const float* b, Addr ba, long long b_bs, long long M,
-                  int N, long long K, const Epi& e, long long y_bs, int batch, cudaStream_t st);
   // `batch` complex products in one real GEMM each: B (2 hn x 2 hk) is the real
   // embedding of src (pack_cplx_kernel: element (i, j) at src + i si + j sj, its parts
   // sp apart, negated block neg = 1 for (0, 1), 2 for (1, 0)); src of batch b at

@@ -169,7 +169,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(const Res
   cluster_sync_all();  // every CTA runs before its shared memory is written; tables and barriers are set
   const uint32_t rbuf_s = smem_u32(rbuf), cbuf_s = smem_u32(cbuf);
   const uint32_t rfull_s = smem_u32(rfull), cfull_s = smem_u32(cfull);
-  const uint32_t winv = (65536u + wc - 1) / wc;  // v / wc == (v winv) >> 16 for v < W <= 256 (checked on the host)
+  // v / wc == (v winv) >> 16: winv = 65536 / wc + e with e <= (wc - 1) / wc, so the product is off by less
+  // than the 65536 / wc to the next quotient while v (wc - 1) < 65536 (clusters have at least 4 CTAs)
+  static_assert((NX - 1) * (NX / 4 - 1) < 65536, "the quotient by multiplication");
+  const uint32_t winv = (65536u + wc - 1) / wc;
   int stopped = -1;  // the slice in which the CTA stopped
 
   for (int s = 0; s < a.slices; ++s) {

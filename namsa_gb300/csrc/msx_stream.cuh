@@ -124,17 +124,11 @@ __device__ __forceinline__ void add_release(int* p, int v) {
 // orders earlier generic-proxy accesses (also those acquired from other threads) before later bulk copies
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
-// Exchange positions of a column in a tile of C interleaved columns.  With eight
-// columns a half warp covers two rows of 64 bytes: the scatter's rows t and t + 1
-// (stride R1 = 16, 32 or 48) would fall into the same banks, so the row's lowest
-// bit is flipped where bit SH is set.
-template <int C, int SH>
+// Exchange positions of a column in a tile of C interleaved columns.
+template <int C>
 struct StreamColumn {
   float2* base;
-  __device__ __forceinline__ float2& operator[](int i) const {
-    if constexpr (C >= 16) return base[i * C];
-    else return base[(i ^ ((i >> SH) & 1)) * C];
-  }
+  __device__ __forceinline__ float2& operator[](int i) const { return base[i * C]; }
 };
 
 // One two-stage line schedule of the persistent kernel.
@@ -143,7 +137,7 @@ struct StreamLineSched {
   static constexpr int N = N_, T = T_, R1 = R1_, R2 = R2_;
   using FFT = LineFFT<N_, T_, Radices<R1_, R2_>>;
   static constexpr int E = FFT::E;
-  static constexpr int SH = swizzle_shift(R1_);  // of the exchange through staged rows and columns
+  static constexpr int SH = swizzle_shift(R1_);  // of the exchange through staged rows
 };
 
 // CT compute threads and a warpgroup of helpers, which hand their registers to the
@@ -378,8 +372,8 @@ __global__ void __launch_bounds__(384, MINB) stream_kernel(const __grid_constant
         const int x = a.x_lo + t.w * C + c;
         const float2 px = __ldg(a.pyx + NY + x);
         const int2 bd = __ldg(a.band + x);
-        static_assert(C >= 8, "a half warp covers at most two rows");
-        const StreamColumn<C, LC::SH> in{st + c};
+        static_assert(C >= 16, "a half warp stays within a row: no two of its accesses share a bank");
+        const StreamColumn<C> in{st + c};
         float2 v[E], out[E];
 #pragma unroll
         for (int m = 0; m < E; ++m) v[m] = st[(tt + T * m) * C + c];
@@ -402,7 +396,6 @@ __global__ void __launch_bounds__(384, MINB) stream_kernel(const __grid_constant
         LC::FFT::gather(v, in, tt);
         LC::FFT::template butterflies<LC::R2, LC::R1, 0, true>(v, out, twc, tt);
         // at the words of this warp's last gather: nobody else reads them any more
-        if constexpr (C < 16) __syncwarp();
 #pragma unroll
         for (int m = 0; m < E; ++m) st[(tt + T * m) * C + c] = out[m];
       }

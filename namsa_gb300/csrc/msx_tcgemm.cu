@@ -88,16 +88,10 @@ __host__ __device__ __forceinline__ long long addr_of(const Addr& a, long long r
 // address and the split of k0 are computed once per thread; the 8 elements step
 // through k incrementally, with two 16-byte loads when they are contiguous.
 __global__ void pack_kernel(const float* __restrict__ src, Addr a, long long rows, long long K, int tile_rows,
-                            long long rows_pad, int kblocks, uint4* __restrict__ img, int batch = 1,
-                            long long src_bs = 0) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+                            long long rows_pad, int kblocks, uint4* __restrict__ img) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long chunks = (long long)kblocks * (BK / 8);
-  const long long per = rows_pad * chunks;
-  if (i >= per * batch) return;
-  const long long bt = i / per;  // batch of this element; its image and source are offset by it
-  i -= bt * per;
-  src += bt * src_bs;
-  img += bt * (per * 8 * 2 / 16);
+  if (i >= rows_pad * chunks) return;
   const long long r = i / chunks;
   const int ch = (int)(i - r * chunks);
   const long long k0 = (long long)ch * 8;
@@ -190,16 +184,8 @@ __global__ void __launch_bounds__(128) gemm_kernel(const uint8_t* __restrict__ A
   __shared__ uint64_t full[STAGES], empty[STAGES], done;
   __shared__ uint32_t tmem_base;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int splits = (kblocks + kper - 1) / kper;
   const int tiles = ntiles_total;
-  const int bt = (int)blockIdx.x / (tiles * splits);  // batch
-  const int inb = (int)blockIdx.x - bt * tiles * splits;
-  const int split = inb / tiles, tile = inb % tiles;
-  A += (size_t)bt * (size_t)(tiles / ntiles_n) * kblocks * A_BYTES;
-  B += (size_t)bt * (size_t)ntiles_n * kblocks * C::B_BYTES;
-  e.y += bt * e.ybs;
-  if (e.add) e.add += bt * e.ybs;
-  if (e.act) e.act += bt * e.ybs;
+  const int split = (int)blockIdx.x / tiles, tile = (int)blockIdx.x % tiles;
   const int mt = tile / ntiles_n, nt = tile % ntiles_n;
   const int kb0 = split * kper, kb1 = kb0 + kper < kblocks ? kb0 + kper : kblocks;
   if (warp == 0) {
@@ -362,21 +348,24 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits,
 }
 
 // ------------------------------------------------------------ persistent, warp-specialised GEMM
-// One CTA of 416 threads per SM loops over the output tiles (batch, mt, nt) =
+// One CTA of 512 threads per SM loops over the items (batch, split, mt, nt) =
 // blockIdx.x, blockIdx.x + gridDim.x, ... (nt fastest):
-//   warps 0-3   operand loaders: bring the FP32 rows of A for a K block into an FP32
-//               staging slot (bulk copies where A's rows or row groups are contiguous,
-//               else 4-byte asynchronous copies), then round them to bfloat16 into the
-//               swizzled stage (no packing pass over A); thread 0 also moves the stage's
-//               packed B block with one bulk copy;
-//   warps 4-11  epilogue, two groups of four taking alternate tiles; warp w reads
+//   warps 0-3   operand loaders: round the FP32 values of a K block from a staging slot
+//               to bfloat16 into the swizzled stage (no packing pass over A; in the FUSE
+//               form B too) and, unless every copy is a bulk copy of whole runs, first
+//               bring them into the slot (16-byte or 4-byte asynchronous copies, loads);
+//   warps 4-11  epilogue, two groups of four taking alternate items; warp w reads
 //               TMEM lanes 32 (w mod 4) .. + 31 (tile rows);
-//   warp 12     holds two BN-column accumulators in TMEM; lane 0 issues the MMAs.
-// The accumulators alternate between tiles, so a tile's epilogue overlaps the next
-// tile's loads and MMAs.  Barriers: afull[slot] (staging slot filled: 128 loader
-// arrivals with the bulk bytes), full[s] (128 loader arrivals: bfloat16 A written),
-// bfull[s] (the B bytes), empty[s] (MMA commit), accf[b] (MMA commit of accumulator
-// b), acce[b] (one arrival per warp of the epilogue group).  Rows of A at or past M
+//   warp 12     holds two BN-column accumulators in TMEM; lane 0 issues the MMAs;
+//   warp 13     the bulk copies of FP32 operands (`bulk` operands only);
+//   warp 14     lane 0: the stage's packed B block with one bulk copy (not FUSE).
+// The accumulators alternate between items, so an item's epilogue overlaps the next
+// one's loads and MMAs.  Barriers: afull[slot] (staging slot filled: warp 13's one
+// arrival with the bytes, else 128 loader arrivals), afree[slot] (a loader arrival:
+// the slot is rounded, warp 13 may fill it again), full[s] (128 loader arrivals:
+// bfloat16 written), bfull[s] (the B bytes, or in the FUSE form a loader arrival),
+// empty[s] (MMA commit), accf[b] (MMA commit of accumulator b), acce[b] (one arrival
+// per warp of the epilogue group).  Rows of A at or past M
 // are not converted (an MMA row depends on its own A row only, and those rows are not
 // stored); K steps of 16 past K are not issued, and the rest of the last K step is
 // zero.  Every wait is bounded; the loaders take each decision together (a barrier
@@ -1501,7 +1490,7 @@ int ws_split_count(int kblocks, int ksplit) {
 
 template <int BN>
 cudaError_t launch_gemm_bn(const uint8_t* a, const uint8_t* b, long long mtiles, int ntiles, int kblocks, int kper,
-                           float* part, const Epi& e, int* err, cudaStream_t st, int batch = 1) {
+                           float* part, const Epi& e, int* err, cudaStream_t st) {
   // the shared-memory attribute is set once per device (it belongs to the device's context)
   static std::atomic<unsigned long long> configured{0};
   int dev = 0;
@@ -1514,7 +1503,7 @@ cudaError_t launch_gemm_bn(const uint8_t* a, const uint8_t* b, long long mtiles,
     configured.fetch_or(bit, std::memory_order_release);
   }
   const int splits = (kblocks + kper - 1) / kper;
-  gemm_kernel<BN><<<(unsigned)(mtiles * ntiles * splits * batch), 128, Cfg<BN>::SMEM, st>>>(
+  gemm_kernel<BN><<<(unsigned)(mtiles * ntiles * splits), 128, Cfg<BN>::SMEM, st>>>(
       a, b, kblocks, ntiles, (int)(mtiles * ntiles), kper, part, e, err);
   if (part) {
     const long long n = e.M * (long long)e.N;
@@ -1638,46 +1627,10 @@ int TcGemm::run(const float* a, Addr aa, const float* b, Addr ba, long long M, i
                                                                    reinterpret_cast<uint4*>(a_img));
   const uint8_t* ai = reinterpret_cast<const uint8_t*>(a_img);
   switch (bn) {
-    case 32: c = tg::launch_gemm_bn<32>(ai, bi, mtiles, ntiles, kblocks, kper, part, e, err, st); break;
     case 64: c = tg::launch_gemm_bn<64>(ai, bi, mtiles, ntiles, kblocks, kper, part, e, err, st); break;
     case 128: c = tg::launch_gemm_bn<128>(ai, bi, mtiles, ntiles, kblocks, kper, part, e, err, st); break;
     default: c = tg::launch_gemm_bn<256>(ai, bi, mtiles, ntiles, kblocks, kper, part, e, err, st); break;
   }
-  return c == cudaSuccess ? MSX_OK : MSX_ERR_CUDA;
-}
-
-int TcGemm::run_batched(const float* a, Addr aa, long long a_bs, const float* b, Addr ba, long long b_bs, long long M,
-                        int N, long long K, const Epi& epi, long long y_bs, int batch, cudaStream_t st) {
-  if (batch < 1 || M <= 0 || N <= 0 || K <= 0 || N > 4096) return MSX_ERR_INVALID;
-  const int bn = bn_for(N);
-  const long long mtiles = (M + tg::BM - 1) / tg::BM;
-  const int ntiles = (N + bn - 1) / bn;
-  const long long kbl = (K + tg::BK - 1) / tg::BK;
-  if (kbl > (1LL << 30) || mtiles * ntiles * batch > (1LL << 30)) return MSX_ERR_INVALID;
-  const int kblocks = (int)kbl;
-  const size_t b_bytes = (size_t)batch * ntiles * kblocks * bn * tg::BK * 2;
-  int rc = reserve(0, b_bytes);
-  if (rc != MSX_OK) return rc;
-  const long long b_rows = (long long)ntiles * bn;
-  const long long b_thr = b_rows * kblocks * (tg::BK / 8) * batch;
-  tg::pack_kernel<<<(unsigned)((b_thr + 255) / 256), 256, 0, st>>>(b, ba, N, K, bn, b_rows, kblocks,
-                                                                   reinterpret_cast<uint4*>(b_img), batch, b_bs);
-  Epi e = epi;
-  e.M = M;
-  e.N = N;
-  e.ybs = y_bs;
-  const uint8_t* bi = reinterpret_cast<const uint8_t*>(b_img);
-  cudaError_t c;
-  tg::WsArgs w{};
-  w.a = tg::ws::Op{a, aa, a_bs, M, 0, 0, 0, 0, 0};
-  w.b_img = bi;
-  w.K = K;
-  w.kblocks = kblocks;
-  w.kper = kblocks;
-  w.splits = 1;
-  w.ntiles = ntiles;
-  w.mtiles = mtiles;
-  c = tg::launch_ws(bn, w, e, err, st, batch);
   return c == cudaSuccess ? MSX_OK : MSX_ERR_CUDA;
 }
 
