@@ -6,8 +6,9 @@
 
 #include <cooperative_groups.h>
 
-#include <atomic>
 #include <cmath>
+#include <map>
+#include <mutex>
 
 namespace msx {
 
@@ -451,16 +452,8 @@ cudaError_t launch_probe(int Ny, int Nx, float kmax, double lambda, float k_semi
   probe_kernel<<<grid, 128, 0, st>>>(Ny, Nx, kmax, lambda, k_semi, C1, C3, C5, smooth, psik, aperture);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || norm == nullptr) return e;
-  // clusters of 16 are above the portable size: allowed once per device
-  static std::atomic<unsigned long long> allowed{0};
   int dev = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (!(allowed.load(std::memory_order_acquire) & bit)) {
-    e = cudaFuncSetAttribute(probe_norm_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    allowed.fetch_or(bit, std::memory_order_release);
-  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(kNormCtas);
   cfg.blockDim = dim3(kNormThreads);
@@ -471,6 +464,28 @@ cudaError_t launch_probe(int Ny, int Nx, float kmax, double lambda, float k_semi
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
+  // clusters of 16 are above the portable size: asked once per device; one CTA sums where
+  // they are refused (part of a GPU)
+  static std::mutex m;
+  static std::map<int, FormState> form;
+  bool cluster;
+  {
+    std::lock_guard<std::mutex> lock(m);
+    cluster = form[dev].ready([&] {
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaError_t r = cudaThreadExchangeStreamCaptureMode(&mode);
+      if (r != cudaSuccess) return r;
+      int n = 0;
+      r = cudaFuncSetAttribute(probe_norm_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (r == cudaSuccess) r = cudaOccupancyMaxActiveClusters(&n, probe_norm_kernel, &cfg);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      return r == cudaSuccess && n < 1 ? cudaErrorInvalidConfiguration : r;
+    });
+  }
+  if (!cluster) {
+    cfg.gridDim = dim3(1);
+    cfg.numAttrs = 0;
+  }
   return cudaLaunchKernelEx(&cfg, probe_norm_kernel, psik, (long long)Ny * Nx, norm);
 }
 
