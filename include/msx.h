@@ -145,7 +145,13 @@ MSX_API int msx_build_probe(int ny, int nx, float kmax, double lambda, float k_s
  * slice; for groups of waves that stay in L2, all slices in one persistent
  * kernel; for a few positions on grids up to 256 x 256, each wave in the shared
  * memory of a thread-block cluster.  All three give the same patterns within
- * float32 rounding.  Replaces the per-batch cuFFT plans and allocations of
+ * float32 rounding (msx_plan_route tells which one a call takes).  The one-kernel
+ * form is a cooperative launch: it starts once every SM has room for it and holds
+ * them through its slices, so it waits for long-running kernels of other streams
+ * and leaves them no SM meanwhile; a cluster needs up to 16 SMs of one GPC at a
+ * time.  Where the GPU is shared with other work, msx_plan_set_schedule makes the
+ * plan run two passes a slice, on whatever SMs are free.  A device that refuses a
+ * form (part of a GPU) runs the passes.  Replaces the per-batch cuFFT plans and allocations of
  * MSAGPU.multislice (namsa/msa.py:843-881) and plan_simulation's batching
  * (namsa/msa.py:445-461).
  */

@@ -579,13 +579,14 @@ int grow(T** buf, size_t* have, size_t words, const char* what) {
 // 1/3): from `few` positions on, and up to `most` MB of band columns of all
 // waves, it was the faster one.  The passes gain with long launches (no
 // part-filled last waves of tiles); the kernel's waits between the passes of one
-// wave cost most on short lines.  Passes / all slices, us, at 1, 16, 64, 256 positions:
-//   256 x 256   226/235   303/274   650/530    2133/2005
-//   384 x 384   473/461   567/545   1442/1243  5203/4855
-//   512 x 512   388/358   706/569   2256/2103  8359/8271
-//   768 x 768   972/729   1574/1259 5123/4917  (128: 9626/10078)
-//   768 x 256   399/371   646/555   1809/1835  6098/7289
-//   256 x 768   414/336   597/530   1796/1712  6515/6762
+// wave cost most on short lines.  Passes (with the schedules of few lines where a
+// call has few) / all slices, us, at 1, 8, 16, 64, 256 positions:
+//   256 x 256   212/235   235/253   304/276   647/529    2130/2012
+//   384 x 384   438/457   462/504   551/543   1438/1241  5195/4844
+//   512 x 512   385/351   491/412   700/569   2256/2117  8349/8333
+//   768 x 768   724/727   966/947   1555/1261 5121/4904  (128: 9653/10068)
+//   768 x 256   349/367   418/413   637/548   1801/1826  6114/7251
+//   256 x 768   343/331   413/421   593/516   1784/1702  6530/6747
 constexpr size_t kStreamBytes = (size_t)80 << 20;
 struct StreamRange {
   int few, most;

@@ -30,9 +30,9 @@ __constant__ CoshTable kCosh{};
 // Bound by double-precision instructions (about two fused multiply-adds a
 // clock and SM): an exponential per quadrature term.  The quadrant takes a
 // quarter of the samples, the table the cosh of every term, the coarser step
-// half of the terms of small x, and one thread per oversampled row of a bin
+// half of the terms of x < 3, and one thread per oversampled row of a bin
 // fills the chip.  94 x 94 bins of one species at oversample 2: 938 us with
-// every bin evaluated by one thread, 110 us so.
+// every bin evaluated by one thread, 116 us so.
 constexpr int kWinThreads = 128;
 
 // sum over b (in order) of the samples (i os + a, j os + b)
