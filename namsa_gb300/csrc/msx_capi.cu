@@ -717,7 +717,7 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
   const int ny = p->ny, nx = p->nx;
   const int cluster = resident_cluster(p, a);
   const int streamed = cluster ? 0 : stream_group(p, a);
-  const int group = streamed ? streamed : a.group;
+  const int group = cluster ? a.num_probes : streamed ? streamed : a.group;
   const int gmax = a.num_probes < group ? a.num_probes : group;
   if (!workspace_holds(p, gmax))
     return fail(MSX_ERR_ALLOC, "the plan's workspace does not hold %d waves (an earlier allocation failed)", gmax);
@@ -778,7 +778,7 @@ int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const Host
     c.x_begin = 0;
     c.ncols = nx;
     MSX_CUDA(p->col_ops->col(COL_INIT, c, st), "probe formation pass");
-    if (cluster) {  // one group: every position
+    if (cluster) {  // one group of every position
       if (hp)
         for (int i = 0; i * hp->chunk < a.num_slices; ++i)
           MSX_CUDA(cudaStreamWaitEvent(st, (*hp->chunk_ev)[i], 0), "cudaStreamWaitEvent");
@@ -1325,7 +1325,8 @@ int msx_multislice_host(msx_plan* p, const float* trans_host, int num_slices, co
   a.num_probes = num_probes; a.kmax = kmax; a.lambda = lambda; a.slice_t = slice_t; a.k_band = k_band;
   a.cbed = p->io_cbed; a.crop_y = crop_y; a.crop_x = crop_x;
   a.group = p->group; a.row_sched = p->row_sched; a.col_sched = p->col_sched;
-  const int streamed = resident_cluster(p, a) ? 0 : stream_group(p, a), step = streamed ? streamed : p->group;
+  const bool cluster = resident_cluster(p, a) > 0;
+  const int streamed = cluster ? 0 : stream_group(p, a), step = cluster ? num_probes : streamed ? streamed : p->group;
   const int ngroups = (num_probes + step - 1) / step;
   const int chunk = 8;
   const int nchunks = (num_slices + chunk - 1) / chunk;

@@ -72,3 +72,23 @@ def test_tuned_batch():
             assert rel(o, w) < 1.2e-6
     batch.check()
     batch.close()
+
+
+def test_clusters_beyond_the_tuned_group_take_one_launch():
+    """Device and host calls: one kernel for all positions, one download."""
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.set_device(0)
+    x = case(128, 128, 5, 6, 8)
+    plan = engine.Plan(128, 128)
+    want = plan.multislice(*x).clone()
+    plan.autotune(*x, iters=2, max_workspace_bytes=1)
+    host = [t.cpu().pin_memory() for t in (x[0], x[1], x[3])]
+    h = plan.multislice_host(host[0], host[1], float(x[2].item()), host[2], *x[4:])
+    torch.cuda.synchronize()
+    assert torch.equal(h, want.cpu())
+    for _ in range(2):  # the first trace of a process starts the tracer late
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            assert torch.equal(plan.multislice(*x), want)
+            torch.cuda.synchronize()
+    assert sum('resident_kernel' in e.name for e in prof.events()) == 1
+    plan.close()
