@@ -1646,6 +1646,7 @@ msx_plan* batch_plan(msx_batch* b, int branch, int ny, int nx, int* rc) {
     }
   msx_plan* p = nullptr;
   *rc = msx_plan_create(ny, nx, waves, &p);
+  if (*rc == MSX_ERR_ALLOC && group < waves) *rc = msx_plan_create(ny, nx, group, &p);  // the passes need no more
   if (*rc != MSX_OK) return nullptr;
   if (tuned) {
     *rc = msx_plan_set_schedule(p, r, c, group);
@@ -1674,8 +1675,8 @@ int batch_set_schedule(msx_batch* b, int ny, int nx, int row_schedule, int col_s
         if (rc != MSX_OK) return rc;
         allow_forms(kv.second, forms);
         if (forms & 3) {
-          rc = ensure_workspace(kv.second, (size_t)batch_waves(ny, nx));
-          if (rc == MSX_OK) rc = prepare_tma(kv.second);
+          rc = ensure_workspace(kv.second, (size_t)batch_waves(ny, nx));  // or the forms go without
+          if (rc == MSX_OK || rc == MSX_ERR_ALLOC) rc = prepare_tma(kv.second);
           if (rc != MSX_OK) return rc;
         }
       }
