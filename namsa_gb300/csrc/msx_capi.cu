@@ -114,6 +114,7 @@ struct msx_plan {
   float2* tw_col = nullptr;
   cudaStream_t work = nullptr;
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
+  cudaEvent_t ev_last = nullptr;  // after the last call that used the plan's waves, tables and counters
   bool use_graph = true;
   cudaGraphExec_t gexec = nullptr;
   std::vector<unsigned char> gkey;
@@ -686,31 +687,41 @@ bool few_launches(msx_plan* p, const MsArgs& a) {
   return g > 0 && a.num_probes <= 2 * g;
 }
 
-// Runs enqueue(stream) on the plan's stream, ordered after and before the caller's: calls
-// of one plan share its waves, tables, partial sums and counters, whichever streams they
-// come from.  Under a capture it joins the caller's stream, and the caller keeps the
-// captured work apart from the plan's other calls.
+// Calls of one plan share its waves, tables, partial sums and counters, so each follows
+// the last one (ev_last), whichever streams they come from.  Under a capture a call
+// joins the caller's stream, and the caller keeps the captured work apart from the
+// plan's other calls.
+int after_last_call(msx_plan* p, cudaStream_t st) {
+  MSX_CUDA(cudaStreamWaitEvent(st, p->ev_last, 0), "cudaStreamWaitEvent");
+  return MSX_OK;
+}
+
+// Runs enqueue(stream) in that order: on the caller's stream, or for recorded graphs and
+// calls of a few launches on the plan's, which follows the caller's and is followed by it.
+// A failed call is ordered too: what was enqueued before the failure uses the caller's buffers.
 template <class F>
-int on_plan_stream(msx_plan* p, cudaStream_t caller, F enqueue) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  MSX_CUDA(cudaStreamIsCapturing(caller, &cap), "cudaStreamIsCapturing");
-  if (cap != cudaStreamCaptureStatusNone) return enqueue(caller, true);
-  MSX_CUDA(cudaEventRecord(p->ev_in, caller), "cudaEventRecord");
-  MSX_CUDA(cudaStreamWaitEvent(p->work, p->ev_in, 0), "cudaStreamWaitEvent");
-  const int rc = enqueue(p->work, false);
+int in_call_order(msx_plan* p, cudaStream_t caller, bool own_stream, F enqueue) {
+  cudaStream_t st = caller;
+  if (own_stream) {
+    MSX_CUDA(cudaEventRecord(p->ev_in, caller), "cudaEventRecord");
+    MSX_CUDA(cudaStreamWaitEvent(p->work, p->ev_in, 0), "cudaStreamWaitEvent");
+    st = p->work;
+  }
+  const int ordered = after_last_call(p, st);
+  if (ordered != MSX_OK) return ordered;
+  const int rc = enqueue(st);
   const std::string msg = g_err;
-  // also after a failure: what was enqueued before it still uses the caller's buffers
-  MSX_CUDA(cudaEventRecord(p->ev_out, p->work), "cudaEventRecord");
-  MSX_CUDA(cudaStreamWaitEvent(caller, p->ev_out, 0), "cudaStreamWaitEvent");
+  MSX_CUDA(cudaEventRecord(p->ev_last, st), "cudaEventRecord");
+  if (own_stream) MSX_CUDA(cudaStreamWaitEvent(caller, p->ev_last, 0), "cudaStreamWaitEvent");
   if (rc != MSX_OK) g_err = msg;
   return rc;
 }
 
-// Orders `st`, on which a tuning or timing call is about to use the plan, after the plan's own work.
-int after_plan_stream(msx_plan* p, cudaStream_t st) {
-  MSX_CUDA(cudaEventRecord(p->ev_out, p->work), "cudaEventRecord");
-  MSX_CUDA(cudaStreamWaitEvent(st, p->ev_out, 0), "cudaStreamWaitEvent");
-  return MSX_OK;
+bool capturing(cudaStream_t st, int* rc) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(st, &cap);
+  *rc = e == cudaSuccess ? MSX_OK : cuda_fail(e, "cudaStreamIsCapturing");
+  return cap != cudaStreamCaptureStatusNone;
 }
 
 int enqueue_multislice(msx_plan* p, const MsArgs& a, cudaStream_t st, const HostPipe* hp = nullptr) {
@@ -950,6 +961,7 @@ int msx_plan_create(int ny, int nx, int group, msx_plan** out) {
     cudaError_t e = cudaStreamCreateWithFlags(&p->work, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->ev_in, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->ev_out, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p->ev_last, cudaEventDisableTiming);
     if (e != cudaSuccess) rc = cuda_fail(e, "plan stream/events");
   }
   if (rc != MSX_OK) {
@@ -976,6 +988,7 @@ int msx_plan_destroy(msx_plan* p) {
   if (p->copy) cudaStreamDestroy(p->copy);
   if (p->ev_in) cudaEventDestroy(p->ev_in);
   if (p->ev_out) cudaEventDestroy(p->ev_out);
+  if (p->ev_last) cudaEventDestroy(p->ev_last);
   if (p->work) cudaStreamDestroy(p->work);
   delete p;
   return MSX_OK;
@@ -1103,8 +1116,13 @@ int msx_multislice(msx_plan* p, const float* trans_dev, int num_slices, const fl
   a.pos = positions_dev; a.num_probes = num_probes; a.kmax = kmax; a.lambda = lambda; a.slice_t = slice_t;
   a.k_band = k_band; a.cbed = cbed_out_dev; a.crop_y = crop_y; a.crop_x = crop_x;
   a.group = p->group; a.row_sched = p->row_sched; a.col_sched = p->col_sched;
-  return on_plan_stream(p, (cudaStream_t)stream, [&](cudaStream_t st, bool captured) -> int {
-    if (captured || !p->use_graph || few_launches(p, a)) return enqueue_multislice(p, a, st);
+  cudaStream_t caller = (cudaStream_t)stream;
+  int rc = MSX_OK;
+  const bool captured = capturing(caller, &rc);
+  if (rc != MSX_OK) return rc;
+  if (captured) return enqueue_multislice(p, a, caller);
+  return in_call_order(p, caller, p->use_graph, [&](cudaStream_t st) -> int {
+    if (!p->use_graph || few_launches(p, a)) return enqueue_multislice(p, a, st);
     std::vector<unsigned char> key(sizeof(MsArgs));
     std::memcpy(key.data(), &a, sizeof(MsArgs));
     if (!p->gexec || key != p->gkey) {
@@ -1162,8 +1180,12 @@ int msx_multislice_detect(msx_plan* p, const float* trans_dev, int num_slices, c
     p->partial_words = need;
   }
   drop_graph(p);  // the detector sequence is launched directly
-  return on_plan_stream(p, (cudaStream_t)stream,
-                        [&](cudaStream_t st, bool) -> int { return enqueue_multislice(p, a, st); });
+  cudaStream_t caller = (cudaStream_t)stream;
+  int rc = MSX_OK;
+  const bool captured = capturing(caller, &rc);
+  if (rc != MSX_OK) return rc;
+  if (captured) return enqueue_multislice(p, a, caller);
+  return in_call_order(p, caller, false, [&](cudaStream_t st) -> int { return enqueue_multislice(p, a, st); });
 }
 
 int msx_propagator_table(int ny, int nx, float kmax, double lambda, double slice_t, float k_band, float* ptab_out_dev,
@@ -1306,10 +1328,14 @@ int msx_multislice_host(msx_plan* p, const float* trans_host, int num_slices, co
   // everything here follows the caller's earlier work and this plan's earlier calls
   MSX_CUDA(cudaEventRecord(p->ev_in, caller), "cudaEventRecord");
   MSX_CUDA(cudaStreamWaitEvent(w, p->ev_in, 0), "cudaStreamWaitEvent");
+  if (cap == cudaStreamCaptureStatusNone) {
+    rc = after_last_call(p, w);
+    if (rc != MSX_OK) return rc;
+  }
   if (graph && p->gexec_host && key == p->gkey_host) {
     MSX_CUDA(cudaGraphLaunch(p->gexec_host, w), "cudaGraphLaunch");
-    MSX_CUDA(cudaEventRecord(p->ev_out, w), "cudaEventRecord");
-    MSX_CUDA(cudaStreamWaitEvent(caller, p->ev_out, 0), "cudaStreamWaitEvent");
+    MSX_CUDA(cudaEventRecord(p->ev_last, w), "cudaEventRecord");
+    MSX_CUDA(cudaStreamWaitEvent(caller, p->ev_last, 0), "cudaStreamWaitEvent");
     return MSX_OK;
   }
   if (graph) {
@@ -1390,8 +1416,9 @@ int msx_multislice_host(msx_plan* p, const float* trans_host, int num_slices, co
     release();
   }
   if (rc != MSX_OK) return rc;
-  MSX_CUDA(cudaEventRecord(p->ev_out, w), "cudaEventRecord");
-  MSX_CUDA(cudaStreamWaitEvent(caller, p->ev_out, 0), "cudaStreamWaitEvent");
+  cudaEvent_t done = cap == cudaStreamCaptureStatusNone ? p->ev_last : p->ev_out;
+  MSX_CUDA(cudaEventRecord(done, w), "cudaEventRecord");
+  MSX_CUDA(cudaStreamWaitEvent(caller, done, 0), "cudaStreamWaitEvent");
   return MSX_OK;
 }
 
@@ -1409,7 +1436,7 @@ int msx_plan_profile(msx_plan* p, const float* trans_dev, int num_slices, const 
   const size_t wave = (size_t)ny * nx;
   cudaStream_t st = (cudaStream_t)stream;
   int rcp = ensure_ptab(p);
-  if (rcp == MSX_OK) rcp = after_plan_stream(p, st);
+  if (rcp == MSX_OK) rcp = after_last_call(p, st);
   if (rcp != MSX_OK) return rcp;
   cudaEvent_t ev[4];
   for (auto& e : ev) MSX_CUDA(cudaEventCreate(&e), "cudaEventCreate");
@@ -1464,7 +1491,7 @@ int msx_plan_autotune(msx_plan* p, const float* trans_dev, int num_slices, const
     return fail(MSX_ERR_INVALID, "autotune needs slices, probes, inputs and iters > 0");
   if (!aligned8({trans_dev, psi_k_dev, positions_dev, normalization_dev})) return fail(MSX_ERR_INVALID, kAlign8);
   int rcp = ensure_ptab(p);
-  if (rcp == MSX_OK) rcp = after_plan_stream(p, (cudaStream_t)stream);
+  if (rcp == MSX_OK) rcp = after_last_call(p, (cudaStream_t)stream);
   if (rcp != MSX_OK) return rcp;
   const SchedOps *rops, *cops;
   const int nr = schedule_table(p->nx, &rops), nc = schedule_table(p->ny, &cops);
